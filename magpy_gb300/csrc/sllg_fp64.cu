@@ -10,7 +10,7 @@
 // step counter, draw 3n increments, take one Heun (lib/integrators.cpp:372)
 // or implicit-midpoint (lib/integrators.cpp:576) step at t = step*dt,
 // optionally renormalise, and write the zero-order-hold sample.
-#include <type_traits>
+#include <algorithm>
 #include "common.cuh"
 #include "llg64.cuh"
 #include "plan.hpp"
@@ -29,50 +29,47 @@ struct Member {
     const double *pt, *rt;  // pair tables of the member's cluster
     const float4 *pr;       // FP32 pair table (r0, r1, r2, P), [N][N], index j*n + q
     double *sm;             // [3n] shared moments
-    float *smf;             // [3n] shared FP32 moments (FP32 dipolar sum)
+    float4 *smf;            // [n] shared FP32 moments (FP32 dipolar sum)
     double *red;            // [p2] shared reduction buffer
     int n, q, p2;
     bool active;
     MemberSync ms;
 };
 
-// Shared-memory doubles per member: moments, reduction buffer and, with the
-// FP32 dipolar sum, FP32 moments.
+// Shared-memory doubles per member: moments and reduction buffer, or with the
+// FP32 dipolar sum FP32 moments (16 bytes a particle) and a reduction buffer
+// (one word per warp of a CTA-wide member).
 __host__ __device__ inline int slot_doubles(int n, int p2, bool dip32)
 {
-    return 3 * n + p2 + (dip32 ? (3 * n + 1) / 2 : 0);
+    return dip32 ? 2 * n + (n > 32 ? 34 : 0) : 3 * n + p2;
 }
 
 // Dipolar sum in FP32 from the (r0, r1, r2, P) pair table: fused products,
 // FP32 partial sums over 32 sources, added in FP64.  The mixed-precision
 // implicit mode uses it inside the FP64 Newton solve.
-__device__ inline void dipolar32(const Member &M, double h[3])
+__device__ inline void dipolar32(const Member &M, double H[3])
 {
     const int n = M.n, q = M.q;
-    double H0 = 0.0, H1 = 0.0, H2 = 0.0;
+    H[0] = H[1] = H[2] = 0.0;
     for (int j0 = 0; j0 < n; j0 += 32) {
         const int j1 = min(n, j0 + 32);
         float h0 = 0.f, h1 = 0.f, h2 = 0.f;
         for (int j = j0; j < j1; j++) {
             const float4 r = __ldg(M.pr + (size_t)j * n + q);  // P = 0 on the diagonal
-            const float mj0 = M.smf[3 * j], mj1 = M.smf[3 * j + 1], mj2 = M.smf[3 * j + 2];
-            const float d3 = 3.f * __fmaf_rn(mj2, r.z, __fmaf_rn(mj1, r.y, __fmul_rn(mj0, r.x)));
-            h0 = __fmaf_rn(r.w, __fmaf_rn(d3, r.x, -mj0), h0);
-            h1 = __fmaf_rn(r.w, __fmaf_rn(d3, r.y, -mj1), h1);
-            h2 = __fmaf_rn(r.w, __fmaf_rn(d3, r.z, -mj2), h2);
+            const float4 mj = M.smf[j];
+            const float d3 = 3.f * __fmaf_rn(mj.z, r.z, __fmaf_rn(mj.y, r.y, __fmul_rn(mj.x, r.x)));
+            h0 = __fmaf_rn(r.w, __fmaf_rn(d3, r.x, -mj.x), h0);
+            h1 = __fmaf_rn(r.w, __fmaf_rn(d3, r.y, -mj.y), h1);
+            h2 = __fmaf_rn(r.w, __fmaf_rn(d3, r.z, -mj.z), h2);
         }
-        H0 += (double)h0;
-        H1 += (double)h1;
-        H2 += (double)h2;
+        H[0] += (double)h0;
+        H[1] += (double)h1;
+        H[2] += (double)h2;
     }
-    h[0] += H0;
-    h[1] += H1;
-    h[2] += H2;
 }
 
 // Effective field of one particle: lib/simulation.cpp:271-290 (anisotropy,
 // lib/field.cpp:116-132; Zeeman along z, :81-88; dipolar pair sum, :187-225).
-template <bool DIP32>
 __device__ void eff_field(const Member &M, const Particle &pa, double h[3], const double s[3],
                           double t)
 {
@@ -83,13 +80,7 @@ __device__ void eff_field(const Member &M, const Particle &pa, double h[3], cons
     h[1] += dot * pa.ax[1];
     h[2] += dot * pa.ax[2];
     h[2] += f64::field_value(M.d->shape, t, M.d->happ, M.d->fapp);
-    if (DIP32 && M.d->interactions && M.n > 1) {
-        if (M.active)
-            for (int c = 0; c < 3; c++) M.smf[3 * M.q + c] = (float)s[c];
-        M.ms.sync();
-        if (M.active) dipolar32(M, h);
-        M.ms.sync();
-    } else if (M.d->interactions && M.n > 1) {
+    if (M.d->interactions && M.n > 1) {
         if (M.active) {
             M.sm[3 * M.q + 0] = s[0];
             M.sm[3 * M.q + 1] = s[1];
@@ -144,13 +135,12 @@ __device__ inline bool member_any(const Member &M, bool pred)
 }
 
 // integrator::heun, lib/integrators.cpp:372-405, on the particle's 3x3 block.
-template <bool DIP32>
 __device__ void heun_step(const Member &M, const Particle &pa, double x[3],
                           const double px[3], const double w[3], double t)
 {
     const double dt = M.d->dt, sq = M.d->sqrt_dt;
     double h[3], a[3], b[9], xt[3];
-    eff_field<DIP32>(M, pa, h, px, t);
+    eff_field(M, pa, h, px, t);
     f64::drift(a, px, pa.alpha, h);
     f64::diffusion(b, px, pa.sr, pa.alpha);
     for (int r = 0; r < 3; r++) {
@@ -158,7 +148,7 @@ __device__ void heun_step(const Member &M, const Particle &pa, double x[3],
         for (int c = 0; c < 3; c++) xt[r] += b[3 * r + c] * w[c] * sq;
     }
     double ta[3], tb[9];
-    eff_field<DIP32>(M, pa, h, xt, t + dt);
+    eff_field(M, pa, h, xt, t + dt);
     f64::drift(ta, xt, pa.alpha, h);
     f64::diffusion(tb, xt, pa.sr, pa.alpha);
     for (int r = 0; r < 3; r++) {
@@ -172,7 +162,6 @@ __device__ void heun_step(const Member &M, const Particle &pa, double x[3],
 // Jacobian is block-diagonal (the field Jacobian ignores the dipolar term,
 // lib/simulation.cpp:292-303), so the dense dgesv is n independent 3x3
 // solves; the convergence norm couples the whole member.
-template <bool DIP32>
 __device__ int32_t implicit_step(const Member &M, const Particle &pa, double x[3],
                                  const double px[3], const double w[3], double t)
 {
@@ -183,7 +172,7 @@ __device__ int32_t implicit_step(const Member &M, const Particle &pa, double x[3
         dwm[c] = ((-Ah < lo) ? lo : -Ah) * sq;       // std::max(-Ah, .) * sqrt(dt)
     }
     double h[3], a[3], b[9];
-    eff_field<DIP32>(M, pa, h, px, t);
+    eff_field(M, pa, h, px, t);
     f64::drift(a, px, pa.alpha, h);
     f64::diffusion(b, px, pa.sr, pa.alpha);
     for (int r = 0; r < 3; r++) {
@@ -198,44 +187,215 @@ __device__ int32_t implicit_step(const Member &M, const Particle &pa, double x[3
     const double tm = t + dt / 2;
     while ((err > tol) && (iter-- > 0)) {
         double xt[3] = {x[0], x[1], x[2]};
-        eff_field<DIP32>(M, pa, h, xt, tm);
+        eff_field(M, pa, h, xt, tm);
         f64::drift(a, xt, pa.alpha, h);
         f64::diffusion(b, xt, pa.sr, pa.alpha);
-        // The residual F is FP64 in both modes (it defines the root); the
-        // quasi-Jacobian only steers the iteration, and the mixed mode forms
-        // it and solves with it in FP32 (JT).
-        using JT = typename std::conditional<DIP32, float, double>::type;
-        JT adash[9], bdash[27], J[9];
+        double adash[9], bdash[27], J[9];
         double F[3];
-        {
-            const JT xj[3] = {(JT)xt[0], (JT)xt[1], (JT)xt[2]};
-            const JT hjv[3] = {(JT)h[0], (JT)h[1], (JT)h[2]};
-            JT hjj[9];
-            for (int k = 0; k < 9; k++) hjj[k] = (JT)pa.hj[k];
-            f64::drift_jacobian<JT>(adash, xj, (JT)pa.alpha, hjv, hjj);
-            f64::diffusion_jacobian<JT>(bdash, xj, (JT)pa.sr, (JT)pa.alpha);
-        }
+        f64::drift_jacobian<double>(adash, xt, pa.alpha, h, pa.hj);
+        f64::diffusion_jacobian<double>(bdash, xt, pa.sr, pa.alpha);
         for (int r = 0; r < 3; r++) {
             F[r] = xt[r] - 0.5 * a[r] * dt - px[r];
             for (int c = 0; c < 3; c++) F[r] -= 0.5 * b[3 * r + c] * dwm[c];
         }
         for (int r = 0; r < 3; r++)
             for (int c = 0; c < 3; c++) {
-                JT v = (JT)(r == c) - (JT)0.5 * adash[3 * r + c];
-                for (int k = 0; k < 3; k++) v -= (JT)0.5 * bdash[9 * r + 3 * k + c] * (JT)dwm[k];
+                double v = (double)(r == c) - 0.5 * adash[3 * r + c];
+                for (int k = 0; k < 3; k++) v -= 0.5 * bdash[9 * r + 3 * k + c] * dwm[k];
                 J[3 * r + c] = v;
             }
-        double sol[3] = {F[0] * -1, F[1] * -1, F[2] * -1};
-        for (int r = 0; r < 3; r++) x[r] = sol[r];
-        JT solj[3] = {(JT)sol[0], (JT)sol[1], (JT)sol[2]};
-        int info = M.active ? f64::solve3<JT>(J, solj) : 0;
+        for (int r = 0; r < 3; r++) x[r] = F[r] * -1;
+        double sol[3] = {x[0], x[1], x[2]};
+        int info = M.active ? f64::solve3<double>(J, sol) : 0;
         if (member_any(M, info != 0)) { flag = ST_SINGULAR; break; }
-        for (int r = 0; r < 3; r++) x[r] = (double)solj[r];
+        for (int r = 0; r < 3; r++) x[r] = sol[r];
         err = member_nrm2(M, x);
         for (int r = 0; r < 3; r++) x[r] += xt[r];
     }
     if (flag == ST_OK && iter == -1) flag = ST_NEWTON_MAXITER;
     for (int r = 0; r < 3; r++) x[r] = 2 * x[r] - px[r];
+    return flag;
+}
+
+// ---- implicit midpoint of the mixed-precision mode ----
+// The equation, its FP64 residual and state, the tolerance (eps times the norm
+// of the reference's first iterate) and the stopping test (|dx| <= tol over
+// the member, at most max_iter iterations) are those of implicit_step; the
+// dipolar sum is FP32 (dipolar32), and the iteration is steered by the
+// equation's own Jacobian instead of the reference's: that one writes the
+// drift term without dt (lib/integrators.cpp:633) and reads another
+// particle's block of the field Jacobian (lib/llg.cpp:386), contracts by
+// about one half per iteration and takes 27-40 of them a step, this one by
+// dt |D| (the dipolar coupling is left out of it) and takes 3.  FP64 costs 64
+// issue cycles a warp instruction here, so the step's length is the count of
+// its FP64 operations: iterations times ~60.  700 members of 13 particles, a
+// cluster each, dt = 2e-13: 100 steps (with the planning of the call) took
+// 35.2 ms with the reference's iteration, 5.8 ms with this one.
+
+// -(m x v) - alpha m x (m x v): drift and diffusion share this map
+// (lib/llg.cpp:14-29, :92-106), linear in v = dt h + sr dwm.
+__device__ inline void stage_map(double o[3], const double m[3], double alpha, const double v[3])
+{
+    double u[3], w[3];
+    u[0] = fma(m[1], v[2], -(m[2] * v[1]));
+    u[1] = fma(m[2], v[0], -(m[0] * v[2]));
+    u[2] = fma(m[0], v[1], -(m[1] * v[0]));
+    w[0] = fma(m[1], u[2], -(m[2] * u[1]));
+    w[1] = fma(m[2], u[0], -(m[0] * u[2]));
+    w[2] = fma(m[0], u[1], -(m[1] * u[0]));
+    for (int c = 0; c < 3; c++) o[c] = fma(-alpha, w[c], -u[c]);
+}
+
+// J = I - 1/2 d(stage_map)/dm in FP32, with v's own dependence on m through
+// the particle's anisotropy (k e e^T, times dt).
+__device__ inline void stage_jacobian(float J[9], const float m[3], float alpha, const float v[3],
+                                      const float e[3], float dtk)
+{
+    const float mv = __fmaf_rn(m[2], v[2], __fmaf_rn(m[1], v[1], m[0] * v[0]));
+    const float mm = __fmaf_rn(m[2], m[2], __fmaf_rn(m[1], m[1], m[0] * m[0]));
+    const float me = __fmaf_rn(m[2], e[2], __fmaf_rn(m[1], e[1], m[0] * e[0]));
+    // p = d(map)/dv e = -(m x e) - alpha (m (m.e) - e |m|^2), times dt k
+    const float cx[3] = {__fmaf_rn(m[1], e[2], -(m[2] * e[1])), __fmaf_rn(m[2], e[0], -(m[0] * e[2])),
+                         __fmaf_rn(m[0], e[1], -(m[1] * e[0]))};
+    float p[3];
+    for (int c = 0; c < 3; c++)
+        p[c] = dtk * __fmaf_rn(alpha, __fmaf_rn(mm, e[c], -(m[c] * me)), -cx[c]);
+    // d(map)/dm: [v]_x - alpha ((m.v) I + m v^T - 2 v m^T)
+    const float V[9] = {0.f, -v[2], v[1], v[2], 0.f, -v[0], -v[1], v[0], 0.f};
+    for (int r = 0; r < 3; r++)
+        for (int c = 0; c < 3; c++) {
+            float t = __fmaf_rn(m[r], v[c], -2.f * (v[r] * m[c])) + (r == c ? mv : 0.f);
+            t = __fmaf_rn(-alpha, t, V[3 * r + c]);
+            t = __fmaf_rn(p[r], e[c], t);
+            J[3 * r + c] = __fmaf_rn(-0.5f, t, r == c ? 1.f : 0.f);
+        }
+}
+
+// Member-wide FP32 sum, the same bits in every thread of the member.
+__device__ inline float member_sum32(const Member &M, float v)
+{
+    if (!M.ms.cta) {
+        const int lane = threadIdx.x & 31, first = lane - M.q;
+        for (int stride = M.p2 >> 1; stride >= 1; stride >>= 1) {
+            const float o = __shfl_sync(M.ms.mask, v, M.q + stride < M.n ? lane + stride : lane);
+            if (M.q + stride < M.n && M.q < stride) v += o;
+        }
+        return __shfl_sync(M.ms.mask, v, first);
+    }
+    float *red = (float *)M.red;
+    for (int d = 16; d >= 1; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    float s = 0.f;
+    for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += red[w];
+    __syncthreads();
+    return s;
+}
+__device__ inline double member_sum64(const Member &M, double v)
+{
+    if (!M.ms.cta) {
+        const int lane = threadIdx.x & 31, first = lane - M.q;
+        for (int stride = M.p2 >> 1; stride >= 1; stride >>= 1) {
+            const double o = __shfl_sync(M.ms.mask, v, M.q + stride < M.n ? lane + stride : lane);
+            if (M.q + stride < M.n && M.q < stride) v += o;
+        }
+        return __shfl_sync(M.ms.mask, v, first);
+    }
+    for (int d = 16; d >= 1; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+    if ((threadIdx.x & 31) == 0) M.red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double s = 0.0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += M.red[w];
+    __syncthreads();
+    return s;
+}
+
+// Stage increment dt a + B dwm at the state s, and its v.
+__device__ inline void stage32(const Member &M, const Particle &pa, const double s[3], double hz,
+                               const double sdw[3], double dt, double g[3], double v[3])
+{
+    double H[3] = {0.0, 0.0, 0.0};
+    if (M.d->interactions && M.n > 1) {
+        if (M.active) M.smf[M.q] = make_float4((float)s[0], (float)s[1], (float)s[2], 0.f);
+        M.ms.sync();
+        if (M.active) dipolar32(M, H);
+        M.ms.sync();
+    }
+    const double dot = pa.k * fma(s[2], pa.ax[2], fma(s[1], pa.ax[1], s[0] * pa.ax[0]));
+    v[0] = fma(dt, fma(dot, pa.ax[0], H[0]), sdw[0]);
+    v[1] = fma(dt, fma(dot, pa.ax[1], H[1]), sdw[1]);
+    v[2] = fma(dt, fma(dot, pa.ax[2], H[2] + hz), sdw[2]);
+    stage_map(g, s, pa.alpha, v);
+}
+
+__device__ int32_t implicit_step32(const Member &M, const Particle &pa, double x[3],
+                                   const double px[3], const double w[3], double t)
+{
+    const MemberDev &d = *M.d;
+    const double dt = d.dt, sq = d.sqrt_dt, Ah = d.Ah;
+    double sdw[3], g[3], v[3];
+    for (int c = 0; c < 3; c++) {
+        const double lo = (w[c] < Ah) ? w[c] : Ah;       // std::min(Ah, dw)
+        sdw[c] = pa.sr * (((-Ah < lo) ? lo : -Ah) * sq);  // std::max(-Ah, .) * sqrt(dt)
+    }
+    stage32(M, pa, px, f64::field_value(d.shape, t, d.happ, d.fapp), sdw, dt, g, v);
+    // the reference's first iterate (g + x0)/2 sets the tolerance; the
+    // iteration starts from the explicit midpoint x0 + g/2, whose error is of
+    // second order in the step
+    double s2 = 0.0;
+    for (int c = 0; c < 3; c++) {
+        const double r = 0.5 * (g[c] + px[c]);
+        s2 = fma(r, r, s2);
+        x[c] = fma(0.5, g[c], px[c]);
+    }
+    s2 = member_sum64(M, M.active ? s2 : 0.0);
+    const double tol2 = d.eps * d.eps * s2;
+    // FP32 bounds that decide the stopping test but for a narrow band, in
+    // which (and where FP32 could underflow) the FP64 norm is formed
+    const float far = (float)(tol2 * 1.0001), near = (float)(tol2 * 0.9999);
+    const bool fp32_ok = near > 1e-30f;
+    int64_t iter = d.max_iter;
+    int32_t flag = ST_OK;
+    const double hm = f64::field_value(d.shape, t + dt / 2, d.happ, d.fapp);
+    // err starts at 2 tol, as in the reference: no iteration for a tolerance
+    // of zero, below zero, infinite or NaN
+    bool going = d.eps > 0 && s2 > 0 && s2 < INFINITY;
+    const float ef[3] = {(float)pa.ax[0], (float)pa.ax[1], (float)pa.ax[2]};
+    const float dtk = (float)(dt * pa.k), alf = (float)pa.alpha;
+    while (going && (iter-- > 0)) {
+        stage32(M, pa, x, hm, sdw, dt, g, v);
+        // F = x - x0 - g/2 (lib/integrators.cpp:621-627), and J sol = -F
+        double mF[3];
+        float sol[3], J[9];
+        for (int c = 0; c < 3; c++) {
+            mF[c] = fma(0.5, g[c], px[c]) - x[c];
+            sol[c] = (float)mF[c];
+        }
+        const float mf[3] = {(float)x[0], (float)x[1], (float)x[2]};
+        const float vf[3] = {(float)v[0], (float)v[1], (float)v[2]};
+        stage_jacobian(J, mf, alf, vf, ef, dtk);
+        const int info = M.active ? f64::solve3<float>(J, sol) : 0;
+        if (member_any(M, info != 0)) {  // as implicit_step: x = -F is the result
+            for (int c = 0; c < 3; c++) x[c] = mF[c];
+            flag = ST_SINGULAR;
+            break;
+        }
+        float e32 = __fmaf_rn(sol[2], sol[2], __fmaf_rn(sol[1], sol[1], sol[0] * sol[0]));
+        e32 = member_sum32(M, M.active ? e32 : 0.f);
+        if (fp32_ok && e32 > far) {
+            going = true;
+        } else if (fp32_ok && e32 < near) {
+            going = false;
+        } else {
+            double e2 = 0.0;
+            for (int c = 0; c < 3; c++) e2 = fma((double)sol[c], (double)sol[c], e2);
+            e2 = member_sum64(M, M.active ? e2 : 0.0);
+            going = e2 > tol2;
+        }
+        for (int c = 0; c < 3; c++) x[c] += (double)sol[c];
+    }
+    if (flag == ST_OK && iter == -1) flag = ST_NEWTON_MAXITER;
+    for (int c = 0; c < 3; c++) x[c] = 2 * x[c] - px[c];
     return flag;
 }
 
@@ -245,7 +405,7 @@ __device__ int32_t implicit_step(const Member &M, const Particle &pa, double x[3
 template <bool IMPLICIT, bool DIP32, int MAXT>
 __global__ void __launch_bounds__(MAXT) sllg_fp64_kernel(DevPlan p)
 {
-    extern __shared__ double smem[];
+    extern __shared__ __align__(16) double smem[];
     const int n = p.n;
     int p2 = 1;
     while (p2 < n) p2 <<= 1;
@@ -273,8 +433,10 @@ __global__ void __launch_bounds__(MAXT) sllg_fp64_kernel(DevPlan p)
         M.ms.mask = (n == 32) ? 0xffffffffu : (((1u << n) - 1u) << (sub * n));
         M.sm = smem + (size_t)slot * slot_size;
     }
-    M.red = M.sm + 3 * n;
-    M.smf = (float *)(M.red + p2);
+    // FP64: moments then the reduction buffer; FP32 dipolar sum: float4
+    // moments (16-byte aligned: 2n doubles a member) then the buffer
+    M.red = M.sm + (DIP32 ? 2 * n : 3 * n);
+    M.smf = (float4 *)M.sm;
     M.n = n;
     M.p2 = p2;
     const MemberDev *md = p.members + e;
@@ -295,7 +457,7 @@ __global__ void __launch_bounds__(MAXT) sllg_fp64_kernel(DevPlan p)
     pa.k = p.k_red[g];
     pa.sr = p.sr[g];
     pa.alpha = md->alpha;
-    if (IMPLICIT)
+    if (IMPLICIT && !DIP32)
         for (int k = 0; k < 9; k++) pa.hj[k] = p.hj[k * P + g];
     const double scale = p.out_scale[e];
     const int64_t S = p.S;
@@ -330,8 +492,9 @@ __global__ void __launch_bounds__(MAXT) sllg_fp64_kernel(DevPlan p)
                 Normals4 r = wiener_normals(md->seed, step, (uint32_t)M.q);
                 w[0] = r.a; w[1] = r.b; w[2] = r.c;
             }
-            if (IMPLICIT) status |= implicit_step<DIP32>(M, pa, x, px, w, t);
-            else heun_step<DIP32>(M, pa, x, px, w, t);
+            if (DIP32) status |= implicit_step32(M, pa, x, px, w, t);
+            else if (IMPLICIT) status |= implicit_step(M, pa, x, px, w, t);
+            else heun_step(M, pa, x, px, w, t);
             if (md->renorm) {  // simulation.cpp:379-387
                 double s2 = 0.0;
                 s2 = s2 + x[0] * x[0];
@@ -375,13 +538,29 @@ cudaError_t launch_fp64(const DevPlan &p, cudaStream_t stream)
     const size_t slot = (size_t)slot_doubles(n, p2, dip32) * sizeof(double);
     dim3 grid, block;
     size_t shmem;
+    DevPlan q = p;  // with the members per warp filled in
     if (n > 32) {
         block = dim3(((n + 31) / 32) * 32);
         grid = dim3((unsigned)p.E);
         shmem = slot;
     } else {
-        const int mpw = (p.members_per_warp > 0 && p.members_per_warp < 32 / n) ? p.members_per_warp : 32 / n;
-        const int warps = p.block_warps > 0 ? p.block_warps : 4;
+        int mpw = (p.members_per_warp > 0 && p.members_per_warp < 32 / n) ? p.members_per_warp : 32 / n;
+        int warps = p.block_warps;
+        if (warps <= 0) {
+            // An FP64 warp instruction takes 64 cycles of its sub-partition
+            // however many lanes are active, and one warp fills that pipe: an
+            // ensemble that needs fewer warps than the chip has
+            // sub-partitions is spread over them one warp each (700 members of
+            // 13 particles, implicit: 350 warps in 88 CTAs of four warps keep
+            // 64 SMs idle), members apart where that costs no second warp.
+            // 10000 dimers, implicit: 8.7-9.2 ms in CTAs of four warps (five SMs
+            // take a second CTA), 6.5 ms in CTAs of one.
+            const int64_t subs = 4 * 152;
+            if (p.members_per_warp <= 0)
+                mpw = (int)std::min<int64_t>(32 / n, std::max<int64_t>(1, (p.E + subs - 1) / subs));
+            warps = (p.E + mpw - 1) / mpw <= 4 * subs ? 1 : 4;
+        }
+        q.members_per_warp = mpw;
         block = dim3(32 * warps);
         const int64_t per_block = (int64_t)warps * mpw;
         grid = dim3((unsigned)((p.E + per_block - 1) / per_block));
@@ -389,17 +568,17 @@ cudaError_t launch_fp64(const DevPlan &p, cudaStream_t stream)
     }
     const unsigned bt = block.x;
     if (p.use_implicit && dip32) {
-        if (bt <= 256) sllg_fp64_kernel<true, true, 256><<<grid, block, shmem, stream>>>(p);
-        else if (bt <= 512) sllg_fp64_kernel<true, true, 512><<<grid, block, shmem, stream>>>(p);
-        else sllg_fp64_kernel<true, true, 1024><<<grid, block, shmem, stream>>>(p);
+        if (bt <= 256) sllg_fp64_kernel<true, true, 256><<<grid, block, shmem, stream>>>(q);
+        else if (bt <= 512) sllg_fp64_kernel<true, true, 512><<<grid, block, shmem, stream>>>(q);
+        else sllg_fp64_kernel<true, true, 1024><<<grid, block, shmem, stream>>>(q);
     } else if (p.use_implicit) {
-        if (bt <= 256) sllg_fp64_kernel<true, false, 256><<<grid, block, shmem, stream>>>(p);
-        else if (bt <= 512) sllg_fp64_kernel<true, false, 512><<<grid, block, shmem, stream>>>(p);
-        else sllg_fp64_kernel<true, false, 1024><<<grid, block, shmem, stream>>>(p);
+        if (bt <= 256) sllg_fp64_kernel<true, false, 256><<<grid, block, shmem, stream>>>(q);
+        else if (bt <= 512) sllg_fp64_kernel<true, false, 512><<<grid, block, shmem, stream>>>(q);
+        else sllg_fp64_kernel<true, false, 1024><<<grid, block, shmem, stream>>>(q);
     } else {
-        if (bt <= 256) sllg_fp64_kernel<false, false, 256><<<grid, block, shmem, stream>>>(p);
-        else if (bt <= 512) sllg_fp64_kernel<false, false, 512><<<grid, block, shmem, stream>>>(p);
-        else sllg_fp64_kernel<false, false, 1024><<<grid, block, shmem, stream>>>(p);
+        if (bt <= 256) sllg_fp64_kernel<false, false, 256><<<grid, block, shmem, stream>>>(q);
+        else if (bt <= 512) sllg_fp64_kernel<false, false, 512><<<grid, block, shmem, stream>>>(q);
+        else sllg_fp64_kernel<false, false, 1024><<<grid, block, shmem, stream>>>(q);
     }
     return cudaGetLastError();
 }

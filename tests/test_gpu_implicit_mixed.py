@@ -1,0 +1,59 @@
+"""The mixed-precision implicit midpoint kernel and the launch shape of the
+warp-packed FP64 kernels."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _cluster(n, seed):
+    rng = np.random.default_rng(seed)
+    side = int(np.ceil(n ** (1 / 3)))
+    grid = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n]
+    axes = rng.normal(size=(n, 3))
+    axes /= np.linalg.norm(axes, axis=1, keepdims=True)
+    return np.full(n, 7e-9), grid * 20e-9 + rng.uniform(-5e-10, 5e-10, (n, 3)), axes
+
+
+def _args(n, E, steps, dt, implicit=True, seed=3):
+    radius, loc, axes = _cluster(n, seed)
+    return (E, radius, np.full(n, 2e4), axes, axes.copy(), loc, 4e5, 0.1, 300.0, False, True,
+            implicit, dt, dt * (steps - 0.5), 3, np.arange(E) + 5, "sine", 1e4, 3e5, 1e-9)
+
+
+@pytest.mark.parametrize("n,E", [(1, 3), (2, 1300), (13, 11), (16, 5), (31, 3), (32, 4), (33, 3),
+                                 (65, 2)])
+def test_mixed_implicit_same_root(gpu_lib, n, E):
+    """Both kernels stop within 1e-9 of the norm of the member's first iterate
+    (about sqrt(n)/2) of the same root, 2 y - x0 doubles it, and 40 steps add
+    up: 40 x 2 x 1e-9 x sqrt(n)/2 each, below 1e-6 for n <= 65; the FP32
+    dipolar sum adds about n 6e-8 |h| dt <= 1e-8 a step."""
+    from magpy_gb300 import core
+    a = core.simulate_ensemble(*_args(n, E, 40, 2e-13), precision="mixed")
+    b = core.simulate_ensemble(*_args(n, E, 40, 2e-13), precision="fp64")
+    assert np.all(a.status == 0) and np.array_equal(a.steps, b.steps)
+    for c in ("mx", "my", "mz"):
+        err = np.abs(getattr(a, c)[-1] - getattr(b, c)[-1]).max() / 4e5
+        assert err < 1.4e-6, (c, err)
+
+
+@pytest.mark.parametrize("n", [5, 40])
+def test_mixed_implicit_status(gpu_lib, n):
+    from magpy_gb300 import _lib, core
+    a = core.simulate_ensemble(*_args(n, 3, 4, 2e-13), precision="mixed", max_iter=1)
+    assert np.all(a.status & _lib.STATUS_NEWTON_MAXITER)
+    assert np.all(np.isfinite(a.mx))
+
+
+@pytest.mark.parametrize("n,E,implicit", [(2, 607, True), (2, 608, False), (3, 609, False),
+                                          (1, 1217, True), (11, 1300, False), (32, 700, False)])
+def test_fp64_launch_shape_is_free(gpu_lib, n, E, implicit):
+    """The members of a warp and the warps of a CTA do not enter a member's
+    arithmetic: bit-identical trajectories for the launcher's shape and for
+    fully packed warps."""
+    from magpy_gb300 import core
+    args = _args(n, E, 3, 1e-12 if implicit else 1e-13, implicit)
+    a = core.EnsemblePlan(*args).run().arrays()
+    b = core.EnsemblePlan(*args).set_launch(4, 0).run().arrays()
+    for c in ("mx", "my", "mz", "status", "steps"):
+        assert np.array_equal(getattr(a, c), getattr(b, c)), c
