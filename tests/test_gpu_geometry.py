@@ -108,3 +108,32 @@ def test_device_outputs_equal_host_outputs_and_feed_an_ensemble(gpu_lib):
                                  False, True, False, 5e-14, 5e-14 * 200, 3, seeds,
                                  per_member_geometry=True, precision="mixed")
     assert np.all(arr.status == 0)
+
+
+@pytest.mark.parametrize("n,members,packing", [(2, 1, 0.6), (33, 3, 0.3), (27, 700, 0.25)])
+def test_packing_takes_the_first_valid_candidate(gpu_lib, n, members, packing):
+    """Locations against a numpy statement of the packing (candidates in order,
+    the first valid one taken): the same candidates for narrow and wide
+    batches, to the rounding of the sphere's radius."""
+    from magpy_gb300 import core
+    g = core.generate_clusters(members, n, np.arange(members) + 40, sigma=0.3,
+                               packing_fraction=packing, spacing=2.1)
+    for e in range(0, members, max(1, members // 3)):
+        assert g["status"][e] == 0
+        r = g["radius"][e]
+        R = 0.5 * 2.1 * r.mean() * np.cbrt(n / packing)
+        pos = np.empty((0, 3))
+        for i in range(n):
+            for base in range(0, 1 << 20, 1024):
+                c = np.arange(base, base + 1024)
+                a, b = (philox4x32_10(np.full_like(c, i), c, np.full_like(c, tag),
+                                      np.full_like(c, 0x9E01), 40 + e, 0)
+                        for tag in (0x6E04, 0x6E05))
+                p = R * (2 * np.stack([_u53(a[0], a[1]), _u53(a[2], a[3]), _u53(b[0], b[1])], 1) - 1)
+                ok = np.sum(p * p, 1) <= R * R
+                for j in range(i):
+                    ok &= np.sum((p - pos[j]) ** 2, 1) >= (2.1 * 0.5 * (r[i] + r[j])) ** 2
+                if ok.any():
+                    pos = np.vstack([pos, p[np.argmax(ok)]])
+                    break
+        np.testing.assert_allclose(g["location"][e], pos, rtol=0, atol=1e-13 * R)
