@@ -171,5 +171,62 @@ __host__ __device__ inline int solve3(T a[9], T b[3])
     return 0;
 }
 
+#ifdef __CUDACC__
+// solve3<double> on the device, the same operations, with the pivots chosen
+// by comparing bits: an FP64 comparison costs as much as any FP64 instruction,
+// and the magnitudes of finite doubles order like their bits.  b is spoiled
+// where a pivot is zero (non-zero result).
+__device__ inline bool larger_mag(double x, double y)
+{
+    const int64_t m = 0x7fffffffffffffffll, inf = 0x7ff0000000000000ll;
+    const int64_t u = __double_as_longlong(x) & m, v = __double_as_longlong(y) & m;
+    if (u >= inf || v >= inf) return fabs(x) > fabs(y);
+    return u > v;
+}
+__device__ inline bool is_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
+
+__device__ inline int solve3_bits(double a[9], double b[3])
+{
+    auto swap_if = [](bool p, double &x, double &y) {
+        const double t = x;
+        x = p ? y : x;
+        y = p ? t : y;
+    };
+    const bool p1 = larger_mag(a[3], a[0]);
+    const bool p2 = larger_mag(a[6], p1 ? a[3] : a[0]);
+    for (int c = 0; c < 3; c++) {
+        swap_if(p1 && !p2, a[c], a[3 + c]);
+        swap_if(p2, a[c], a[6 + c]);
+    }
+    swap_if(p1 && !p2, b[0], b[1]);
+    swap_if(p2, b[0], b[2]);
+    if (is_zero(a[0])) return 1;
+    double l1 = a[3] / a[0], l2 = a[6] / a[0];
+    a[4] = a[4] - l1 * a[1];
+    a[5] = a[5] - l1 * a[2];
+    a[7] = a[7] - l2 * a[1];
+    a[8] = a[8] - l2 * a[2];
+    const bool p = larger_mag(a[7], a[4]);
+    swap_if(p, a[4], a[7]);
+    swap_if(p, a[5], a[8]);
+    swap_if(p, l1, l2);
+    swap_if(p, b[1], b[2]);
+    if (is_zero(a[4])) return 2;
+    const double l = a[7] / a[4];
+    a[8] = a[8] - l * a[5];
+    if (is_zero(a[8])) return 3;
+    b[1] = b[1] - b[0] * l1;
+    b[2] = b[2] - b[0] * l2;
+    b[2] = b[2] - b[1] * l;
+    b[2] = b[2] / a[8];
+    b[0] = b[0] - b[2] * a[2];
+    b[1] = b[1] - b[2] * a[5];
+    b[1] = b[1] / a[4];
+    b[0] = b[0] - b[1] * a[1];
+    b[0] = b[0] / a[0];
+    return 0;
+}
+#endif
+
 }  // namespace f64
 }  // namespace magpy

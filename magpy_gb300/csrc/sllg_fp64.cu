@@ -68,18 +68,79 @@ __device__ inline void dipolar32(const Member &M, double H[3])
     }
 }
 
+// 0.0 + x without an FP64 instruction: x, but +0 for -0.
+__device__ inline double plus_zero(double x)
+{
+    const bool mz = __double2hiint(x) == (int)0x80000000 && __double2loint(x) == 0;
+    return mz ? 0.0 : x;
+}
+
+// The applied field at a step's two evaluation times, t = step dt and t + dt
+// (Heun) or t + dt/2 (implicit midpoint).  An FP64 sine takes ~1300 cycles of
+// a warp, as much as 20 other FP64 instructions, and every lane of a warp
+// needs the same one when its members share their waveform and schedule: the
+// lanes then compute consecutive steps, one each, and hand them out by
+// shuffle.  (Same function, same argument, same bits.)  Members that do not
+// share compute their own.
+struct AppliedField {
+    double a, b;      // this lane's step of the block
+    int64_t base;     // steps before the block
+    unsigned mask;    // lanes that share, 0: none
+    int lanes;        // their number (they are lanes 0 .. lanes-1)
+
+    __device__ inline void init(const MemberDev &d, bool share)
+    {
+        mask = 0;
+        lanes = 0;
+        base = 0;
+        a = b = d.happ;  // constant field
+        if (d.shape == FIELD_CONSTANT || !share) return;
+        const unsigned act = __activemask();
+        if ((act & (act + 1)) == 0 && act != 1u) {
+            mask = act;
+            lanes = __popc(act);
+            base = -64;  // nothing computed yet
+        }
+    }
+    __device__ static inline double second(double t, double dt, bool half)
+    {
+        return half ? t + dt / 2 : t + dt;
+    }
+    template <bool HALF>
+    __device__ inline void at(const MemberDev &d, int64_t step, double &h1, double &h2)
+    {
+        if (d.shape == FIELD_CONSTANT) {
+            h1 = a;
+            h2 = b;
+        } else if (mask) {
+            int64_t i = step - 1 - base;
+            if (i >= lanes) {
+                base = step - 1;
+                i = 0;
+                const double t = (double)(step + (threadIdx.x & 31)) * d.dt;
+                a = f64::field_value(d.shape, t, d.happ, d.fapp);
+                b = f64::field_value(d.shape, second(t, d.dt, HALF), d.happ, d.fapp);
+            }
+            h1 = __shfl_sync(mask, a, (int)i);
+            h2 = __shfl_sync(mask, b, (int)i);
+        } else {
+            const double t = (double)step * d.dt;
+            h1 = f64::field_value(d.shape, t, d.happ, d.fapp);
+            h2 = f64::field_value(d.shape, second(t, d.dt, HALF), d.happ, d.fapp);
+        }
+    }
+};
+
 // Effective field of one particle: lib/simulation.cpp:271-290 (anisotropy,
 // lib/field.cpp:116-132; Zeeman along z, :81-88; dipolar pair sum, :187-225).
-__device__ void eff_field(const Member &M, const Particle &pa, double h[3], const double s[3],
-                          double t)
+__device__ inline void eff_field(const Member &M, const Particle &pa, double h[3],
+                                 const double s[3], double hz)
 {
-    h[0] = 0.0; h[1] = 0.0; h[2] = 0.0;
     double dot = s[0] * pa.ax[0] + s[1] * pa.ax[1] + s[2] * pa.ax[2];
     dot *= pa.k;
-    h[0] += dot * pa.ax[0];
-    h[1] += dot * pa.ax[1];
-    h[2] += dot * pa.ax[2];
-    h[2] += f64::field_value(M.d->shape, t, M.d->happ, M.d->fapp);
+    h[0] = plus_zero(dot * pa.ax[0]);
+    h[1] = plus_zero(dot * pa.ax[1]);
+    h[2] = plus_zero(dot * pa.ax[2]) + hz;
     if (M.d->interactions && M.n > 1) {
         if (M.active) {
             M.sm[3 * M.q + 0] = s[0];
@@ -106,26 +167,48 @@ __device__ void eff_field(const Member &M, const Particle &pa, double h[3], cons
     }
 }
 
-// Member-wide 2-norm with the shim's order: per-particle sequential sum of
-// squares, then a pairwise tree over a power-of-two padded particle index.
-__device__ double member_nrm2(const Member &M, const double x[3])
+// Square of the member-wide 2-norm with the shim's order: per-particle
+// sequential sum of squares, then a pairwise tree over a power-of-two padded
+// particle index (the padding's zeros are not added: the partial sums are
+// never -0).  The same bits in every thread of the member.
+__device__ inline double member_sumsq(const Member &M, const double x[3])
 {
-    if (M.active) {
-        double s = 0.0;
-        s = s + x[0] * x[0];
-        s = s + x[1] * x[1];
-        s = s + x[2] * x[2];
-        M.red[M.q] = s;
-        if (M.n + M.q < M.p2) M.red[M.n + M.q] = 0.0;
+    double s = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
+    if (!M.ms.cta) {
+        if (M.n == 1) return s;
+        const int lane = threadIdx.x & 31;
+        for (int stride = M.p2 >> 1; stride >= 1; stride >>= 1) {
+            const bool add = M.q < stride && M.q + stride < M.n;
+            const double o = __shfl_sync(M.ms.mask, s, add ? lane + stride : lane);
+            if (add) s = s + o;
+        }
+        return __shfl_sync(M.ms.mask, s, lane - M.q);
     }
+    if (M.active) M.red[M.q] = s;
     M.ms.sync();
     for (int stride = M.p2 / 2; stride >= 1; stride >>= 1) {
-        if (M.q < stride) M.red[M.q] = M.red[M.q] + M.red[M.q + stride];
+        if (M.q < stride && M.q + stride < M.n) M.red[M.q] = M.red[M.q] + M.red[M.q + stride];
         M.ms.sync();
     }
-    double r = sqrt(M.red[0]);
+    const double r = M.red[0];
     M.ms.sync();
     return r;
+}
+
+// sqrt(sq) > tol for tol > 0 and tol2 = tol * tol, without the root (~600
+// cycles) but within a few ulp of equality; comparisons of the bits, as doubles of one
+// sign order like integers (an FP64 comparison costs an FP64 instruction).
+__device__ inline bool norm_above(double sq, double tol, double tol2)
+{
+    const int64_t band = 16;  // ulp; sqrt, tol2 and the root's rounding are within 4
+    const int64_t inf = 0x7ff0000000000000ll;
+    const int64_t s = __double_as_longlong(sq), t = __double_as_longlong(tol2);
+    if (s > inf || s < 0) return false;                     // NaN
+    if (t > 0x0100000000000000ll && t < 0x7e00000000000000ll) {  // no underflow, no overflow
+        if (s > t + band) return true;
+        if (s < t - band) return false;
+    }
+    return sqrt(sq) > tol;
 }
 
 __device__ inline bool member_any(const Member &M, bool pred)
@@ -136,11 +219,11 @@ __device__ inline bool member_any(const Member &M, bool pred)
 
 // integrator::heun, lib/integrators.cpp:372-405, on the particle's 3x3 block.
 __device__ void heun_step(const Member &M, const Particle &pa, double x[3],
-                          const double px[3], const double w[3], double t)
+                          const double px[3], const double w[3], double hz1, double hz2)
 {
     const double dt = M.d->dt, sq = M.d->sqrt_dt;
     double h[3], a[3], b[9], xt[3];
-    eff_field(M, pa, h, px, t);
+    eff_field(M, pa, h, px, hz1);
     f64::drift(a, px, pa.alpha, h);
     f64::diffusion(b, px, pa.sr, pa.alpha);
     for (int r = 0; r < 3; r++) {
@@ -148,7 +231,7 @@ __device__ void heun_step(const Member &M, const Particle &pa, double x[3],
         for (int c = 0; c < 3; c++) xt[r] += b[3 * r + c] * w[c] * sq;
     }
     double ta[3], tb[9];
-    eff_field(M, pa, h, xt, t + dt);
+    eff_field(M, pa, h, xt, hz2);
     f64::drift(ta, xt, pa.alpha, h);
     f64::diffusion(tb, xt, pa.sr, pa.alpha);
     for (int r = 0; r < 3; r++) {
@@ -162,55 +245,132 @@ __device__ void heun_step(const Member &M, const Particle &pa, double x[3],
 // Jacobian is block-diagonal (the field Jacobian ignores the dipolar term,
 // lib/simulation.cpp:292-303), so the dense dgesv is n independent 3x3
 // solves; the convergence norm couples the whole member.
+//
+// What bounds it: the count of FP64 instructions (64 issue cycles each), 27-40
+// iterations a step.  So an iteration is written out with every product and
+// sum that llg::drift, llg::diffusion and their Jacobians (llg64.cuh) share
+// formed once, in their association, and with multiplications by powers of
+// two taken out, which round to the same bits: 0.5 b dwm is b (dwm/2),
+// 2 x y + z and d - 0.5 j are one fused operation with an exact product.  The
+// applied field is the step's, the root of the norm is avoided (norm_above),
+// comparisons are integer: about 335 FP64 instructions an iteration, 470 with
+// the functions called one by one (250 steps of one particle 86.9 -> 66.9 ms;
+// 10 steps of 10000 dimers 6.5 -> 5.3 ms).
 __device__ int32_t implicit_step(const Member &M, const Particle &pa, double x[3],
-                                 const double px[3], const double w[3], double t)
+                                 const double px[3], const double w[3], double hz1, double hz2)
 {
     const double dt = M.d->dt, sq = M.d->sqrt_dt, Ah = M.d->Ah;
-    double dwm[3];
-    for (int c = 0; c < 3; c++) {
-        double lo = (w[c] < Ah) ? w[c] : Ah;         // std::min(Ah, dw)
-        dwm[c] = ((-Ah < lo) ? lo : -Ah) * sq;       // std::max(-Ah, .) * sqrt(dt)
+    double hw[3];  // dwm / 2
+    double h[3];
+    {
+        double dwm[3], a[3], b[9];
+        for (int c = 0; c < 3; c++) {
+            double lo = (w[c] < Ah) ? w[c] : Ah;         // std::min(Ah, dw)
+            dwm[c] = ((-Ah < lo) ? lo : -Ah) * sq;       // std::max(-Ah, .) * sqrt(dt)
+            hw[c] = 0.5 * dwm[c];
+        }
+        eff_field(M, pa, h, px, hz1);
+        f64::drift(a, px, pa.alpha, h);
+        f64::diffusion(b, px, pa.sr, pa.alpha);
+        for (int r = 0; r < 3; r++) {
+            double g = a[r] * dt;
+            for (int c = 0; c < 3; c++) g += b[3 * r + c] * dwm[c];
+            x[r] = (g + px[r]) / 2;
+        }
     }
-    double h[3], a[3], b[9];
-    eff_field(M, pa, h, px, t);
-    f64::drift(a, px, pa.alpha, h);
-    f64::diffusion(b, px, pa.sr, pa.alpha);
-    for (int r = 0; r < 3; r++) {
-        double g = a[r] * dt;
-        for (int c = 0; c < 3; c++) g += b[3 * r + c] * dwm[c];
-        x[r] = (g + px[r]) / 2;
-    }
-    const double tol = M.d->eps * member_nrm2(M, x);
-    double err = 2 * tol;
+    const double tol = M.d->eps * sqrt(member_sumsq(M, x)), tol2 = tol * tol;
+    bool going = 2 * tol > tol;  // err starts at 2 tol
     int64_t iter = M.d->max_iter;
     int32_t flag = ST_OK;
-    const double tm = t + dt / 2;
-    while ((err > tol) && (iter-- > 0)) {
-        double xt[3] = {x[0], x[1], x[2]};
-        eff_field(M, pa, h, xt, tm);
-        f64::drift(a, xt, pa.alpha, h);
-        f64::diffusion(b, xt, pa.sr, pa.alpha);
-        double adash[9], bdash[27], J[9];
-        double F[3];
-        f64::drift_jacobian<double>(adash, xt, pa.alpha, h, pa.hj);
-        f64::diffusion_jacobian<double>(bdash, xt, pa.sr, pa.alpha);
-        for (int r = 0; r < 3; r++) {
-            F[r] = xt[r] - 0.5 * a[r] * dt - px[r];
-            for (int c = 0; c < 3; c++) F[r] -= 0.5 * b[3 * r + c] * dwm[c];
+    const double hdt = 0.5 * dt, al = pa.alpha, sr = pa.sr, asr = al * sr;
+    const double *j = pa.hj;
+    while (going && (iter-- > 0)) {
+        const double m0 = x[0], m1 = x[1], m2 = x[2];
+        eff_field(M, pa, h, x, hz2);
+        const double s00 = m0 * m0, s11 = m1 * m1, s22 = m2 * m2;
+        const double s12 = s11 + s22, s02 = s00 + s22, s01 = s00 + s11;
+        const double p0 = m0 * h[0], p1 = m1 * h[1], p2 = m2 * h[2];
+        const double q12 = p1 + p2, q02 = p0 + p2, q01 = p0 + p1;
+        const double m2h1 = m2 * h[1], m1h2 = m1 * h[2], m0h2 = m0 * h[2], m2h0 = m2 * h[0],
+                     m1h0 = m1 * h[0], m0h1 = m0 * h[1];
+        double F[3], J[9];
+        {
+            // F = x - 0.5 a dt - x0 - 0.5 B dwm
+            const double a0 = (m2h1 - m1h2) + al * (h[0] * s12 - m0 * q12);
+            const double a1 = (m0h2 - m2h0) + al * (h[1] * s02 - m1 * q02);
+            const double a2 = (m1h0 - m0h1) + al * (h[2] * s01 - m2 * q01);
+            const double am0 = al * m0, A01 = am0 * m1, A02 = am0 * m2, A12 = al * m1 * m2;
+            F[0] = (m0 - a0 * hdt) - px[0];
+            F[0] -= (asr * s12) * hw[0];
+            F[0] -= (sr * (m2 - A01)) * hw[1];
+            F[0] += (sr * (m1 + A02)) * hw[2];
+            F[1] = (m1 - a1 * hdt) - px[1];
+            F[1] += (sr * (m2 + A01)) * hw[0];
+            F[1] -= (asr * s02) * hw[1];
+            F[1] -= (sr * (m0 - A12)) * hw[2];
+            F[2] = (m2 - a2 * hdt) - px[2];
+            F[2] -= (sr * (m1 - A02)) * hw[0];
+            F[2] += (sr * (m0 + A12)) * hw[1];
+            F[2] -= (asr * s01) * hw[2];
         }
-        for (int r = 0; r < 3; r++)
-            for (int c = 0; c < 3; c++) {
-                double v = (double)(r == c) - 0.5 * adash[3 * r + c];
-                for (int k = 0; k < 3; k++) v -= 0.5 * bdash[9 * r + 3 * k + c] * dwm[k];
-                J[3 * r + c] = v;
-            }
-        for (int r = 0; r < 3; r++) x[r] = F[r] * -1;
-        double sol[3] = {x[0], x[1], x[2]};
-        int info = M.active ? f64::solve3<double>(J, sol) : 0;
-        if (member_any(M, info != 0)) { flag = ST_SINGULAR; break; }
-        for (int r = 0; r < 3; r++) x[r] = sol[r];
-        err = member_nrm2(M, x);
-        for (int r = 0; r < 3; r++) x[r] += xt[r];
+        {
+            // drift Jacobian a' (lib/llg.cpp:68-81) into J = I - 0.5 a'
+            const double m0j0 = m0 * j[0], m1j0 = m1 * j[0], m2j0 = m2 * j[0];
+            const double m0j3 = m0 * j[3], m1j3 = m1 * j[3], m2j3 = m2 * j[3];
+            const double m0j6 = m0 * j[6], m1j6 = m1 * j[6], m2j6 = m2 * j[6];
+            J[0] = (m2j3 - m1j6) + al * ((s12 * j[0] - q12) - m0 * (m1j3 + m2j6));
+            J[3] = ((h[2] - m2j0) + m0j6) +
+                   al * (fma(2.0, m0h1, s02 * j[3]) - m1 * ((h[0] + m0j0) + m2j6));
+            J[6] = ((m1j0 - h[1]) - m0j3) +
+                   al * (fma(2.0, m0h2, s01 * j[6]) - m2 * ((h[0] + m0j0) + m1j3));
+            const double m0j1 = m0 * j[1], m1j1 = m1 * j[1], m2j1 = m2 * j[1];
+            const double m0j4 = m0 * j[4], m1j4 = m1 * j[4], m2j4 = m2 * j[4];
+            const double m0j7 = m0 * j[7], m1j7 = m1 * j[7], m2j7 = m2 * j[7];
+            J[1] = ((m2j4 - h[2]) - m1j7) +
+                   al * (fma(2.0, m1h0, s12 * j[1]) - m0 * ((h[1] + m1j4) + m2j7));
+            J[4] = (m0j7 - m2j1) + al * ((s02 * j[4] - q02) - m1 * (m0j1 + m2j7));
+            J[7] = ((h[0] + m1j1) - m0j4) +
+                   al * (fma(2.0, m1h2, s01 * j[7]) - m2 * ((h[1] + m0j1) + m1j4));
+            const double m0j2 = m0 * j[2], m1j2 = m1 * j[2], m2j2 = m2 * j[2];
+            const double m0j5 = m0 * j[5], m1j5 = m1 * j[5], m2j5 = m2 * j[5];
+            const double m0j8 = m0 * j[8], m1j8 = m1 * j[8], m2j8 = m2 * j[8];
+            J[2] = ((h[1] + m2j5) - m1j8) +
+                   al * (fma(2.0, m2h0, s12 * j[2]) - m0 * ((h[2] + m1j5) + m2j8));
+            J[5] = ((-h[0] - m2j2) + m0j8) +
+                   al * (fma(2.0, m2h1, s02 * j[5]) - m1 * ((h[2] + m0j2) + m2j8));
+            J[8] = (m1j2 - m0j5) + al * ((s01 * j[8] - q01) - m2 * (m0j2 + m1j5));
+            for (int k = 0; k < 9; k++) J[k] = fma(-0.5, J[k], k % 4 == 0 ? 1.0 : 0.0);
+        }
+        {
+            // - 0.5 b'_k dwm_k (lib/llg.cpp:118-158), k = 0, 1, 2 in turn: b' has
+            // the entries +-sr, -asr m, 2 asr m and 0 (whose zero products
+            // change nothing: an entry of J is never -0)
+            const double c0 = asr * m0, c1 = asr * m1, c2 = asr * m2;
+            const double p00 = c0 * hw[0], p01 = c0 * hw[1], p02 = c0 * hw[2];
+            const double p10 = c1 * hw[0], p11 = c1 * hw[1], p12 = c1 * hw[2];
+            const double p20 = c2 * hw[0], p21 = c2 * hw[1], p22 = c2 * hw[2];
+            const double t0 = sr * hw[0], t1 = sr * hw[1], t2 = sr * hw[2];
+            J[0] = (J[0] + p11) + p22;
+            J[1] = (fma(-2.0, p10, J[1]) + p21) + t2;
+            J[2] = (fma(-2.0, p20, J[2]) - t1) + p02;
+            J[3] = fma(-2.0, p01, J[3] + p10) - t2;
+            J[4] = (J[4] + p00) + p22;
+            J[5] = fma(-2.0, p21, J[5] + t0) + p12;
+            J[6] = fma(-2.0, p02, (J[6] + p20) + t1);
+            J[7] = fma(-2.0, p22, (J[7] - t0) + p21);
+            J[8] = (J[8] + p00) + p11;
+        }
+        double sol[3] = {-F[0], -F[1], -F[2]};
+        int info = M.active ? f64::solve3_bits(J, sol) : 0;
+        if (member_any(M, info != 0)) {
+            flag = ST_SINGULAR;
+            x[0] = -F[0]; x[1] = -F[1]; x[2] = -F[2];
+            break;
+        }
+        going = norm_above(member_sumsq(M, sol), tol, tol2);
+        x[0] = sol[0] + m0;
+        x[1] = sol[1] + m1;
+        x[2] = sol[2] + m2;
     }
     if (flag == ST_OK && iter == -1) flag = ST_NEWTON_MAXITER;
     for (int r = 0; r < 3; r++) x[r] = 2 * x[r] - px[r];
@@ -329,7 +489,7 @@ __device__ inline void stage32(const Member &M, const Particle &pa, const double
 }
 
 __device__ int32_t implicit_step32(const Member &M, const Particle &pa, double x[3],
-                                   const double px[3], const double w[3], double t)
+                                   const double px[3], const double w[3], double hz1, double hz2)
 {
     const MemberDev &d = *M.d;
     const double dt = d.dt, sq = d.sqrt_dt, Ah = d.Ah;
@@ -338,7 +498,7 @@ __device__ int32_t implicit_step32(const Member &M, const Particle &pa, double x
         const double lo = (w[c] < Ah) ? w[c] : Ah;       // std::min(Ah, dw)
         sdw[c] = pa.sr * (((-Ah < lo) ? lo : -Ah) * sq);  // std::max(-Ah, .) * sqrt(dt)
     }
-    stage32(M, pa, px, f64::field_value(d.shape, t, d.happ, d.fapp), sdw, dt, g, v);
+    stage32(M, pa, px, hz1, sdw, dt, g, v);
     // the reference's first iterate (g + x0)/2 sets the tolerance; the
     // iteration starts from the explicit midpoint x0 + g/2, whose error is of
     // second order in the step
@@ -356,14 +516,13 @@ __device__ int32_t implicit_step32(const Member &M, const Particle &pa, double x
     const bool fp32_ok = near > 1e-30f;
     int64_t iter = d.max_iter;
     int32_t flag = ST_OK;
-    const double hm = f64::field_value(d.shape, t + dt / 2, d.happ, d.fapp);
     // err starts at 2 tol, as in the reference: no iteration for a tolerance
     // of zero, below zero, infinite or NaN
     bool going = d.eps > 0 && s2 > 0 && s2 < INFINITY;
     const float ef[3] = {(float)pa.ax[0], (float)pa.ax[1], (float)pa.ax[2]};
     const float dtk = (float)(dt * pa.k), alf = (float)pa.alpha;
     while (going && (iter-- > 0)) {
-        stage32(M, pa, x, hm, sdw, dt, g, v);
+        stage32(M, pa, x, hz2, sdw, dt, g, v);
         // F = x - x0 - g/2 (lib/integrators.cpp:621-627), and J sol = -F
         double mF[3];
         float sol[3], J[9];
@@ -470,6 +629,17 @@ __global__ void __launch_bounds__(MAXT) sllg_fp64_kernel(DevPlan p)
         p.my[g] = x[1] * scale;
         p.mz[g] = x[2] * scale;
     }
+    // lanes of a warp share the applied field where their members take the
+    // same steps through the same waveform
+    AppliedField af;
+    {
+        const unsigned act = __activemask();
+        const MemberDev *d0 = p.members + __shfl_sync(act, e, __ffs(act) - 1);
+        af.init(*md, __all_sync(act, md->dt == d0->dt && md->happ == d0->happ &&
+                                         md->fapp == d0->fapp && md->shape == d0->shape &&
+                                         md->sched_off == d0->sched_off &&
+                                         md->noise_len == d0->noise_len));
+    }
     int32_t status = ST_OK;
     uint64_t step = 0;
     int64_t s = 1;
@@ -478,7 +648,7 @@ __global__ void __launch_bounds__(MAXT) sllg_fp64_kernel(DevPlan p)
         while ((int64_t)step < ks) {
             px[0] = x[0]; px[1] = x[1]; px[2] = x[2];
             step++;
-            const double t = (double)step * md->dt;
+            double hz1, hz2;
             double w[3];
             if (noise) {
                 if ((int64_t)step * per_step > md->noise_len) {
@@ -492,9 +662,10 @@ __global__ void __launch_bounds__(MAXT) sllg_fp64_kernel(DevPlan p)
                 Normals4 r = wiener_normals(md->seed, step, (uint32_t)M.q);
                 w[0] = r.a; w[1] = r.b; w[2] = r.c;
             }
-            if (DIP32) status |= implicit_step32(M, pa, x, px, w, t);
-            else if (IMPLICIT) status |= implicit_step(M, pa, x, px, w, t);
-            else heun_step(M, pa, x, px, w, t);
+            af.at<IMPLICIT>(*md, (int64_t)step, hz1, hz2);
+            if (DIP32) status |= implicit_step32(M, pa, x, px, w, hz1, hz2);
+            else if (IMPLICIT) status |= implicit_step(M, pa, x, px, w, hz1, hz2);
+            else heun_step(M, pa, x, px, w, hz1, hz2);
             if (md->renorm) {  // simulation.cpp:379-387
                 double s2 = 0.0;
                 s2 = s2 + x[0] * x[0];

@@ -57,3 +57,24 @@ def test_fp64_launch_shape_is_free(gpu_lib, n, E, implicit):
     b = core.EnsemblePlan(*args).set_launch(4, 0).run().arrays()
     for c in ("mx", "my", "mz", "status", "steps"):
         assert np.array_equal(getattr(a, c), getattr(b, c)), c
+
+
+@pytest.mark.parametrize("n,implicit", [(1, True), (3, False), (33, True)])
+@pytest.mark.parametrize("shape", ["sine", "square"])
+def test_shared_applied_field(gpu_lib, n, implicit, shape):
+    """Lanes compute the applied field of consecutive steps for each other only
+    where all members of their warp share it: members beside one of another
+    frequency (who compute their own) take the same bits; 70 steps cross a
+    block of 32."""
+    from magpy_gb300 import core
+    E = 40
+    args = list(_args(n, E, 70, 1e-12 if implicit else 1e-13, implicit))
+    args[16] = shape
+    f = np.full(E, 3e5)
+    a = core.simulate_ensemble(*args, per_member={"field_frequency": f})
+    f[::7] = 4e9
+    b = core.simulate_ensemble(*args, per_member={"field_frequency": f})
+    same = np.repeat(f == 3e5, n)
+    for c in ("mx", "my", "mz"):
+        assert np.array_equal(getattr(a, c)[:, same], getattr(b, c)[:, same])
+        assert not np.array_equal(getattr(a, c)[:, ~same], getattr(b, c)[:, ~same])
