@@ -403,6 +403,7 @@ int make_plan(const std::vector<const Reduced *> &members, const std::vector<uin
     p.n = (int32_t)n;
     p.use_implicit = use_implicit;
     p.shared_cluster = shared ? 1 : 0;
+    p.one_schedule = sched_of.size() <= 1 ? 1 : 0;
     int rc;
     if ((rc = upload(b[0], md, st, &p.members))) return rc;
     if (shared) {
@@ -1389,6 +1390,8 @@ extern "C" int magpy_batch_create(const magpy_ensemble_desc *groups, int64_t n_g
                     if (full >= 4) mpws.push_back(full / 4);
                     if (full > 1) mpws.push_back(1);
                     shapes.clear();
+                    // the launcher's own choice, which may take another kernel
+                    if (!mixed) shapes.push_back({0, 0});
                     for (int32_t w : {1, 2, 4, 8})
                         for (int32_t m : mpws) shapes.push_back({w, m});
                 }

@@ -21,6 +21,7 @@ struct DevPlan {
     int32_t members_per_warp = 0; // members packed per warp (n <= 32); 0: as many as fit;
                                   // n > 32, mixed precision: members per CTA (1, 2 or 4)
     int32_t shared_cluster = 0;   // every member has the same cluster and parameters
+    int32_t one_schedule = 0;     // every member takes the same steps and samples
     uint32_t wait_limit = 1u << 24; // polls of a tensor-core phase wait before the watchdog
                                     // status (the final drain keeps its own long bound)
     const MemberDev *members = nullptr;
@@ -51,6 +52,10 @@ void pool_trim(int device);
 
 // Launchers (one translation unit each).
 cudaError_t launch_fp64(const DevPlan &p, cudaStream_t stream);
+// FP64-faithful kernel for small ensembles of small clusters: several lanes
+// per particle (sllg_fp64_lanes.cu).
+bool fp64_lanes_fit(const DevPlan &p);
+cudaError_t launch_fp64_lanes(const DevPlan &p, cudaStream_t stream);
 cudaError_t launch_mixed(const DevPlan &p, cudaStream_t stream);
 // Builds the FP32 pair table (from p.pt / p.rt, `clusters` tables of n*n)
 // and the per-step field table for a launch whose members share one

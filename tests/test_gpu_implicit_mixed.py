@@ -45,18 +45,50 @@ def test_mixed_implicit_status(gpu_lib, n):
     assert np.all(np.isfinite(a.mx))
 
 
-@pytest.mark.parametrize("n,E,implicit", [(2, 607, True), (2, 608, False), (3, 609, False),
-                                          (1, 1217, True), (11, 1300, False), (32, 700, False)])
+@pytest.mark.parametrize("n,E,implicit", [
+    # several lanes per particle, its Newton matrix over 16 or 4 lanes
+    (1, 1, True), (1, 1215, True), (1, 1217, True), (2, 607, True), (2, 609, True), (3, 5, True),
+    (5, 608, True), (8, 3, True), (1, 1, False), (1, 9729, False), (2, 608, False),
+    (3, 609, False), (7, 100, False), (8, 1216, False),
+    # past them: one thread per particle
+    (8, 609, True), (8, 1217, False), (1, 4865, True), (11, 1300, False), (32, 700, False)])
 def test_fp64_launch_shape_is_free(gpu_lib, n, E, implicit):
-    """The members of a warp and the warps of a CTA do not enter a member's
-    arithmetic: bit-identical trajectories for the launcher's shape and for
-    fully packed warps."""
+    """The lanes of a particle, the members of a warp and the warps of a CTA do
+    not enter a member's arithmetic: bit-identical trajectories for the
+    launcher's choice and for one thread per particle in fully packed warps."""
     from magpy_gb300 import core
     args = _args(n, E, 3, 1e-12 if implicit else 1e-13, implicit)
     a = core.EnsemblePlan(*args).run().arrays()
     b = core.EnsemblePlan(*args).set_launch(4, 0).run().arrays()
     for c in ("mx", "my", "mz", "status", "steps"):
         assert np.array_equal(getattr(a, c), getattr(b, c)), c
+
+
+@pytest.mark.parametrize("n,implicit", [(1, True), (2, True), (3, True), (8, False)])
+def test_fp64_lanes_special_members(gpu_lib, n, implicit):
+    """Members beside one that hits the iteration limit, that starts from NaN,
+    or without noise and off the field's axis (exact zeros): as with one thread
+    per particle."""
+    from magpy_gb300 import core
+    E = 9
+    radius, loc, axes = _cluster(n, 3)
+    m0 = np.tile(axes, (E, 1)).reshape(E, n, 3)
+    axes = m0.copy()
+    m0[1, 0] = np.nan
+    axes[2] = m0[2] = [0.0, 0.0, 1.0]
+    axes[3] = m0[3] = [-1.0, 0.0, 0.0]
+    tile = lambda v: np.concatenate([v] * E)  # noqa: E731
+    T = np.full(E, 300.0)
+    T[2:4] = 0.0
+    for renorm, max_iter in ((False, 1000), (True, 7)):
+        args = (E, tile(radius), np.full(E * n, 2e4), axes, m0, tile(loc), 4e5, 0.1, 300.0, renorm,
+                True, implicit, 1e-12, 1e-12 * 39.5, 4, np.arange(E), "square", 1e4, 1e10, 1e-9)
+        kw = dict(per_member_geometry=True, per_member={"temperature": T}, max_iter=max_iter)
+        a = core.EnsemblePlan(*args, **kw).run().arrays()
+        b = core.EnsemblePlan(*args, **kw).set_launch(4, 0).run().arrays()
+        for c in ("mx", "my", "mz", "status", "steps"):
+            np.testing.assert_array_equal(getattr(a, c), getattr(b, c))
+        assert a.status[1] & 4 and np.all(a.status[4:] == (1 if implicit and max_iter == 7 else 0))
 
 
 @pytest.mark.parametrize("n,implicit", [(1, True), (3, False), (33, True)])
@@ -72,7 +104,7 @@ def test_shared_applied_field(gpu_lib, n, implicit, shape):
     args[16] = shape
     f = np.full(E, 3e5)
     a = core.simulate_ensemble(*args, per_member={"field_frequency": f})
-    f[::7] = 4e9
+    f[::7] = 4e11  # half periods of 1.25 ps: the square wave turns within the run
     b = core.simulate_ensemble(*args, per_member={"field_frequency": f})
     same = np.repeat(f == 3e5, n)
     for c in ("mx", "my", "mz"):
