@@ -899,6 +899,7 @@ int magpy_dom_dynamics(const magpy_dom_desc *d, double *mz, double *field, doubl
 
     std::vector<DomMember> hm(E);
     std::vector<std::pair<double, int64_t>> key(E);
+    const double step_rate = std::min(3.3, 0.5 * std::pow(d->time_step / 1e-10, 0.2));
     for (int64_t e = 0; e < E; e++) {
         DomMember &m = hm[e];
         m.v = d->volume[e];
@@ -911,18 +912,31 @@ int magpy_dom_dynamics(const magpy_dom_desc *d, double *mz, double *field, doubl
         m.f = d->field_frequency[e];
         m.p0 = d->initial_probabilities[2 * e];
         m.p1 = d->initial_probabilities[2 * e + 1];
-        // launch order: by the zero-field relaxation rate, the main driver of
-        // the step count, fastest (most steps) first, so that a warp's
-        // particles take similar step counts and the heavy warps start first
+        // launch order: by the expected step count, largest first, so that a
+        // warp's particles take similar step counts and the heavy warps start
+        // first.  The step is end/1000 at most and about x over the relaxation
+        // rate where that is less; x = 0.5 (tolerance / 1e-10)^(1/5) fits the
+        // step counts of sigma = 1.3 .. 5 at a tolerance of 1e-10 (2490 .. 1008
+        // steps), 3.3 is the scheme's stability limit.  The rate is largest
+        // near the field's amplitude (lib/dom.cpp:33-59).
         const double sigma = m.k * m.v / KB / m.T;
         const double taun = m.v * m.ms * (1 + m.alpha * m.alpha) / 2.0 / GYROMAG / m.alpha / KB /
                             m.T;
-        const double lr = -sigma + 1.5 * std::log(sigma) - std::log(taun * std::sqrt(M_PI));
-        key[e] = {std::isfinite(lr) ? -lr : 1e300, e};
+        const double h = std::abs(m.h) * (d->field_shape == MAGPY_FIELD_SINE ? 0.85 : 1.0);
+        const double rate = sigma * std::sqrt(sigma) / (taun * std::sqrt(M_PI)) * (1 - h * h) *
+                            ((1 - h) * std::exp(-sigma * (1 - h) * (1 - h)) +
+                             (1 + h) * std::exp(-sigma * (1 + h) * (1 + h)));
+        const double steps = rate * d->end_time / 1000.0 / step_rate;
+        key[e] = {std::isfinite(steps) ? -std::max(1.0, steps) : -1e3, e};
+        if (steps < 1.0) key[e].first = -1.0 + 1e-9 * (1.0 - steps);  // ties in rate order
     }
     std::sort(key.begin(), key.end());
     std::vector<int64_t> order(E);
-    for (int64_t e = 0; e < E; e++) order[e] = key[e].second;
+    std::vector<double> expected(E);
+    for (int64_t e = 0; e < E; e++) {
+        order[e] = key[e].second;
+        expected[e] = -key[e].first;
+    }
 
     cudaStream_t st = (cudaStream_t)stream;
     const size_t EN = (size_t)E * (size_t)N;
@@ -942,6 +956,7 @@ int magpy_dom_dynamics(const magpy_dom_desc *d, double *mz, double *field, doubl
     a.N = N;
     a.members = (const DomMember *)bm.p;
     a.order = (const int64_t *)bo.p;
+    a.lanes = dom_lanes_rule(expected.data(), E);
     a.shape = d->field_shape;
     a.ncomp = d->field_n_components;
     a.time_step = d->time_step;

@@ -115,6 +115,7 @@ struct DomArgs {
     int64_t E = 0, N = 0;       // particles, samples per particle
     const DomMember *members = nullptr;
     const int64_t *order = nullptr;  // launch order of the particles, or null
+    int64_t lanes = 0;               // particles, first in that order, with five lanes each
     int32_t shape = 2;
     int64_t ncomp = 1;
     double time_step = 0, end_time = 0, sampling_time = 0;
@@ -124,6 +125,9 @@ struct DomArgs {
     int64_t *steps = nullptr;
 };
 cudaError_t launch_dom(const DomArgs &a, cudaStream_t stream);
+// How many of E particles, in descending order of their expected relative step
+// counts, get five lanes.
+int64_t dom_lanes_rule(const double *steps, int64_t E);
 // Seeded cluster geometry (geometry.cu): one CTA per member.
 struct GeoArgs {
     int64_t E = 0;
