@@ -114,9 +114,10 @@ __device__ __forceinline__ double mul_int(double a, double b)
     const uint32_t e = (ah & 0x7ff00000u) + (bh & 0x7ff00000u) - (1023u << 20) - (sh << 20);
     // half the last place rounds up with an odd mantissa: carry of the rest
     const uint32_t half = (ml & 1u) + 0x7fffffffu;
-    uint32_t carry, rl, rh;
-    asm("add.cc.u32 %0, %3, %4;\n\taddc.cc.u32 %1, %5, 0;\n\taddc.u32 %2, %6, %7;"
-        : "=r"(carry), "=r"(rl), "=r"(rh)
+    uint32_t rl, rh;
+    asm("{\n\t.reg .u32 t;\n\tadd.cc.u32 t, %2, %3;\n\taddc.cc.u32 %0, %4, 0;\n\t"
+        "addc.u32 %1, %5, %6;\n\t}"
+        : "=r"(rl), "=r"(rh)
         : "r"(rest), "r"(half), "r"(ml), "r"(mh), "r"(e));
     const bool zero = (int)e < (256 << 20);
     rl = zero ? 0u : rl;

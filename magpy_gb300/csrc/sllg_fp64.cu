@@ -13,6 +13,7 @@
 #include <algorithm>
 #include "common.cuh"
 #include "fp64_common.cuh"
+#include "implicit32.cuh"
 #include "llg64.cuh"
 #include "plan.hpp"
 
@@ -71,9 +72,10 @@ __device__ inline void dipolar32(const Member &M, double H[3])
             h1 = __fmaf_rn(r.w, __fmaf_rn(d3, r.y, -mj.y), h1);
             h2 = __fmaf_rn(r.w, __fmaf_rn(d3, r.z, -mj.z), h2);
         }
-        H[0] += (double)h0;
-        H[1] += (double)h1;
-        H[2] += (double)h2;
+        const double d0 = widen(h0), d1 = widen(h1), d2 = widen(h2);
+        H[0] = j0 ? H[0] + d0 : d0;
+        H[1] = j0 ? H[1] + d1 : d1;
+        H[2] = j0 ? H[2] + d2 : d2;
     }
 }
 
@@ -343,45 +345,6 @@ __device__ int32_t implicit_step(const Member &M, const Particle &pa, double x[3
 // cluster each, dt = 2e-13: 100 steps (with the planning of the call) took
 // 35.2 ms with the reference's iteration, 5.8 ms with this one.
 
-// -(m x v) - alpha m x (m x v): drift and diffusion share this map
-// (lib/llg.cpp:14-29, :92-106), linear in v = dt h + sr dwm.
-__device__ inline void stage_map(double o[3], const double m[3], double alpha, const double v[3])
-{
-    double u[3], w[3];
-    u[0] = fma(m[1], v[2], -(m[2] * v[1]));
-    u[1] = fma(m[2], v[0], -(m[0] * v[2]));
-    u[2] = fma(m[0], v[1], -(m[1] * v[0]));
-    w[0] = fma(m[1], u[2], -(m[2] * u[1]));
-    w[1] = fma(m[2], u[0], -(m[0] * u[2]));
-    w[2] = fma(m[0], u[1], -(m[1] * u[0]));
-    for (int c = 0; c < 3; c++) o[c] = fma(-alpha, w[c], -u[c]);
-}
-
-// J = I - 1/2 d(stage_map)/dm in FP32, with v's own dependence on m through
-// the particle's anisotropy (k e e^T, times dt).
-__device__ inline void stage_jacobian(float J[9], const float m[3], float alpha, const float v[3],
-                                      const float e[3], float dtk)
-{
-    const float mv = __fmaf_rn(m[2], v[2], __fmaf_rn(m[1], v[1], m[0] * v[0]));
-    const float mm = __fmaf_rn(m[2], m[2], __fmaf_rn(m[1], m[1], m[0] * m[0]));
-    const float me = __fmaf_rn(m[2], e[2], __fmaf_rn(m[1], e[1], m[0] * e[0]));
-    // p = d(map)/dv e = -(m x e) - alpha (m (m.e) - e |m|^2), times dt k
-    const float cx[3] = {__fmaf_rn(m[1], e[2], -(m[2] * e[1])), __fmaf_rn(m[2], e[0], -(m[0] * e[2])),
-                         __fmaf_rn(m[0], e[1], -(m[1] * e[0]))};
-    float p[3];
-    for (int c = 0; c < 3; c++)
-        p[c] = dtk * __fmaf_rn(alpha, __fmaf_rn(mm, e[c], -(m[c] * me)), -cx[c]);
-    // d(map)/dm: [v]_x - alpha ((m.v) I + m v^T - 2 v m^T)
-    const float V[9] = {0.f, -v[2], v[1], v[2], 0.f, -v[0], -v[1], v[0], 0.f};
-    for (int r = 0; r < 3; r++)
-        for (int c = 0; c < 3; c++) {
-            float t = __fmaf_rn(m[r], v[c], -2.f * (v[r] * m[c])) + (r == c ? mv : 0.f);
-            t = __fmaf_rn(-alpha, t, V[3 * r + c]);
-            t = __fmaf_rn(p[r], e[c], t);
-            J[3 * r + c] = __fmaf_rn(-0.5f, t, r == c ? 1.f : 0.f);
-        }
-}
-
 // Member-wide FP32 sum, the same bits in every thread of the member.
 __device__ inline float member_sum32(const Member &M, float v)
 {
@@ -427,7 +390,7 @@ __device__ inline void stage32(const Member &M, const Particle &pa, const double
 {
     double H[3] = {0.0, 0.0, 0.0};
     if (M.d->interactions && M.n > 1) {
-        if (M.active) M.smf[M.q] = make_float4((float)s[0], (float)s[1], (float)s[2], 0.f);
+        if (M.active) M.smf[M.q] = make_float4(narrow(s[0]), narrow(s[1]), narrow(s[2]), 0.f);
         M.ms.sync();
         if (M.active) dipolar32(M, H);
         M.ms.sync();
@@ -470,6 +433,8 @@ __device__ int32_t implicit_step32(const Member &M, const Particle &pa, double x
     // err starts at 2 tol, as in the reference: no iteration for a tolerance
     // of zero, below zero, infinite or NaN
     bool going = d.eps > 0 && s2 > 0 && s2 < INFINITY;
+    if (!going)  // the result is the reference's first iterate
+        for (int c = 0; c < 3; c++) x[c] = fma(-0.5, px[c], x[c]);
     const float ef[3] = {(float)pa.ax[0], (float)pa.ax[1], (float)pa.ax[2]};
     const float dtk = (float)(dt * pa.k), alf = (float)pa.alpha;
     while (going && (iter-- > 0)) {
@@ -479,10 +444,10 @@ __device__ int32_t implicit_step32(const Member &M, const Particle &pa, double x
         float sol[3], J[9];
         for (int c = 0; c < 3; c++) {
             mF[c] = fma(0.5, g[c], px[c]) - x[c];
-            sol[c] = (float)mF[c];
+            sol[c] = narrow(mF[c]);
         }
-        const float mf[3] = {(float)x[0], (float)x[1], (float)x[2]};
-        const float vf[3] = {(float)v[0], (float)v[1], (float)v[2]};
+        const float mf[3] = {narrow(x[0]), narrow(x[1]), narrow(x[2])};
+        const float vf[3] = {narrow(v[0]), narrow(v[1]), narrow(v[2])};
         stage_jacobian(J, mf, alf, vf, ef, dtk);
         const int info = M.active ? f64::solve3<float>(J, sol) : 0;
         if (member_any(M, info != 0)) {  // as implicit_step: x = -F is the result
@@ -502,7 +467,7 @@ __device__ int32_t implicit_step32(const Member &M, const Particle &pa, double x
             e2 = member_sum64(M, M.active ? e2 : 0.0);
             going = e2 > tol2;
         }
-        for (int c = 0; c < 3; c++) x[c] += (double)sol[c];
+        for (int c = 0; c < 3; c++) x[c] += widen(sol[c]);
     }
     if (flag == ST_OK && iter == -1) flag = ST_NEWTON_MAXITER;
     for (int c = 0; c < 3; c++) x[c] = 2 * x[c] - px[c];

@@ -39,6 +39,7 @@
 #include <algorithm>
 #include <cuda_fp16.h>
 #include "common.cuh"
+#include "implicit32.cuh"
 #include "llg32.cuh"
 #include "llg64.cuh"
 #include "plan.hpp"
@@ -800,51 +801,45 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
 // product are computed and not used), so each member takes the iterations
 // the per-member loop would.  State, increments, residual and the
 // convergence norms are FP64; the dipolar field comes from the tensor cores
-// (~22 significant bits) and the quasi-Jacobian and its 3x3 solves are FP32,
-// as in the mixed implicit mode of the CUDA-core kernel.  The Newton
-// equation, its FP64 residual and the stopping test (|dx| <= eps |guess|,
-// member-wide, at most max_iter iterations) are the reference's; the
-// Jacobian that steers it is J = I - dt a'/2 - sum_k b'_k dwm_k / 2 with each
-// particle's own anisotropy field Jacobian k e e^T and without the dipolar
-// coupling (block-diagonal).  The reference writes the drift term without dt
-// (integrators.cpp:633) and hands llg::drift_jacobian another particle's
-// block of the field Jacobian (llg.cpp:386); its iteration then contracts by
-// ~1/2 per step and needs ~40 iterations per step at dt = 2e-13 s, this one
-// by ~dt |D| and a few.  Both converge to the same root within the same
-// tolerance (the FP64-faithful kernel keeps the reference's iteration).  The member-wide norms are summed
-// over the CTA's particles in a fixed order, then over the cluster's CTAs in
-// rank order through distributed shared memory: every CTA takes the same
-// decisions from the same numbers.
+// (~22 significant bits) and the Jacobian and its 3x3 solves are FP32, as in
+// the mixed implicit mode of the CUDA-core kernel.  The Newton equation, its
+// FP64 residual, the tolerance (eps times the norm of the reference's first
+// iterate) and the stopping test (|dx| <= tol, member-wide, at most max_iter
+// iterations) are the reference's; the iteration starts from the explicit
+// midpoint and is steered by the equation's own Jacobian without the dipolar
+// coupling (implicit32.cuh: block-diagonal, contracts by ~dt |D|).  The
+// reference writes the drift term without dt (integrators.cpp:633) and hands
+// llg::drift_jacobian another particle's block of the field Jacobian
+// (llg.cpp:386); its iteration contracts by ~1/2 and needs ~40 iterations a
+// step at dt = 2e-13 s.  Both converge to the same root within the same
+// tolerance (the FP64-faithful kernel keeps the reference's iteration).  The
+// member-wide norms are summed over the CTA's particles in a fixed order, then
+// over the cluster's CTAs in rank order through distributed shared memory:
+// every CTA takes the same decisions from the same numbers.
 //
-// Stage increments use dt a + B dwm = F(m, dt h + sr dwm), the LLG map of
-// llg32.cuh in FP64 (drift and diffusion share the form).
-__device__ inline void llg_F64(double o[3], const double m[3], double alpha, const double v[3])
-{
-    const double c0 = m[1] * v[2] - m[2] * v[1];
-    const double c1 = m[2] * v[0] - m[0] * v[2];
-    const double c2 = m[0] * v[1] - m[1] * v[0];
-    const double mv = m[0] * v[0] + m[1] * v[1] + m[2] * v[2];
-    const double mm = m[0] * m[0] + m[1] * m[1] + m[2] * m[2];
-    o[0] = fma(alpha, v[0] * mm - m[0] * mv, -c0);
-    o[1] = fma(alpha, v[1] * mm - m[1] * mv, -c1);
-    o[2] = fma(alpha, v[2] * mm - m[2] * mv, -c2);
-}
+// What bounds it: the FP64 pipe (two lanes a clock an SM), on which conversions
+// run too.  A particle's iteration is 35 FP64 instructions (stage increments
+// dt a + B dwm = F(m, dt h + sr dwm), the residual, the update), its
+// conversions are integer (narrow, widen), its share of the stopping norm is
+// summed as float-float (exact squares), and starting from the explicit
+// midpoint saves one iteration of four.  512 members of 512 particles, 40
+// steps: 18.0 -> 12.8 ms.
 
 // Per-particle constants of a CTA's 42 particles: FP64 for the residual,
 // FP32 copies for the Jacobian.
 struct ImpPar {
     double ax[PPC][3], k[PPC], sr[PPC];
-    float axf[PPC][3], kf[PPC], srf[PPC], hjf[PPC][9];
+    float axf[PPC][3], dtk[PPC];
 };
 
 __host__ __device__ inline size_t tcc_imp_smem(const TccLayout &L)
 {
     // after the Heun layout: particle constants, per-(p0, member) partial
     // sums, and the cluster-exchanged partials / flags (double-buffered)
-    // ... and, in the 32- and 40-member forms, each particle's step increments kept
-    // for the Newton iterations: sr dwm (FP64) and dwm (FP32), 3 each
+    // ... and, in the 32- and 40-member forms, each particle's step increments
+    // sr dwm kept for the Newton iterations
     const size_t kept =
-        L.nb <= 40 ? (size_t)(8 + 4) * 3 * 2 * ITEMS * (PAIRS * (size_t)L.nb / ITEMS) : 0;
+        L.nb <= 40 ? (size_t)8 * 3 * 2 * ITEMS * (PAIRS * (size_t)L.nb / ITEMS) : 0;
     return tcc_up(L.total, 16) + sizeof(ImpPar) + (size_t)8 * 7 * L.nb + (size_t)8 * 2 * L.nb +
            (size_t)4 * 2 * L.nb + (size_t)8 * L.nb + (size_t)4 * L.nb + 64 + kept;
 }
@@ -872,12 +867,11 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
     double *sNorm = (double *)(pflag + 2 * NB);               // [NB] combined norm
     int *sSing = (int *)(sNorm + NB);                         // [NB] combined singular flag
     double *sField = (double *)(sSing + NB);                  // applied field at t, t + dt/2
-    // 32-member form: the step's sr dwm (FP64) and dwm (FP32) per particle,
+    // 32- and 40-member forms: the step's sr dwm per particle,
     // [(i*2 + k)*3 + c][IT], written at the initial guess, read by the
-    // Newton iterations (the larger forms recompute them)
+    // Newton iterations (the larger form recomputes them)
     constexpr bool KEEP_DW = NB <= 40;
     double *sSdw = sField + 8;
-    float *sDwf = (float *)(sSdw + (KEEP_DW ? 6 * ITEMS * C::IT : 0));
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const MemberDev *m0d = p.members;
@@ -889,12 +883,7 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
         par->k[lq] = p.k_red[gq];
         par->sr[lq] = p.sr[gq];
         for (int c = 0; c < 3; c++) par->axf[lq][c] = (float)par->ax[lq][c];
-        par->kf[lq] = (float)par->k[lq];
-        par->srf[lq] = (float)par->sr[lq];
-        // the particle's own anisotropy field Jacobian k e e^T
-        for (int a = 0; a < 3; a++)
-            for (int b = 0; b < 3; b++)
-                par->hjf[lq][3 * a + b] = (float)(par->k[lq] * par->ax[lq][a] * par->ax[lq][b]);
+        par->dtk[lq] = (float)(m0d->dt * par->k[lq]);
     }
     if (threadIdx.x < NB) sFlag[threadIdx.x] = 0;
     if (threadIdx.x == 0) *sErr = 0;
@@ -906,7 +895,7 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
     const double dt = m0d->dt, sq = m0d->sqrt_dt, alpha = m0d->alpha, Ah = m0d->Ah;
     const double eps = m0d->eps;
     const int64_t max_iter = m0d->max_iter;
-    const float alpha_f = (float)alpha, dt_f = (float)dt, sq_f = (float)sq;
+    const float alpha_f = (float)alpha;
     const bool renorm = m0d->renorm != 0;
     const int64_t S = p.S;
     const int64_t *sched = p.sched + m0d->sched_off;
@@ -940,8 +929,8 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
     auto write_B = [&](int buf) {
 #pragma unroll
         for (int i = 0; i < ITEMS; i++) {
-            const float m6[6] = {(float)x[i][0][0], (float)x[i][0][1], (float)x[i][0][2],
-                                 (float)x[i][1][0], (float)x[i][1][1], (float)x[i][1][2]};
+            const float m6[6] = {narrow(x[i][0][0]), narrow(x[i][0][1]), narrow(x[i][0][2]),
+                                 narrow(x[i][1][0]), narrow(x[i][1][1]), narrow(x[i][1][2])};
             put_pair_g<NB>(Bbuf[buf], r, p0 + 7 * i, j, live[i][0], live[i][1], m6);
         }
     };
@@ -1035,29 +1024,37 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
             sField[0] = f64::field_value(m0d->shape, t, m0d->happ, m0d->fapp);
             sField[1] = f64::field_value(m0d->shape, t + dt / 2, m0d->happ, m0d->fapp);
         }
-        // increments of this step, clamped and scaled (integrators.cpp:599-602),
-        // are recomputed where needed rather than kept: FP64 for the residual,
-        // FP32 for the Jacobian.  The generator's normals never reach the
-        // clamp (|w| <= 5.65 < Ah), so only injected increments are clamped.
-        auto dwm_of = [&](int i, int k, double out[3], float outf[3]) {
+        // sr dwm of this step, clamped and scaled (integrators.cpp:599-602).
+        // The generator's normals never reach the clamp (|w| <= 5.65 < Ah), so
+        // only injected increments are clamped.
+        auto sdw_of = [&](int i, int k, double out[3]) {
             const int q = PPC * r + 2 * (p0 + 7 * i) + k;
+            const double sr = par->sr[2 * (p0 + 7 * i) + k];
             if (noise) {
                 const double *wp = noise + (step - 1) * per_step + 3 * q;
                 for (int c = 0; c < 3; c++) {
                     const double lo = (wp[c] < Ah) ? wp[c] : Ah;
-                    out[c] = ((-Ah < lo) ? lo : -Ah) * sq;
-                    outf[c] = (float)out[c];
+                    out[c] = sr * (((-Ah < lo) ? lo : -Ah) * sq);
                 }
             } else {
                 const Normals4 nr = wiener_normals(seed, (uint64_t)step, (uint32_t)q);
                 const float w[3] = {nr.a, nr.b, nr.c};
-                for (int c = 0; c < 3; c++) {
-                    out[c] = (double)w[c] * sq;
-                    outf[c] = w[c] * sq_f;
-                }
+                for (int c = 0; c < 3; c++) out[c] = sr * (widen(w[c]) * sq);
             }
         };
-        // field at the current state -> the initial guess (g + x0) / 2
+        // stage increment g at m (and its v), hz the applied field
+        auto stage = [&](int i, int k, const double m[3], double hz, const double sdw[3],
+                         double g[3], double v[3]) {
+            const int lq = 2 * (p0 + 7 * i) + k;
+            const double *ax = par->ax[lq];
+            const double dot = par->k[lq] * fma(m[2], ax[2], fma(m[1], ax[1], m[0] * ax[0]));
+            const float *f = F + (3 * lq) * C::FS + j;
+            v[0] = fma(dt, fma(dot, ax[0], widen(f[0])), sdw[0]);
+            v[1] = fma(dt, fma(dot, ax[1], widen(f[C::FS])), sdw[1]);
+            v[2] = fma(dt, fma(dot, ax[2], widen(f[2 * C::FS]) + hz), sdw[2]);
+            stage_map(g, m, alpha, v);
+        };
+        // field at the current state -> the first iterate
         field();
         const double h_t = sField[0], h_m = sField[1];
         double part_v = 0.0;
@@ -1068,28 +1065,19 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
                 for (int k = 0; k < 2; k++) {
                     px[i][k][0] = x[i][k][0]; px[i][k][1] = x[i][k][1]; px[i][k][2] = x[i][k][2];
                     if (!live[i][k]) continue;
-                    const int lq = 2 * (p0 + 7 * i) + k;
-                    const double *ax = par->ax[lq];
                     const double *m = px[i][k];
-                    const double dot = (m[0] * ax[0] + m[1] * ax[1] + m[2] * ax[2]) * par->k[lq];
-                    double dwm[3];
-                    float dwf[3];
-                    dwm_of(i, k, dwm, dwf);
-                    const double sr = par->sr[lq];
+                    double sdw[3], g[3], v[3];
+                    sdw_of(i, k, sdw);
                     if constexpr (KEEP_DW)
-                        for (int c = 0; c < 3; c++) {
-                            sSdw[((i * 2 + k) * 3 + c) * C::IT + threadIdx.x] = sr * dwm[c];
-                            sDwf[((i * 2 + k) * 3 + c) * C::IT + threadIdx.x] = dwf[c];
-                        }
-                    const double v[3] = {
-                        dt * (dot * ax[0] + (double)F[(3 * lq) * C::FS + j]) + sr * dwm[0],
-                        dt * (dot * ax[1] + (double)F[(3 * lq + 1) * C::FS + j]) + sr * dwm[1],
-                        dt * (dot * ax[2] + h_t + (double)F[(3 * lq + 2) * C::FS + j]) + sr * dwm[2]};
-                    double g[3];
-                    llg_F64(g, m, alpha, v);
+                        for (int c = 0; c < 3; c++)
+                            sSdw[((i * 2 + k) * 3 + c) * C::IT + threadIdx.x] = sdw[c];
+                    stage(i, k, m, h_t, sdw, g, v);
                     for (int c = 0; c < 3; c++) {
-                        x[i][k][c] = (g[c] + m[c]) / 2;
-                        part_v += x[i][k][c] * x[i][k][c];
+                        // the reference's first iterate (g + x0)/2 sets the
+                        // tolerance; the iteration starts from x0 + g/2
+                        const double y = 0.5 * (g[c] + m[c]);
+                        part_v = fma(y, y, part_v);
+                        x[i][k][c] = fma(0.5, g[c], m[c]);
                     }
                 }
         }
@@ -1103,6 +1091,10 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
         int64_t iter = max_iter;
         bool active = valid;
         int32_t mflag = ST_OK;
+        if (active && !(err > tol))  // no iteration: the result is the reference's first iterate
+            for (int i = 0; i < ITEMS; i++)
+                for (int k = 0; k < 2; k++)
+                    for (int c = 0; c < 3; c++) x[i][k][c] = fma(-0.5, px[i][k][c], x[i][k][c]);
         for (;;) {
             // while ((err > tol) && (iter-- > 0)), per member
             bool go = false;
@@ -1115,7 +1107,7 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
             }
             if (!__syncthreads_or(go)) break;
             field();  // dipolar field at every member's current iterate
-            double dsum = 0.0;
+            DDf dsum{0.f, 0.f};
             int sing = 0;
             if (go) {
 #pragma unroll
@@ -1124,68 +1116,39 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
                     for (int k = 0; k < 2; k++) {
                         if (!live[i][k]) continue;
                         const int lq = 2 * (p0 + 7 * i) + k;
-                        const double *ax = par->ax[lq];
                         const double xt[3] = {x[i][k][0], x[i][k][1], x[i][k][2]};
-                        const double dot =
-                            (xt[0] * ax[0] + xt[1] * ax[1] + xt[2] * ax[2]) * par->k[lq];
-                        const double h[3] = {dot * ax[0] + (double)F[(3 * lq) * C::FS + j],
-                                             dot * ax[1] + (double)F[(3 * lq + 1) * C::FS + j],
-                                             dot * ax[2] + h_m +
-                                                 (double)F[(3 * lq + 2) * C::FS + j]};
-                        double sdw[3];  // sr dwm
-                        float dwf[3];
+                        double sdw[3], g[3], v[3];
                         if constexpr (KEEP_DW) {
-                            for (int c = 0; c < 3; c++) {
+                            for (int c = 0; c < 3; c++)
                                 sdw[c] = sSdw[((i * 2 + k) * 3 + c) * C::IT + threadIdx.x];
-                                dwf[c] = sDwf[((i * 2 + k) * 3 + c) * C::IT + threadIdx.x];
-                            }
                         } else {
-                            double dwm[3];
-                            dwm_of(i, k, dwm, dwf);
-                            for (int c = 0; c < 3; c++) sdw[c] = par->sr[lq] * dwm[c];
+                            sdw_of(i, k, sdw);
                         }
-                        const double v[3] = {fma(dt, h[0], sdw[0]), fma(dt, h[1], sdw[1]),
-                                             fma(dt, h[2], sdw[2])};
-                        double g[3];
-                        llg_F64(g, xt, alpha, v);
+                        stage(i, k, xt, h_m, sdw, g, v);
                         // F(y) = y - a dt / 2 - x0 - B dwm / 2 (integrators.cpp:621-627)
-                        float sol[3];
+                        float sol[3], J[9];
                         for (int c = 0; c < 3; c++)
-                            sol[c] = (float)(fma(0.5, g[c], px[i][k][c]) - xt[c]);
-                        // Jacobian in FP32 from FP32 copies of the state and field
-                        const float xf[3] = {(float)xt[0], (float)xt[1], (float)xt[2]};
-                        const float *axf = par->axf[lq];
-                        const float dotf = (xf[0] * axf[0] + xf[1] * axf[1] + xf[2] * axf[2]) *
-                                           par->kf[lq];
-                        const float hf[3] = {fmaf(dotf, axf[0], F[(3 * lq) * C::FS + j]),
-                                             fmaf(dotf, axf[1], F[(3 * lq + 1) * C::FS + j]),
-                                             fmaf(dotf, axf[2], F[(3 * lq + 2) * C::FS + j]) +
-                                                 (float)h_m};
-                        float adash[9], bdash[27], J[9];
-                        f64::drift_jacobian<float>(adash, xf, alpha_f, hf, par->hjf[lq]);
-                        f64::diffusion_jacobian<float>(bdash, xf, par->srf[lq], alpha_f);
-                        for (int rr = 0; rr < 3; rr++)
-                            for (int c = 0; c < 3; c++) {
-                                float jv = (float)(rr == c) - 0.5f * dt_f * adash[3 * rr + c];
-                                for (int kk = 0; kk < 3; kk++)
-                                    jv -= 0.5f * bdash[9 * rr + 3 * kk + c] * dwf[kk];
-                                J[3 * rr + c] = jv;
-                            }
+                            sol[c] = narrow(fma(0.5, g[c], px[i][k][c]) - xt[c]);
+                        const float xf[3] = {narrow(xt[0]), narrow(xt[1]), narrow(xt[2])};
+                        const float vf[3] = {narrow(v[0]), narrow(v[1]), narrow(v[2])};
+                        stage_jacobian(J, xf, alpha_f, vf, par->axf[lq], par->dtk[lq]);
                         if (f64::solve3<float>(J, sol) != 0) {
                             sing = 1;
                             continue;  // the member stops with its current iterate
                         }
                         for (int c = 0; c < 3; c++) {
-                            const double d = (double)sol[c];
-                            dsum += d * d;
-                            x[i][k][c] = xt[c] + d;
+                            // exact square, added to the float-float sum
+                            const float s2 = sol[c] * sol[c];
+                            dsum.lo += __fmaf_rn(sol[c], sol[c], -s2);
+                            dsum = dd_add_ts(dsum, s2);
+                            x[i][k][c] = xt[c] + widen(sol[c]);
                         }
                     }
             }
             write_B(wb ^ 1);
             wb ^= 1;
             double d2;
-            cluster_sum(dsum, sing, d2, sing_any);
+            cluster_sum((double)dsum.hi + (double)dsum.lo, sing, d2, sing_any);
             err = sqrt(d2);
             if (go && sing_any) { mflag |= ST_SINGULAR; active = false; }
         }
@@ -1285,11 +1248,6 @@ cudaError_t tcc_launch(Kern kern, const TccLayout &L, size_t smem, int threads, 
 bool tcc_supported(int n) { return n > 64 && n <= PPC * TCC_MAX_T; }
 
 bool tcc_implicit_supported(int n) { return n >= 2 && n <= PPC * TCC_MAX_T; }
-
-int tcc_members_per_cluster(int members_per_warp_hint)
-{
-    return members_per_warp_hint == 32 ? 32 : 64;
-}
 
 size_t tcc_d_elems(int n)
 {

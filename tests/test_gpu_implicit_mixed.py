@@ -110,3 +110,19 @@ def test_shared_applied_field(gpu_lib, n, implicit, shape):
     for c in ("mx", "my", "mz"):
         assert np.array_equal(getattr(a, c)[:, same], getattr(b, c)[:, same])
         assert not np.array_equal(getattr(a, c)[:, ~same], getattr(b, c)[:, ~same])
+
+
+@pytest.mark.parametrize("precision,n", [("mixed", 5), ("mixed", 40), ("mixed_tc", 5),
+                                         ("mixed_tc", 70)])
+def test_no_iteration_with_zero_tolerance(gpu_lib, precision, n):
+    """A tolerance of zero stops the reference's iteration before it begins: its
+    first iterate is the result.  Two steps of an FP32 dipolar sum (n 6e-8 of
+    fields of order 1, times dt 4e-3) differ by below 1e-6."""
+    from magpy_gb300 import core
+    args = list(_args(n, 3, 3, 2e-13))
+    args[-1] = 0.0
+    a = core.simulate_ensemble(*args, precision=precision)
+    b = core.simulate_ensemble(*args, precision="fp64")
+    assert np.all(a.status == 0) and np.all(b.status == 0)
+    for c in ("mx", "my", "mz"):
+        assert np.abs(getattr(a, c) - getattr(b, c)).max() / 4e5 < 1e-6
