@@ -63,6 +63,12 @@ cudaError_t launch_mixed(const DevPlan &p, cudaStream_t stream);
 cudaError_t mixed_prepare(const DevPlan &p, int64_t clusters, int64_t K, double dt, int shape,
                           double happ, double fapp, float **ftab, float4 **pr,
                           cudaStream_t stream);
+// Pair tables of `clusters` clusters of n particles from their locations
+// ([c][n][3], m), reduced volumes ([c][n]) and (distance scale, prefactor)
+// ([c][2]): pr [c][n][n] and, unless null, FP64 tables at pt: [c][n][n] pair
+// factors, then [c][3][n][n] unit vectors (index j * n + q as DevPlan's).
+cudaError_t mixed_build_pairs(const double *loc, const double *vol, const double *par, int64_t n,
+                              int64_t clusters, float4 *pr, double *pt, cudaStream_t stream);
 // As mixed_prepare, into tables the caller provides (2K floats, clusters*n*n float4).
 cudaError_t mixed_fill_tables(const DevPlan &p, int64_t clusters, int64_t K, double dt,
                               int shape, double happ, double fapp, float *ftab, float4 *pr,

@@ -434,6 +434,36 @@ __global__ void pair_table_kernel(float4 *out, const double *pt, const double *r
     out[i] = make_float4((float)R[r], (float)R[nn + r], (float)R[2 * nn + r], (float)P[r]);
 }
 
+// lib/distances.cpp:20-113 and lib/field.cpp:212-225 in FP64, one pair (j, q)
+// a thread; one division and one square root (FP64 is the narrow pipe), good
+// to a few units of FP64's last place.  The diagonal is zero.
+__global__ void build_pairs_kernel(const double *loc, const double *vol, const double *par, int n,
+                                   int64_t clusters, float4 *pr, double *pt)
+{
+    const int64_t nn = (int64_t)n * n, tot = nn * clusters;
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= tot) return;
+    const int64_t c = i / nn, r = i % nn;
+    const int j = (int)(r / n), q = (int)(r % n);
+    double P = 0.0, u[3] = {0.0, 0.0, 0.0};
+    if (j != q) {
+        const double *lj = loc + 3 * (c * n + j), *lq = loc + 3 * (c * n + q);
+        const double d0 = lj[0] - lq[0], d1 = lj[1] - lq[1], d2 = lj[2] - lq[2];
+        const double inv = 1.0 / sqrt(d0 * d0 + d1 * d1 + d2 * d2);
+        u[0] = d0 * inv;
+        u[1] = d1 * inv;
+        u[2] = d2 * inv;
+        const double s = par[2 * c] * inv;  // one over the reduced distance
+        P = par[2 * c + 1] * (vol[c * n + j] * (s * s * s));
+    }
+    pr[i] = make_float4((float)u[0], (float)u[1], (float)u[2], (float)P);
+    if (pt) {
+        pt[i] = P;
+        double *rt = pt + tot + 3 * c * nn;
+        for (int k = 0; k < 3; k++) rt[k * nn + r] = u[k];
+    }
+}
+
 __global__ void wiener_kernel(uint64_t seed, int64_t n, int64_t K, double *out)
 {
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -472,6 +502,16 @@ cudaError_t mixed_prepare(const DevPlan &p, int64_t clusters, int64_t K, double 
         if ((err = cudaGetLastError()) != cudaSuccess) return err;
     }
     return cudaSuccess;
+}
+
+cudaError_t mixed_build_pairs(const double *loc, const double *vol, const double *par, int64_t n,
+                              int64_t clusters, float4 *pr, double *pt, cudaStream_t stream)
+{
+    const int64_t tot = clusters * n * n;
+    if (tot == 0) return cudaSuccess;
+    build_pairs_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, stream>>>(loc, vol, par, (int)n,
+                                                                        clusters, pr, pt);
+    return cudaGetLastError();
 }
 
 cudaError_t mixed_fill_tables(const DevPlan &p, int64_t clusters, int64_t K, double dt,
