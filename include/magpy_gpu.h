@@ -154,7 +154,10 @@ int magpy_plan_copy_out(magpy_plan *plan, magpy_ensemble_out *out, void *stream)
 int magpy_plan_shape(const magpy_plan *plan, int64_t *n_members, int64_t *n_particles,
                      int64_t *n_samples, int64_t *max_steps);
 /* Launch shape of the warp-packed kernels (clusters of <= 32 particles):
- * warps per CTA and members per warp (0 = as many as fit).  For larger
+ * warps per CTA and members per warp (0 = as many as fit); until it is set,
+ * the launcher chooses both by the ensemble's size.  (In MAGPY_PRECISION_MIXED
+ * Heun runs of one or two particles a thread holds two particles and the
+ * shape is not used.)  For larger
  * clusters in MAGPY_PRECISION_MIXED whose members share one cluster,
  * members_per_warp = 2 or 4 puts that many members in one CTA.  In
  * MAGPY_PRECISION_MIXED_TC with more than 64 particles (and in its implicit
