@@ -1738,8 +1738,14 @@ extern "C" int magpy_adjoint_create(const magpy_ensemble_desc *d, int64_t checkp
     const size_t nck = (size_t)(K / C + 1);
     CUDA_TRY(pool_alloc(&A->bufs[0], P * sizeof(double)));
     CUDA_TRY(cudaMemcpy(A->bufs[0], vred.data(), P * sizeof(double), cudaMemcpyHostToDevice));
-    CUDA_TRY(pool_alloc(&A->bufs[1], nck * 6 * P * sizeof(float)));
-    CUDA_TRY(pool_alloc(&A->bufs[2], (size_t)std::min(C, std::max<int64_t>(K, 1)) * 3 * P * sizeof(float)));
+    // checkpoints and the segment's moments, two members side by side
+    const size_t P2 = (size_t)(E + 1) / 2 * 2 * n;
+    CUDA_TRY(pool_alloc(&A->bufs[1], nck * 6 * P2 * sizeof(float)));
+    // the dipolar fields of a segment (6 floats a particle and step beside the
+    // moments' 3) are kept where that takes 4 GiB at most
+    const size_t seg = (size_t)std::min(C, std::max<int64_t>(K, 1)) * P2 * sizeof(float);
+    A->a.kept = d->interactions && n > 1 && seg <= ((size_t)4 << 30) / 9;
+    CUDA_TRY(pool_alloc(&A->bufs[2], (A->a.kept ? 9 : 3) * seg));
     CUDA_TRY(pool_alloc(&A->bufs[3], std::max<int64_t>(A->S, 1) * sizeof(double)));
     CUDA_TRY(pool_alloc(&A->bufs[4], 5 * sizeof(double)));
     if (R.shape != MAGPY_FIELD_CONSTANT && K > 0) {

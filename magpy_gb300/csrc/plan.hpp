@@ -156,7 +156,8 @@ struct AdjointArgs {
     float happ, dt, sq, alpha, c;
     int64_t K;
     int C, interactions;
-    float *ck, *seg;
+    float *ck, *seg;      // checkpoints, and the moments of the segment being swept
+    bool kept = false;    // seg has room for the dipolar fields too
     const double *wz;     // [S]
     double *grad;         // [5]
 };
