@@ -42,10 +42,20 @@ constexpr int GM = 16;           // members per group (two groups per CTA)
 constexpr int ITEM_THREADS = 512; // 16 item warps: 4 TMEM sub-partitions x 4 column quarters
 constexpr int TC_THREADS = ITEM_THREADS + 64;  // + one warp per 128-row tile that only
                                                // issues that tile's MMAs
-// Field tile row stride (floats): 20 makes the epilogue's 128-bit stores (32
-// consecutive rows, four columns) and the integrator's reads (8 member
-// columns of 4 particle pairs) free of bank conflicts.
+// Field tile row stride (floats), and four more floats for every second block
+// of 24 rows (four particle pairs): 20 makes the epilogue's 128-bit stores (32
+// consecutive rows, four columns) free of bank conflicts, the skew the
+// integrator's reads (4 member columns of 8 particle pairs).
 constexpr int GH_STRIDE = 20;
+// A group's B tile: 32 rows (four 128-byte core matrices) per 8 K elements, and
+// 64 bytes more to the next 8: a warp's word stores (4 members x 8 particle
+// pairs) then fall into different banks (without them two ways).
+constexpr uint32_t B_LBO = (2 * GM / 8) * 128 + 64;
+__host__ __device__ inline uint32_t b_offset(uint32_t row, uint32_t k)
+{
+    return (k >> 3) * (B_LBO / 2) + ((row >> 3) << 6) + ((row & 7) << 3) + (k & 7);
+}
+__device__ inline int gh_row(int row) { return row * GH_STRIDE + 4 * ((row / 24) & 1); }
 constexpr int HS_STRIDE = NM + 1;  // field exchange of the single-round dipolar entry
 constexpr int ITEMS = 2;         // (particle, member) items per thread and group
 constexpr uint32_t WAIT_LIMIT = 1u << 24;
@@ -88,7 +98,7 @@ __host__ __device__ inline TcLayout tc_layout(int n)
     L.a_span = (size_t)16 * L.tiles * L.a_sbo;
     L.buf_off = 2 * L.d_bytes;
     const size_t reach = L.d_bytes + L.a_span;  // end of D_lo's MMA reads
-    L.gb_bytes = up((size_t)2 * GM * L.KP * 2, 128);
+    L.gb_bytes = up((size_t)(L.KP / 8) * B_LBO, 128);
     L.gh_bytes = up((size_t)L.n3 * GH_STRIDE * 4, 128);
     L.w_off = 2 * L.gb_bytes + 2 * L.gh_bytes;  // integrator buffers start at 0
     L.a_off = L.w_off + (size_t)2 * 3 * ITEM_THREADS * 16;  // [g][3] float4 per thread
@@ -279,11 +289,14 @@ __global__ void __launch_bounds__(ITEM_THREADS, 1)
 
 // ---- the integrator ----
 // Items are (particle q, member j) pairs.  In each group warp w serves the
-// 8 members j = 8 (w % 2) + (lane % 8) and the particle pairs
-// pp = 4 (w / 2) + lane / 8, so a thread owns particles 2 pp and 2 pp + 1 of
-// one member per group (one generator call gives the pair's six normals, and
-// the pair's six components are three aligned words of a B-tile row), and
-// the same particles of the same member slot in both groups.
+// 4 members j = 4 a + (lane % 4), a = w / 4, and the particle pairs
+// pp = 8 b + lane / 4, b = (w - a) mod 4, so a thread owns particles 2 pp and
+// 2 pp + 1 of one member per group (one generator call gives the pair's six
+// normals, and the pair's six components are three aligned words of a B-tile
+// row), and the same particles of the same member slot in both groups.  A
+// group of 12, 8 or 4 members leaves whole warps without work, and a cluster of
+// fewer pairs too, in each case the same number of every sub-partition (warp
+// index mod 4).
 // Per item the state is a float-float triple x; between the two Heun stages
 // it keeps A = F(m, v1) / 2 and the increments w; the stage map F and the
 // state update are those of llg32.cuh.
@@ -295,8 +308,8 @@ __global__ void __launch_bounds__(ITEM_THREADS, 1)
 constexpr uint32_t G_LO_SHIFT = (GM / 8) * 64;  // element distance from row j to row j + 16
 __device__ inline void pair_offsets(int j, int pp, uint32_t &o01, uint32_t &o2)
 {
-    o01 = tc::cm_offset(j, 6 * pp, 2 * GM) | (tc::cm_offset(j, 6 * pp + 2, 2 * GM) << 16);
-    o2 = tc::cm_offset(j, 6 * pp + 4, 2 * GM);
+    o01 = b_offset(j, 6 * pp) | (b_offset(j, 6 * pp + 2) << 16);
+    o2 = b_offset(j, 6 * pp + 4);
 }
 
 // One word of B_hi and of B_lo: x ~ hi + lo / 2048 for two K elements.
@@ -322,25 +335,24 @@ __device__ inline void put_pair(__half *bt, uint32_t o01, uint32_t o2, bool live
     if (live1) put_word(bt, o2, m[4], m[5]);
 }
 
-__device__ inline void write_sample(const DevPlan &p, int64_t s, int64_t e, int n, int q,
-                                    const DDf xk[3])
+// Sample s of a thread's one or two particles: x = (hi + lo) scale, the low
+// words of component c at xl[c ITEM_THREADS].  o: the first particle's index
+// in a component's [S][P] plane.  Not inlined, as field_block is not: what a
+// step rarely runs is kept out of the step loop's code.  The kernel is bound by
+// the latency of its four phases a step, and instruction fetches are part of
+// it: with both inlined a step took 2.91, 3.39 and 5.10 us at 16, 32 and 64
+// particles and 32 members a CTA (4096 members), without 2.63, 3.25 and 4.90.
+__device__ __noinline__ void write_pair(double *mx, double *my, double *mz, int64_t o, double sc,
+                                        float2 x, float2 y, float2 z, const float2 *xl, bool two)
 {
-    const int64_t o = s * p.P + e * n + q;
-    const double sc = p.out_scale[e];
-    p.mx[o] = ((double)xk[0].hi + (double)xk[0].lo) * sc;
-    p.my[o] = ((double)xk[1].hi + (double)xk[1].lo) * sc;
-    p.mz[o] = ((double)xk[2].hi + (double)xk[2].lo) * sc;
-}
-
-// Item k (0 or 1) of a thread's packed state as a float-float triple; the
-// low words of component c at xl[c ITEM_THREADS].
-__device__ inline void item_state(DDf out[3], const float2 xh[3], const float2 *xl, int k)
-{
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-        const float2 lo = xl[c * ITEM_THREADS];
-        out[c] = k == 0 ? DDf{xh[c].x, lo.x} : DDf{xh[c].y, lo.y};
-    }
+    const float2 lx = xl[0], ly = xl[ITEM_THREADS], lz = xl[2 * ITEM_THREADS];
+    mx[o] = ((double)x.x + (double)lx.x) * sc;
+    my[o] = ((double)y.x + (double)ly.x) * sc;
+    mz[o] = ((double)z.x + (double)lz.x) * sc;
+    if (!two) return;
+    mx[o + 1] = ((double)x.y + (double)lx.y) * sc;
+    my[o + 1] = ((double)y.y + (double)ly.y) * sc;
+    mz[o + 1] = ((double)z.y + (double)lz.y) * sc;
 }
 
 // Per-CTA state of the two groups' tensor-core rounds.
@@ -351,6 +363,8 @@ struct Rounds {
     uint64_t *bar;
     uint32_t tmem;
     uint32_t phase[2];
+    int gm[2];       // members of each group (4, 8, 12 or 16)
+    uint32_t rows;   // this thread's field-tile offsets of tiles 0 and 1 (16 bits each)
     uint32_t limit;  // polls of a phase wait before the watchdog gives up
     bool inflight[2];
 };
@@ -401,13 +415,17 @@ __device__ inline void issue(Rounds &R, int g)
         tc::fence_after_sync();
         constexpr uint32_t idesc32 = tc::idesc_f16_f32(128, 2 * GM);
         constexpr uint32_t idesc16 = tc::idesc_f16_f32(128, GM);
-        constexpr uint32_t b_lbo = (2 * GM / 8) * 128;
-        constexpr uint32_t b_kstep = (2 * b_lbo) >> 4;
-        const uint64_t b0 = tc::smem_desc(tc::smem_addr(R.sB[g]), b_lbo, 128);
+        constexpr uint32_t b_kstep = (2 * B_LBO) >> 4;
+        const uint64_t b0 = tc::smem_desc(tc::smem_addr(R.sB[g]), B_LBO, 128);
         const int ksteps = R.L.KP / 16;
         const uint32_t acc = R.tmem + 64 * it + 32 * g;
         const uint32_t a_hi = R.tmem + tmem_d_col(R.L, it, 0);
         const uint32_t a_lo = R.tmem + tmem_d_col(R.L, it, 1);
+        // Two k-steps at a time: the compiler's own four make the loop's four
+        // copies 19 KB longer, which small clusters on all SMs pay for (32
+        // particles, 4096 members: 3.79 us a step against 3.04), one at a time
+        // issues too slowly (64 particles: 5.12 us against 4.56).
+#pragma unroll 2
         for (int s = 0; s < ksteps; s++) {
             const uint64_t b = b0 + (uint64_t)(b_kstep * s);
             // [main | corr] (+)= D_hi [B_hi | B_lo]; corr += D_lo B_hi  (K = 16)
@@ -423,18 +441,19 @@ __device__ inline void issue(Rounds &R, int g)
 // field tile and make it visible to the CTA.  Returns false (uniformly) if
 // the completion did not arrive in time.  No MMA is in flight while the
 // accumulators are read: the other group's MMAs are issued after this
-// function's barrier.  RT_LIMIT: the bound is the plan's run-time setting
-// (a separate instantiation: a run-time bound in this wait measured 2.8 %
-// slower on the headline workload than the compile-time WAIT_LIMIT).
-template <bool RT_LIMIT>
+// function's barrier.  GENERAL: the bound is the plan's run-time setting, and
+// the increments may be injected ones (a separate instantiation: a run-time
+// bound in this wait measured 2.8 % slower on the headline workload than the
+// compile-time WAIT_LIMIT, and neither's code is fetched where it isn't used).
+template <bool GENERAL>
 __device__ inline bool finish(Rounds &R, int g)
 {
     const bool ok = __all_sync(
-        0xffffffffu, tc::mbar_wait_bounded(&R.bar[g], R.phase[g], RT_LIMIT ? R.limit : WAIT_LIMIT));
+        0xffffffffu, tc::mbar_wait_bounded(&R.bar[g], R.phase[g], GENERAL ? R.limit : WAIT_LIMIT));
     tc::fence_after_sync();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sub = warp & 3, quarter = warp >> 2;
-    if (ok && threadIdx.x < ITEM_THREADS) {
+    if (ok && threadIdx.x < ITEM_THREADS && 4 * quarter < R.gm[g]) {
         const uint32_t lanes = (uint32_t)(32 * sub) << 16;
         for (int t = 0; t < R.L.tiles; t++) {
             float vm[4], vc[4];
@@ -444,7 +463,7 @@ __device__ inline bool finish(Rounds &R, int g)
             tc::tmem_ld_wait();
             const int row = 128 * t + 32 * sub + lane;
             if (row < R.L.n3)
-                *reinterpret_cast<float4 *>(R.sH[g] + row * GH_STRIDE + 4 * quarter) =
+                *reinterpret_cast<float4 *>(R.sH[g] + (t ? R.rows >> 16 : R.rows & 0xffffu)) =
                     make_float4(fmaf(vc[0], 1.0f / tc::SPLIT_SCALE, vm[0]),
                                 fmaf(vc[1], 1.0f / tc::SPLIT_SCALE, vm[1]),
                                 fmaf(vc[2], 1.0f / tc::SPLIT_SCALE, vm[2]),
@@ -471,7 +490,7 @@ __device__ inline bool finish(Rounds &R, int g)
 // block b's first step, and the integrator first reads it more than 30
 // steps later; the slot it overwrites (block b - 1) was last read before
 // that barrier.
-__device__ inline void field_block(float2 *sF2, const MemberDev *md, int64_t b, int64_t K)
+__device__ __noinline__ void field_block(float2 *sF2, const MemberDev *md, int64_t b, int64_t K)
 {
     const int it = ((int)threadIdx.x - ITEM_THREADS) >> 5, lane = threadIdx.x & 31;
     const int64_t k = FIELD_BLOCK * b + 1 + lane;
@@ -481,7 +500,7 @@ __device__ inline void field_block(float2 *sF2, const MemberDev *md, int64_t b, 
     }
 }
 
-template <bool RT_LIMIT>
+template <bool GENERAL>
 __device__ inline void issuer_loop(Rounds &R, int64_t K, int64_t noise_steps,
                                    const MemberDev *md, float2 *sF2)
 {
@@ -490,7 +509,7 @@ __device__ inline void issuer_loop(Rounds &R, int64_t K, int64_t noise_steps,
         if (step > noise_steps) break;
 #pragma unroll
         for (int g = 0; g < 2; g++) {
-            if (!finish<RT_LIMIT>(R, g)) { alive = false; break; }
+            if (!finish<GENERAL>(R, g)) { alive = false; break; }
             issue(R, 1 - g);
             if (g == 0 && ((step - 1) % FIELD_BLOCK) == 0)
                 field_block(sF2, md, (step - 1) / FIELD_BLOCK + 1, K);
@@ -498,15 +517,15 @@ __device__ inline void issuer_loop(Rounds &R, int64_t K, int64_t noise_steps,
         if (!alive) break;
 #pragma unroll
         for (int g = 0; g < 2; g++) {
-            if (!finish<RT_LIMIT>(R, g)) { alive = false; break; }
+            if (!finish<GENERAL>(R, g)) { alive = false; break; }
             if (g == 0 || step < K) issue(R, 1 - g);
         }
     }
 }
 
-template <bool RT_LIMIT>
+template <bool GENERAL>
 __global__ void __launch_bounds__(TC_THREADS, 1)
-    sllg_tc_kernel(DevPlan p, const __half *dhi)
+    sllg_tc_kernel(DevPlan p, const __half *dhi, int gm0, int gm1)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
     const int n = p.n;
@@ -536,14 +555,22 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     float4 *sAW = (float4 *)(sm + L.w_off);
     float2 *sXL = (float2 *)(sm + L.a_off);
     R.phase[0] = R.phase[1] = 0;
+    R.gm[0] = gm0;
+    R.gm[1] = gm1;
+    {
+        const int row = 32 * ((threadIdx.x >> 5) & 3) + (threadIdx.x & 31);
+        const int col = 4 * (threadIdx.x >> 7);
+        R.rows = (uint32_t)(gh_row(row) + col) | (uint32_t)(gh_row(row + 128) + col) << 16;
+    }
     R.limit = p.wait_limit;
     R.inflight[0] = R.inflight[1] = false;
 
-    // both B tiles zero (the K-padding rows 3N..KP stay zero for the run)
+    // both B tiles zero (the K-padding rows 3N..KP stay zero for the run, and
+    // the rows of members a group does not have)
     uint4 *bz = (uint4 *)sm;
     for (int i = threadIdx.x; i < (int)(2 * L.gb_bytes / 16); i += blockDim.x)
         bz[i] = make_uint4(0, 0, 0, 0);
-    const int64_t base = (int64_t)blockIdx.x * NM;
+    const int64_t base = (int64_t)blockIdx.x * (gm0 + gm1);
     const MemberDev *m0d = p.members + base;  // members of a launch share their parameters
     const int64_t P = p.P;
     for (int i = threadIdx.x; i < (n + 1) / 2; i += blockDim.x) {
@@ -565,8 +592,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         sSr[i] = make_float2(r[0], r[1]);
     }
     if (threadIdx.x < NM) {
-        const int64_t em = base + threadIdx.x;
-        const bool ok = em < p.E;
+        // member slots GM g + j of the two groups
+        const int g = threadIdx.x / GM, j = threadIdx.x % GM;
+        const int64_t em = base + gm0 * g + j;
+        const bool ok = j < (g ? gm1 : gm0) && em < p.E;
         sFlag[threadIdx.x] = 0;
         sSeed[threadIdx.x] = ok ? p.members[em].seed : 0;
         sNoff[threadIdx.x] = ok ? p.members[em].noise_off : 0;
@@ -590,14 +619,17 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     const int64_t per_step = 3 * (int64_t)n;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int jl = 8 * (warp & 1) + (lane & 7);      // member slot within a group
-    // particles 2 pp + k; the issuing warps get pp >= 32: no items
-    const int pp = 4 * (warp >> 1) + (lane >> 3);
+    const int quad = warp >> 2;
+    const int jl = 4 * quad + (lane & 3);            // member slot within a group
+    // particles 2 pp + k; the issuing warps have none
+    const int pp = warp < ITEM_THREADS / 32 ? 8 * ((warp - quad) & 3) + (lane >> 2) : n;
     const int q0 = 2 * pp;
     const bool live[ITEMS] = {q0 < n, q0 + 1 < n};
-    const int64_t e0 = base + jl;  // member of group g: e0 + GM g
+    const int64_t e0 = base + jl;  // member of group g: e0 + gm0 g
+    // the particle's fields in a field tile: rows 6 pp .. 6 pp + 5, column jl
+    const int hoff = 6 * pp * GH_STRIDE + 4 * ((pp >> 2) & 1) + jl;
     bool valid[2];
-    const bool inj = p.noise != nullptr;  // injected increments instead of the generator
+    const bool inj = GENERAL && p.noise != nullptr;  // injected increments instead of the generator
     uint32_t o01 = 0, o2 = 0;
     if (q0 < n) pair_offsets(jl, pp, o01, o2);
     // State: component c of both items (particles q0, q0 + 1) as the .x and
@@ -609,7 +641,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     float2 xh[2][3];
     float2 *const xlt = sXL + threadIdx.x;
 #pragma unroll
-    for (int g = 0; g < 2; g++) valid[g] = e0 + GM * g < p.E;
+    for (int g = 0; g < 2; g++) valid[g] = jl < R.gm[g] && e0 + gm0 * g < p.E;
+    const auto record = [&](int64_t smp, int g) {
+        const int64_t e = e0 + gm0 * g;
+        if (live[0] && valid[g])
+            write_pair(p.mx, p.my, p.mz, smp * P + e * n + q0, p.out_scale[e], xh[g][0], xh[g][1],
+                       xh[g][2], xlt + 3 * g * ITEM_THREADS, live[1]);
+    };
 #pragma unroll
     for (int g = 0; g < 2; g++)
         for (int c = 0; c < 3; c++) {
@@ -618,7 +656,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 const int q = q0 + k;
                 hv[k] = lv[k] = 0.f;
                 if (q < n && valid[g]) {
-                    const double v = p.m0[c * P + (e0 + GM * g) * n + q];
+                    const double v = p.m0[c * P + (e0 + gm0 * g) * n + q];
                     hv[k] = (float)v;
                     lv[k] = (float)(v - (double)hv[k]);
                 }
@@ -632,13 +670,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         const float m6[6] = {xh[g][0].x, xh[g][1].x, xh[g][2].x,
                              xh[g][0].y, xh[g][1].y, xh[g][2].y};
         put_pair(R.sB[g], o01, o2, live[0], live[1], m6);
-        if (p.mx && valid[g])  // sample 0: the initial state (lib/simulation.cpp:212-219)
-            for (int k = 0; k < ITEMS; k++)
-                if (q0 + k < n) {
-                    DDf t[3];
-                    item_state(t, xh[g], xlt + 3 * g * ITEM_THREADS, k);
-                    write_sample(p, 0, e0 + GM * g, n, q0 + k, t);
-                }
+        if (p.mx) record(0, g);  // the initial state (lib/simulation.cpp:212-219)
     }
     if (threadIdx.x >= ITEM_THREADS) field_block(sF2, m0d, 0, K);  // steps 1..32
     tc::fence_proxy_async();
@@ -651,10 +683,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     // No global load sits at the head of a step: the step of the next sample
     // is kept in a register and the applied field is fetched a step ahead.
     int64_t next_sample = S > 1 ? sched[1] : -1;
-    const int64_t noise_steps = p.noise ? m0d->noise_len / per_step : K;
+    const int64_t noise_steps = GENERAL && p.noise ? m0d->noise_len / per_step : K;
     if (threadIdx.x >= ITEM_THREADS) {  // issuing warps
         if (K > 0) issue(R, 0);
-        issuer_loop<RT_LIMIT>(R, K, noise_steps, m0d, sF2);
+        issuer_loop<GENERAL>(R, K, noise_steps, m0d, sF2);
     } else {
     if (K > 0) R.inflight[0] = true;
     for (step = 1; step <= K && alive; step++) {
@@ -662,13 +694,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         while (next_sample == step) {
             if (p.mx)
                 for (int g = 0; g < 2; g++)
-                    if (valid[g])
-                        for (int k = 0; k < ITEMS; k++)
-                            if (q0 + k < n) {
-                                DDf t[3];
-                                item_state(t, xh[g], xlt + 3 * g * ITEM_THREADS, k);
-                                write_sample(p, s_next, e0 + GM * g, n, q0 + k, t);
-                            }
+                    record(s_next, g);
             s_next++;
             next_sample = s_next < S ? sched[s_next] : -1;
         }
@@ -684,17 +710,17 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         // stage 1 of each group: field at the current state -> predictor
 #pragma unroll
         for (int g = 0; g < 2; g++) {
-            if (!finish<RT_LIMIT>(R, g)) { status |= ST_WATCHDOG; alive = false; break; }
+            if (!finish<GENERAL>(R, g)) { status |= ST_WATCHDOG; alive = false; break; }
             R.inflight[1 - g] = true;  // (1, 1) on the state, or (0, 2) on the predictor
+            const bool work = live[0] && 4 * quad < R.gm[g];
             PairNormals wn;
-            if (!inj && live[0])
+            if (!inj && work)
                 wn = wiener_pair(sSeed[GM * g + jl], (uint64_t)step, (uint32_t)pp);
-            if (live[0]) {
+            if (work) {
                 // both items; a particle past the cluster (odd n) reads the
                 // first one's tables, and its results are dropped
-                const int qa = q0, qb = live[1] ? q0 + 1 : q0;
-                const float *ha = R.sH[g] + 3 * qa * GH_STRIDE + jl;
-                const float *hb = R.sH[g] + 3 * qb * GH_STRIDE + jl;
+                const float *ha = R.sH[g] + hoff;
+                const float *hb = live[1] ? ha + 3 * GH_STRIDE : ha;
                 const float2 hd[3] = {make_float2(ha[0], hb[0]),
                                       make_float2(ha[GH_STRIDE], hb[GH_STRIDE]),
                                       make_float2(ha[2 * GH_STRIDE], hb[2 * GH_STRIDE])};
@@ -743,13 +769,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         // stage 2 of each group: field at the predictor -> corrector
 #pragma unroll
         for (int g = 0; g < 2; g++) {
-            if (!finish<RT_LIMIT>(R, g)) { status |= ST_WATCHDOG; alive = false; break; }
+            if (!finish<GENERAL>(R, g)) { status |= ST_WATCHDOG; alive = false; break; }
             // (1, 2) on the predictor, or (0, 1) of the next step on the new state
             if (g == 0 || step < K) R.inflight[1 - g] = true;
-            if (live[0]) {
-                const int qa = q0, qb = live[1] ? q0 + 1 : q0;
-                const float *ha = R.sH[g] + 3 * qa * GH_STRIDE + jl;
-                const float *hb = R.sH[g] + 3 * qb * GH_STRIDE + jl;
+            if (live[0] && 4 * quad < R.gm[g]) {
+                const float *ha = R.sH[g] + hoff;
+                const float *hb = live[1] ? ha + 3 * GH_STRIDE : ha;
                 const float2 hd[3] = {make_float2(ha[0], hb[0]),
                                       make_float2(ha[GH_STRIDE], hb[GH_STRIDE]),
                                       make_float2(ha[2 * GH_STRIDE], hb[2 * GH_STRIDE])};
@@ -814,25 +839,23 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 for (int64_t s = s_next; s < S; s++)
                     for (int k = 0; k < ITEMS; k++)
                         if (q0 + k < n) {
-                            const int64_t o = s * P + (e0 + GM * g) * n + q0 + k;
+                            const int64_t o = s * P + (e0 + gm0 * g) * n + q0 + k;
                             p.mx[o] = NAN; p.my[o] = NAN; p.mz[o] = NAN;
                         }
     for (int g = 0; g < 2; g++) {
-        bool bad = false;
-        for (int k = 0; k < ITEMS; k++)
-            if (q0 + k < n) {
-                DDf t[3];
-                item_state(t, xh[g], xlt + 3 * g * ITEM_THREADS, k);
-                bad |= !(isfinite(t[0].hi) && isfinite(t[1].hi) && isfinite(t[2].hi));
-            }
+        bool bad = false;  // (a particle past the cluster stays at zero)
+        for (int c = 0; c < 3; c++) bad |= !(isfinite(xh[g][c].x) && isfinite(xh[g][c].y));
         if (valid[g] && bad) atomicOr(&sFlag[GM * g + jl], ST_NONFINITE);
     }
     tc::fence_before_sync();
     __syncthreads();
-    if (threadIdx.x < NM && base + threadIdx.x < p.E) {
-        const int64_t em = base + threadIdx.x;
-        if (p.status) p.status[em] = status | sFlag[threadIdx.x];
-        if (p.steps) p.steps[em] = step;
+    if (threadIdx.x < NM) {
+        const int g = threadIdx.x / GM, j = threadIdx.x % GM;
+        const int64_t em = base + gm0 * g + j;
+        if (j < (g ? gm1 : gm0) && em < p.E) {
+            if (p.status) p.status[em] = status | sFlag[threadIdx.x];
+            if (p.steps) p.steps[em] = step;
+        }
     }
     if (threadIdx.x < 32) {
         tc::fence_after_sync();
@@ -907,12 +930,23 @@ cudaError_t launch_tc(const DevPlan &p, const __half *dhi, const __half *dlo, cu
     if (!tc_supported(p.n)) return cudaErrorNotSupported;
     cudaError_t err = tc_init_attributes();
     if (err != cudaSuccess) return err;
-    const unsigned grid = (unsigned)((p.E + NM - 1) / NM);
+    // Members per CTA: the fewest that need no more waves of CTAs than 32 (a
+    // CTA's step takes less time with fewer: 3.75, 3.9, 4.2 and 4.9 us with 8,
+    // 16, 20 and 32 members of 64 particles, 2.63 and 2.65 with 8 and 32 of 16),
+    // unless a launch shape is set: the groups of a batch share the SMs, and 32 a
+    // CTA cost the least SM time.
+    int nm = NM;
+    if (p.block_warps <= 0) {
+        const int64_t sms = 152, waves = ((p.E + NM - 1) / NM + sms - 1) / sms;
+        while (nm > 8 && (p.E + nm - 5) / (nm - 4) <= waves * sms) nm -= 4;
+    }
+    const int gm0 = (nm / 2 + 3) / 4 * 4, gm1 = nm - gm0;
+    const unsigned grid = (unsigned)((p.E + nm - 1) / nm);
     // the plan's default phase-wait bound is the compile-time one
-    if (p.wait_limit == WAIT_LIMIT)
-        sllg_tc_kernel<false><<<grid, TC_THREADS, tc_layout(p.n).total, stream>>>(p, dhi);
+    if (p.wait_limit == WAIT_LIMIT && !p.noise)
+        sllg_tc_kernel<false><<<grid, TC_THREADS, tc_layout(p.n).total, stream>>>(p, dhi, gm0, gm1);
     else
-        sllg_tc_kernel<true><<<grid, TC_THREADS, tc_layout(p.n).total, stream>>>(p, dhi);
+        sllg_tc_kernel<true><<<grid, TC_THREADS, tc_layout(p.n).total, stream>>>(p, dhi, gm0, gm1);
     return cudaGetLastError();
 }
 
