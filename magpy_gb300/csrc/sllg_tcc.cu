@@ -25,6 +25,14 @@
 //   3. the accumulators, h = acc_main + acc_corr / 2048, go through a shared
 //      field tile to the threads that integrate the CTA's own particles,
 //      which write the next stage's B slab (step 1).
+// Up to three CTAs (65 to 126 particles) the Heun kernel keeps D in tensor
+// memory and has no chunks to stream: B is in every CTA's shared memory, a CTA
+// stores its K slab in its own tile and copies it to its peers' (distributed
+// shared memory), a cluster barrier orders that before the MMAs, and a second
+// one, waited for only after the integration, tells that no tile is read any
+// more.  Streaming B through L2 gave 18 bytes a clock an SM (a 61 KB tile in
+// 3300 clocks of a stage's 9400).  100 particles, 512 members: 10.0 -> 8.8 us a
+// step, 65 particles 9.2 -> 7.6.
 // Everything else -- anisotropy and Zeeman terms, the LLG map, increments
 // from the in-kernel generator, the compensated state, samples -- is the
 // tensor-core kernel's (sllg_tc.cu) per-particle arithmetic, on the same
@@ -53,9 +61,9 @@ namespace {
 constexpr int PPC = 42;           // particles per CTA
 constexpr int RT = 128;           // rows of D per CTA (one MMA tile)
 constexpr int KC = 64;            // K elements per streamed chunk
-constexpr int NS = 3;             // ring stages
+constexpr int NS = 3;             // ring stages (D and B chunks)
 constexpr int PAIRS = PPC / 2;    // particle pairs per CTA
-constexpr int ITEMS = 3;          // pair items per integrating thread
+constexpr int ITEMS = 3;          // pair items per integrating thread (implicit, dipolar field)
 constexpr int TCC_MAX_T = 16;     // CTAs per cluster (non-portable above 8)
 constexpr int FIELD_BLOCK = 32;   // steps of applied field computed at a time (one per lane)
 constexpr uint32_t DRAIN_LIMIT = 1u << 24;
@@ -67,11 +75,13 @@ constexpr int32_t ST_WATCHDOG = 16;
 // and the correction MMA's N = NB rounded up to a multiple of 16 from column
 // NB (for NB = 40, eight columns past 2 NB).
 __host__ __device__ constexpr int tcc_acc_cols(int nb) { return nb + (nb + 15) / 16 * 16; }
-template <int NB> struct Cfg {
-    static constexpr int IT = PAIRS * NB / ITEMS;             // integrating threads (7 NB)
+// NI pair items per integrating thread.
+constexpr int EPI_WARPS = 8;  // epilogue warps (0..7)
+template <int NB, int NI = ITEMS> struct Cfg {
+    static constexpr int COLS = (PAIRS + NI - 1) / NI;        // threads per member
+    static constexpr int IT = COLS * NB;                      // integrating threads
     static constexpr int IW = (IT + 31) / 32;                 // integrating warps
-    static constexpr int EPI = 8;                             // epilogue warps (0..7)
-    static constexpr int PROD = IW > EPI ? IW : EPI;          // producer warp
+    static constexpr int PROD = IW > EPI_WARPS ? IW : EPI_WARPS;  // producer warp
     static constexpr int MMA = PROD + 1;                      // MMA-issuing warp
     static constexpr int THREADS = 32 * (MMA + 1);
     static constexpr int FS = NB + 4;                         // field-tile row stride (floats)
@@ -85,13 +95,17 @@ struct TccLayout {
     int n, T, K, nK, nb;
     size_t a_chunk, b_chunk, stage;  // bytes: D chunk (hi + lo), B chunk, one ring stage
     size_t f_off, par_off, sr_off, flag_off, bar_off, fld_off, total;
+    bool dres;  // D resident in tensor memory: a B tile in place of the ring
 };
 
 __host__ __device__ inline size_t tcc_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
-__host__ __device__ inline TccLayout tcc_layout(int n, int nb)
+// head: bytes before the field tile, 0 for the ring of D and B chunks (with a
+// resident D, a B tile, the stage hand-off and low words).
+__host__ __device__ inline TccLayout tcc_layout(int n, int nb, size_t head = 0)
 {
     TccLayout L;
+    L.dres = head != 0;
     L.n = n;
     L.nb = nb;
     L.T = (n + PPC - 1) / PPC;
@@ -100,7 +114,7 @@ __host__ __device__ inline TccLayout tcc_layout(int n, int nb)
     L.a_chunk = (size_t)2 * RT * KC * 2;
     L.b_chunk = (size_t)2 * nb * KC * 2;
     L.stage = L.a_chunk + L.b_chunk;
-    L.f_off = NS * L.stage;
+    L.f_off = head ? tcc_up(head, 16) : NS * L.stage;
     L.par_off = tcc_up(L.f_off + (size_t)RT * (nb + 4) * 4, 16);
     L.sr_off = L.par_off + (size_t)16 * PPC;
     L.flag_off = tcc_up(L.sr_off + (size_t)4 * PPC, 16);
@@ -156,22 +170,36 @@ struct Pipe {
     uint32_t commits; // MMA thread: completion commits made on accf
     uint32_t limit;
     uint32_t ncols;   // tensor-memory columns allocated
-    uint32_t dcol;    // D resident in tensor memory from this column (0: D streamed)
-    uint32_t sbytes;  // bytes per ring stage: D and B chunks, or B alone when D is resident
-    uint32_t boff;    // offset of the B chunk in a stage
+};
+
+constexpr int DRES_K = 384;  // largest K of a resident D (3 CTAs a cluster)
+
+// Column of tensor memory from which D is resident (past every accumulator
+// column).
+template <int NB> constexpr uint32_t DCOL = tcc_acc_cols(NB);
+
+
+// The MMAs of one 64-deep K chunk: A main and correction descriptors of
+// k-step s from `a`, B at shared address b0.
+template <int NB> struct Idesc {
+    static constexpr uint32_t MAIN = tc::idesc_f16_f32(RT, 2 * NB);
+    // D_lo B_hi into [NB, NB + NC): N a multiple of 16 (for NB = 40 the
+    // last 8 columns multiply the first B_lo rows into accumulator
+    // columns that nothing reads)
+    static constexpr uint32_t CORR = tc::idesc_f16_f32(RT, tcc_acc_cols(NB) - NB);
+    static constexpr uint32_t B_LBO = (2 * NB / 8) * 128;  // between K-adjacent core matrices of B
 };
 
 // D B for this CTA's 128 rows and the NB members of the cluster: the
-// producer thread streams the chunks of B tile `btile` and, unless D is
-// resident in tensor memory (P.dcol != 0), of D tile `dtile`; the MMA thread
-// consumes them.  Returns false in the thread whose wait ran out.  Every
-// thread advances the chunk count.
-template <int NB>
+// producer thread streams the chunks of B tile `btile` and of D tile `dtile`;
+// the MMA thread consumes them.  Returns false in the thread whose wait ran
+// out.  Every thread advances the chunk count.
+template <class C, int NB>
 __device__ inline bool tcc_gemm(Pipe &P, const TccLayout &L, const unsigned char *dtile,
                                 const unsigned char *btile, int warp, int lane)
 {
     bool ok = true;
-    if (warp == Cfg<NB>::PROD && lane == 0) {
+    if (warp == C::PROD && lane == 0) {
         tc::fence_proxy_async_global();  // B slabs written by generic stores (peers: barrier)
         for (int i = 0; i < L.nK; i++) {
             const uint32_t gi = P.g + (uint32_t)i, slot = gi % NS, use = gi / NS;
@@ -179,28 +207,19 @@ __device__ inline bool tcc_gemm(Pipe &P, const TccLayout &L, const unsigned char
                 ok = false;
                 break;
             }
-            unsigned char *st = P.ring + slot * P.sbytes;
+            unsigned char *st = P.ring + slot * (uint32_t)L.stage;
             P.issued = gi + 1;
-            tc::mbar_arrive_expect_tx(&P.full[slot],
-                                      (uint32_t)((P.dcol ? 0 : L.a_chunk) + L.b_chunk));
-            if (!P.dcol)
-                tc::bulk_g2s(st, dtile + (size_t)i * L.a_chunk, (uint32_t)L.a_chunk,
-                             &P.full[slot]);
-            tc::bulk_g2s(st + P.boff, btile + (size_t)i * L.b_chunk, (uint32_t)L.b_chunk,
+            tc::mbar_arrive_expect_tx(&P.full[slot], (uint32_t)L.stage);
+            tc::bulk_g2s(st, dtile + (size_t)i * L.a_chunk, (uint32_t)L.a_chunk, &P.full[slot]);
+            tc::bulk_g2s(st + L.a_chunk, btile + (size_t)i * L.b_chunk, (uint32_t)L.b_chunk,
                          &P.full[slot]);
         }
     }
     // The whole MMA warp runs the chain (warp-uniform operands) and one
     // elected lane issues each MMA and commit.
-    if (warp == Cfg<NB>::MMA) {
-        const uint32_t idesc_main = tc::idesc_f16_f32(RT, 2 * NB);
-        // D_lo B_hi into [NB, NB + NC): N a multiple of 16 (for NB = 40 the
-        // last 8 columns multiply the first B_lo rows into accumulator
-        // columns that nothing reads)
-        constexpr uint32_t NC = tcc_acc_cols(NB) - NB;
-        const uint32_t idesc_corr = tc::idesc_f16_f32(RT, NC);
+    if (warp == C::MMA) {
         const uint32_t a_sbo = (KC / 8) * 128;        // between 8-row groups of D
-        const uint32_t b_lbo = (2 * NB / 8) * 128;    // between K-adjacent core matrices of B
+        constexpr uint32_t b_lbo = Idesc<NB>::B_LBO;
         for (int i = 0; i < L.nK; i++) {
             const uint32_t gi = P.g + (uint32_t)i, slot = gi % NS, use = gi / NS;
             if (!__all_sync(0xffffffffu,
@@ -209,29 +228,15 @@ __device__ inline bool tcc_gemm(Pipe &P, const TccLayout &L, const unsigned char
                 break;
             }
             tc::fence_after_sync();
-            const uint32_t a0 = tc::smem_addr(P.ring + slot * P.sbytes);
-            const uint32_t b0 = a0 + P.boff;
-            if (P.dcol) {
-                // A from tensor memory: K element k of split sp in column
-                // dcol + sp K/2 + k/2
-                const uint32_t ahi = P.tmem + P.dcol + (uint32_t)(KC / 2 * i);
-                const uint32_t alo = ahi + (uint32_t)(L.K / 2);
+            const uint32_t a0 = tc::smem_addr(P.ring + slot * (uint32_t)L.stage);
+            const uint32_t b0 = a0 + (uint32_t)L.a_chunk;
 #pragma unroll
-                for (int s = 0; s < KC / 16; s++) {
-                    const uint64_t bd = tc::smem_desc(b0 + 2u * b_lbo * s, b_lbo, 128);
-                    tc::mma_f16_ta_warp(P.tmem, ahi + 8u * s, bd, idesc_main,
-                                        (i > 0 || s > 0) ? 1u : 0u);
-                    tc::mma_f16_ta_warp(P.tmem + NB, alo + 8u * s, bd, idesc_corr, 1u);
-                }
-            } else {
-#pragma unroll
-                for (int s = 0; s < KC / 16; s++) {
-                    const uint64_t ahi = tc::smem_desc(a0 + 256u * s, 128, a_sbo);
-                    const uint64_t alo = tc::smem_desc(a0 + RT * KC * 2 + 256u * s, 128, a_sbo);
-                    const uint64_t bd = tc::smem_desc(b0 + 2u * b_lbo * s, b_lbo, 128);
-                    tc::mma_f16_warp(P.tmem, ahi, bd, idesc_main, (i > 0 || s > 0) ? 1u : 0u);
-                    tc::mma_f16_warp(P.tmem + NB, alo, bd, idesc_corr, 1u);
-                }
+            for (int s = 0; s < KC / 16; s++) {
+                const uint64_t ahi = tc::smem_desc(a0 + 256u * s, 128, a_sbo);
+                const uint64_t alo = tc::smem_desc(a0 + RT * KC * 2 + 256u * s, 128, a_sbo);
+                const uint64_t bd = tc::smem_desc(b0 + 2u * b_lbo * s, b_lbo, 128);
+                tc::mma_f16_warp(P.tmem, ahi, bd, Idesc<NB>::MAIN, (i > 0 || s > 0) ? 1u : 0u);
+                tc::mma_f16_warp(P.tmem + NB, alo, bd, Idesc<NB>::CORR, 1u);
             }
             tc::mma_commit_warp(&P.empty[slot]);
         }
@@ -242,6 +247,28 @@ __device__ inline bool tcc_gemm(Pipe &P, const TccLayout &L, const unsigned char
     return ok;
 }
 
+// The same product with D in tensor memory and the whole B tile in shared
+// memory (at the start of the ring): K element k of D's split sp is in column
+// DCOL + sp K/2 + k/2.
+template <class C, int NB>
+__device__ inline void tcc_gemm_resident(Pipe &P, const TccLayout &L, int warp)
+{
+    if (warp != C::MMA) return;
+    tc::fence_proxy_async_cluster();
+    tc::fence_after_sync();
+    constexpr uint32_t b_lbo = Idesc<NB>::B_LBO;
+    const uint32_t b0 = tc::smem_addr(P.ring);
+    const uint32_t ahi = P.tmem + DCOL<NB>, alo = ahi + (uint32_t)(L.K / 2);
+#pragma unroll 2
+    for (int s = 0; s < L.K / 16; s++) {
+        const uint64_t bd = tc::smem_desc(b0 + 2u * b_lbo * s, b_lbo, 128);
+        tc::mma_f16_ta_warp(P.tmem, ahi + 8u * s, bd, Idesc<NB>::MAIN, s > 0 ? 1u : 0u);
+        tc::mma_f16_ta_warp(P.tmem + NB, alo + 8u * s, bd, Idesc<NB>::CORR, 1u);
+    }
+    tc::mma_commit_warp(P.accf);
+    P.commits++;
+}
+
 // Accumulators -> field tile F[row][member] (epilogue warps 0..7: lane quarter
 // warp % 4, member half warp / 4).  Returns false if the completion did not
 // arrive in time.
@@ -249,7 +276,7 @@ template <int NB>
 __device__ inline bool tcc_epilogue(Pipe &P, float *F, int warp, int lane)
 {
     bool ok = true;
-    if (warp < Cfg<NB>::EPI) {
+    if (warp < EPI_WARPS) {
         ok = __all_sync(0xffffffffu, tc::mbar_wait_bounded(P.accf, P.gemms & 1u, P.limit));
         tc::fence_after_sync();
         if (ok) {
@@ -325,21 +352,62 @@ __device__ inline void put_pair_g(__half *btile, int r, int p, int j, bool live0
     }
 }
 
-__device__ inline void tcc_write_sample(const DevPlan &p, int64_t s, int64_t e, int n, int q,
-                                        const DDf xk[3])
+// The same into the CTA's own slab of a B tile in shared memory.  Eight
+// members by four pairs a warp: 32 different banks.
+template <int NB>
+__device__ inline void put_pair_s(__half *slab, int p, int j, bool live0, bool live1,
+                                  const float m[6])
 {
-    const int64_t o = s * p.P + e * n + q;
-    const double sc = p.out_scale[e];
-    p.mx[o] = ((double)xk[0].hi + (double)xk[0].lo) * sc;
-    p.my[o] = ((double)xk[1].hi + (double)xk[1].lo) * sc;
-    p.mz[o] = ((double)xk[2].hi + (double)xk[2].lo) * sc;
+    if (!live0) return;
+#pragma unroll
+    for (int w = 0; w < 3; w++) {
+        if (w == 2 && !live1) break;
+        put_word_g<NB>(slab, j, 6 * p + 2 * w, m[2 * w], (w == 1 && !live1) ? 0.f : m[2 * w + 1]);
+    }
+}
+
+// This CTA's slab of the B tile to the same place in the cluster's other CTAs.
+template <class C, int NB>
+__device__ inline void push_slab(const unsigned char *slab, int r, int T)
+{
+    constexpr int V = RT * 2 * NB * 2 / 16;
+    const uint32_t a0 = tc::smem_addr(slab);
+    for (int v = threadIdx.x; v < V; v += C::THREADS) {
+        const uint4 x = reinterpret_cast<const uint4 *>(slab)[v];
+        for (int k = 1; k < T; k++) {
+            const int rr = r + k < T ? r + k : r + k - T;
+            tc::st_cluster_v4(tc::mapa(a0 + 16u * v, (uint32_t)rr), x);
+        }
+    }
+}
+
+// One particle's sample: x = (hi + lo) sc, o its index in a component's
+// [S][P] planes.  Not inlined, as field_block is not: what a step rarely runs
+// is kept out of the step loop's code.
+__device__ __noinline__ void tcc_write_sample(double *mx, double *my, double *mz, int64_t o,
+                                              double sc, float xh, float xl, float yh, float yl,
+                                              float zh, float zl)
+{
+    mx[o] = ((double)xh + (double)xl) * sc;
+    my[o] = ((double)yh + (double)yl) * sc;
+    mz[o] = ((double)zh + (double)zl) * sc;
+}
+
+// The applied field of step FIELD_BLOCK b + 1 + lane, at t or (second) t + dt.
+__device__ __noinline__ void tcc_field_block(float2 *sF2, const MemberDev *md, int64_t b, int64_t K,
+                                             int second)
+{
+    const int lane = threadIdx.x & 31;
+    const int64_t k = FIELD_BLOCK * b + 1 + lane;
+    if (k <= K)
+        reinterpret_cast<float *>(sF2 + FIELD_BLOCK * (b & 1) + lane)[second] =
+            f64::heun_field_f32(md->shape, md->dt, md->happ, md->fapp, k, second);
 }
 
 // Common set-up of a CTA: shared-memory carve-up, mbarriers, tensor memory
-// (the accumulators, and D when `dres`: then 512 columns).
+// (the accumulators, and D when it is resident: then 512 columns).
 template <int NB>
-__device__ inline void tcc_setup(Pipe &P, unsigned char *sm, const TccLayout &L, uint32_t limit,
-                                 bool dres = false)
+__device__ inline void tcc_setup(Pipe &P, unsigned char *sm, const TccLayout &L, uint32_t limit)
 {
     P.ring = sm;
     P.full = (uint64_t *)(sm + L.bar_off);
@@ -351,11 +419,7 @@ __device__ inline void tcc_setup(Pipe &P, unsigned char *sm, const TccLayout &L,
     P.issued = 0;
     P.commits = 0;
     P.limit = limit;
-    P.ncols = dres ? 512u : Cfg<NB>::TMEM_COLS;
-    P.dcol = dres ? (uint32_t)tcc_acc_cols(NB) : 0u;  // past every accumulator column
-    // with D resident the ring holds B chunks only, packed at its start
-    P.sbytes = (uint32_t)(dres ? L.b_chunk : L.stage);
-    P.boff = dres ? 0u : (uint32_t)L.a_chunk;
+    P.ncols = L.dres ? 512u : Cfg<NB>::TMEM_COLS;
     if (threadIdx.x == 0) {
         for (int i = 0; i < NS; i++) {
             tc::mbar_init(&P.full[i], 1);
@@ -372,7 +436,7 @@ __device__ inline void tcc_setup(Pipe &P, unsigned char *sm, const TccLayout &L,
 
 // D tile (global, [chunk][split][128 x KC, row groups outermost]) into tensor
 // memory for the MMAs' A operand: row r in lane r, split sp's K element k in
-// column dcol + sp K/2 + k/2 (two 16-bit elements per column, the even K in
+// column DCOL + sp K/2 + k/2 (two 16-bit elements per column, the even K in
 // the low half).  Warps 0..7: lane quarter warp % 4, split warp / 4.  Ends
 // with the stores complete; a CTA barrier must follow before the first MMA.
 template <int NB>
@@ -392,7 +456,7 @@ __device__ inline void tcc_load_d_tmem(const Pipe &P, const TccLayout &L, const 
                                 tc::cm_offset_rows(row, (uint32_t)kk, KC);
             v[c] = *reinterpret_cast<const uint32_t *>(src);
         }
-        tc::tmem_st8(P.tmem + lanes + P.dcol + (uint32_t)(sp * (L.K / 2) + c0), v);
+        tc::tmem_st8(P.tmem + lanes + DCOL<NB> + (uint32_t)(sp * (L.K / 2) + c0), v);
     }
     tc::tmem_st_wait();
     tc::fence_before_sync();
@@ -400,15 +464,15 @@ __device__ inline void tcc_load_d_tmem(const Pipe &P, const TccLayout &L, const 
 
 // Before the tensor memory is released: the producer waits (long bound) for
 // the copies it issued, the MMA thread for its MMAs (the last commit).
-template <int NB>
+template <class C>
 __device__ inline void tcc_drain(Pipe &P, int warp, int lane)
 {
-    if (warp == Cfg<NB>::PROD && lane == 0)
+    if (warp == C::PROD && lane == 0)
         for (uint32_t k = 0; k < (uint32_t)NS && k < P.issued; k++) {
             const uint32_t gi = P.issued - 1 - k;  // the last copy into each slot
             tc::mbar_wait_bounded(&P.full[gi % NS], (gi / NS) & 1u, DRAIN_LIMIT);
         }
-    if (warp == Cfg<NB>::MMA && lane == 0 && P.commits > 0)
+    if (warp == C::MMA && lane == 0 && P.commits > 0)
         tc::mbar_wait_bounded(P.accf, (P.commits - 1) & 1u, DRAIN_LIMIT);
     tc::fence_before_sync();
     __syncthreads();
@@ -433,26 +497,41 @@ __device__ inline int cluster_any_error(int *sErr, int T)
 }
 
 // ---- the integrator ----
-// Thread t < IT integrates, for member j = t % NB of the cluster's tile, the
-// CTA-local particle pairs p = t / NB + 7 i (i < 3), so consecutive threads
-// read consecutive members of a field-tile row.
+// Eight consecutive threads serve eight consecutive members j of the
+// cluster's tile, the next eight threads the next pair column p0 of COLS, then
+// the next eight members; a thread integrates the CTA-local particle pairs
+// p = p0 + COLS i.  A warp's reads of the field tile (8 members x 4 pairs, rows
+// 6 (NB + 4) floats apart) then fall into 32 different banks.
+template <int NB, bool DRES> constexpr int HEUN_ITEMS = NB <= 48 ? 2 : 3;
+template <int NB, bool DRES> using HeunCfg = Cfg<NB, HEUN_ITEMS<NB, DRES>>;
+// state low words in shared memory
+template <int NB, bool DRES> constexpr bool HEUN_LO = DRES && NB <= 48;
+
+// Bytes before the field tile when D is resident: a whole B tile, the stage
+// hand-off and the states' low words.
+template <int NB> constexpr size_t heun_head()
+{
+    return (size_t)DRES_K * 2 * NB * 2 +
+           (size_t)4 * (HEUN_LO<NB, true> ? 18 : 12) * HEUN_ITEMS<NB, true> * HeunCfg<NB, true>::IT;
+}
+
 template <int NB, bool DRES>
-__global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
+__global__ void __launch_bounds__(HeunCfg<NB, DRES>::THREADS, 1)
     sllg_tcc_kernel(DevPlan p, const __half *dglob, __half *bglob, int64_t tiles)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
-    using C = Cfg<NB>;
+    using C = HeunCfg<NB, DRES>;
+    constexpr int ITEMS = HEUN_ITEMS<NB, DRES>;
     const int n = p.n;
-    const TccLayout L = tcc_layout(n, NB);
+    const TccLayout L = tcc_layout(n, NB, DRES ? heun_head<NB>() : 0);
     const int r = (int)tc::cluster_ctarank();
     const int64_t tile = (int64_t)blockIdx.x / L.T;
     Pipe P;
     // DRES (up to three CTAs per cluster, n <= 126): the D tile fits in
-    // tensor memory beside the accumulators, is loaded once and only B is
-    // streamed; the ring's D slots are then free and hold the stage hand-off
-    // instead of registers
-    const bool dres = DRES;
-    tcc_setup<NB>(P, sm, L, p.wait_limit, dres);
+    // tensor memory beside the accumulators and is loaded once, the B tile is in
+    // every CTA's shared memory (each CTA stores its slab there and to its
+    // peers), and so is the stage hand-off instead of in registers
+    tcc_setup<NB>(P, sm, L, p.wait_limit);
     float *F = (float *)(sm + L.f_off);
     float4 *sPar = (float4 *)(sm + L.par_off);
     float *sSr = (float *)(sm + L.sr_off);
@@ -479,8 +558,15 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
     __half *B0 = bglob + (size_t)tile * tile_elems;               // states
     __half *B1 = bglob + (size_t)(tiles + tile) * tile_elems;     // predictors
     const unsigned char *dtile = (const unsigned char *)dglob + (size_t)r * L.nK * L.a_chunk;
-    // (ordered before the first MMA by the CTA and cluster barriers below)
-    if (dres) tcc_load_d_tmem<NB>(P, L, (const __half *)dtile, warp, lane);
+    __half *slab = (__half *)sm + (size_t)r * RT * 2 * NB;  // DRES: this CTA's part of B
+    if constexpr (DRES) {
+        // (ordered before the first MMA by the CTA and cluster barriers below)
+        tcc_load_d_tmem<NB>(P, L, (const __half *)dtile, warp, lane);
+        uint4 *bz = (uint4 *)sm;  // padding, absent particles and members stay zero
+        for (int i = threadIdx.x; i < DRES_K * 2 * NB * 2 / 16; i += blockDim.x)
+            bz[i] = make_uint4(0, 0, 0, 0);
+        __syncthreads();
+    }
     const float dt = (float)m0d->dt, sq = (float)m0d->sqrt_dt, alpha = (float)m0d->alpha;
     const bool renorm = m0d->renorm != 0;
     const int64_t S = p.S;
@@ -489,43 +575,48 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
     const int64_t per_step = 3 * (int64_t)n;
 
     const bool integ = (int)threadIdx.x < C::IT;
-    const int j = (int)threadIdx.x % NB;
-    const int p0 = (int)threadIdx.x / NB;
+    const int j = 8 * ((int)threadIdx.x / (8 * C::COLS)) + ((int)threadIdx.x & 7);
+    const int p0 = ((int)threadIdx.x >> 3) % C::COLS;
     const int64_t e = tile * NB + j;
     const bool valid = integ && e < p.E;
     const uint64_t seed = valid ? p.members[e].seed : 0;
     const double *noise = (p.noise && valid) ? p.noise + p.members[e].noise_off : nullptr;
     bool live[ITEMS][2];
     // state: float-float per component, the high words in registers; the
-    // low words (read and written once per step) in the D ring's freed
-    // space when D is resident and there is room (up to 48 members), else
-    // in registers
-    constexpr bool LO_SMEM = DRES && NB <= 48;
+    // low words (read and written once per step) in shared memory when D is
+    // resident and there is room (up to 48 members), else in registers
+    constexpr bool LO_SMEM = HEUN_LO<NB, DRES>;
     float xh[ITEMS][2][3], xlr[LO_SMEM ? 1 : ITEMS][2][3];
     // stage hand-off per pair item: A = F(m, v1)/2 and the increments W
     float Areg[ITEMS][6], Wreg[ITEMS][6];
-    float *hand = (float *)(sm + NS * L.b_chunk);  // DRES: [24 ITEMS][THREADS]
+    float *hand = (float *)(sm + DRES_K * 2 * NB * 2);  // DRES: [12 ITEMS][IT]
     auto HA = [&](int i, int c) -> float & {
-        if constexpr (DRES) return hand[(i * 6 + c) * C::THREADS + threadIdx.x];
+        if constexpr (DRES) return hand[(i * 6 + c) * C::IT + threadIdx.x];
         else return Areg[i][c];
     };
     auto HW = [&](int i, int c) -> float & {
-        if constexpr (DRES) return hand[((ITEMS + i) * 6 + c) * C::THREADS + threadIdx.x];
+        if constexpr (DRES) return hand[((ITEMS + i) * 6 + c) * C::IT + threadIdx.x];
         else return Wreg[i][c];
     };
-    float *xlo = hand + 2 * ITEMS * 6 * C::THREADS;  // LO_SMEM: [ITEMS 2 3][THREADS]
+    float *xlo = hand + 2 * ITEMS * 6 * C::IT;  // LO_SMEM: [ITEMS 2 3][IT]
     auto XL = [&](int i, int k, int c) -> float & {
-        if constexpr (LO_SMEM) return xlo[((i * 2 + k) * 3 + c) * C::THREADS + threadIdx.x];
+        if constexpr (LO_SMEM) return xlo[((i * 2 + k) * 3 + c) * C::IT + threadIdx.x];
         else return xlr[LO_SMEM ? 0 : i][k][c];
     };
-    auto item = [&](DDf out[3], int i, int k) {
-        for (int c = 0; c < 3; c++) out[c] = DDf{xh[i][k][c], XL(i, k, c)};
+    auto record = [&](int64_t smp) {
+        for (int i = 0; i < ITEMS; i++)
+            for (int k = 0; k < 2; k++)
+                if (live[i][k])
+                    tcc_write_sample(p.mx, p.my, p.mz,
+                                     smp * P_ + e * n + PPC * r + 2 * (p0 + C::COLS * i) + k,
+                                     p.out_scale[e], xh[i][k][0], XL(i, k, 0), xh[i][k][1],
+                                     XL(i, k, 1), xh[i][k][2], XL(i, k, 2));
     };
 #pragma unroll
     for (int i = 0; i < ITEMS; i++) {
-        const int q0 = PPC * r + 2 * (p0 + 7 * i);
-        live[i][0] = valid && q0 < n;
-        live[i][1] = valid && q0 + 1 < n;
+        const int q0 = PPC * r + 2 * (p0 + C::COLS * i);
+        live[i][0] = valid && p0 + C::COLS * i < PAIRS && q0 < n;
+        live[i][1] = live[i][0] && q0 + 1 < n;
 #pragma unroll
         for (int k = 0; k < 2; k++)
 #pragma unroll
@@ -537,24 +628,19 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
                     lo = (float)(v - (double)hi);
                 }
                 xh[i][k][c] = hi;
-                XL(i, k, c) = lo;
+                if (integ) XL(i, k, c) = lo;
             }
     }
     // initial state -> B0, sample 0 (lib/simulation.cpp:212-219)
 #pragma unroll
     for (int i = 0; i < ITEMS; i++) {
-        const int pl = p0 + 7 * i;
+        const int pl = p0 + C::COLS * i;
         const float m6[6] = {xh[i][0][0], xh[i][0][1], xh[i][0][2],
                              xh[i][1][0], xh[i][1][1], xh[i][1][2]};
-        put_pair_g<NB>(B0, r, pl, j, live[i][0], live[i][1], m6);
-        if (p.mx)
-            for (int k = 0; k < 2; k++)
-                if (live[i][k]) {
-                    DDf t[3];
-                    item(t, i, k);
-                    tcc_write_sample(p, 0, e, n, PPC * r + 2 * pl + k, t);
-                }
+        if constexpr (DRES) put_pair_s<NB>(slab, pl, j, live[i][0], live[i][1], m6);
+        else put_pair_g<NB>(B0, r, pl, j, live[i][0], live[i][1], m6);
     }
+    if (p.mx) record(0);
     // The producer and MMA warps compute the applied field, FIELD_BLOCK steps
     // at a time (lane l: step 32 b + 1 + l of block b; the producer warp at t,
     // the MMA warp at t + dt; an FP64 sine takes ~1.6 k cycles on this part's
@@ -563,15 +649,10 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
     // many barriers) later, and the slot it overwrites (block b - 1) was last
     // read a step (and several barriers) earlier.
     auto field_block = [&](int64_t b) {
-        if (warp == C::PROD || warp == C::MMA) {
-            const int second = warp == C::MMA;
-            const int64_t k = FIELD_BLOCK * b + 1 + lane;
-            if (k <= K)
-                reinterpret_cast<float *>(sF2 + FIELD_BLOCK * (b & 1) + lane)[second] =
-                    f64::heun_field_f32(m0d->shape, m0d->dt, m0d->happ, m0d->fapp, k, second);
-        }
+        if (warp == C::PROD || warp == C::MMA) tcc_field_block(sF2, m0d, b, K, warp == C::MMA);
     };
     field_block(0);
+    if constexpr (DRES) tc::cluster_sync();  // every CTA's tile is zeroed
     __syncthreads();
 
     int32_t status = ST_OK;
@@ -592,15 +673,7 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
         if (!stop && step > noise_steps) { status |= ST_NOISE_EXHAUSTED; stop = true; }
         if (stop) break;
         while (next_sample == step) {
-            if (p.mx)
-#pragma unroll
-                for (int i = 0; i < ITEMS; i++)
-                    for (int k = 0; k < 2; k++)
-                        if (live[i][k]) {
-                            DDf t[3];
-                            item(t, i, k);
-                            tcc_write_sample(p, s_next, e, n, PPC * r + 2 * (p0 + 7 * i) + k, t);
-                        }
+            if (p.mx) record(s_next);
             s_next++;
             next_sample = s_next < S ? sched[s_next] : -1;
         }
@@ -610,26 +683,35 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
         const float h1 = hf.x, h2 = hf.y;
 #pragma unroll 1
         for (int stage = 0; stage < 2; stage++) {
-            // every CTA's slab of this stage's B tile is written
-            tc::fence_proxy_async_global();
-            tc::cluster_sync();
-            const __half *Bin = stage == 0 ? B0 : B1;
             bool ok = true;
-            // a CTA whose pipeline broke skips its waits (read once per warp:
-            // the MMA warp's collectives need the whole warp)
-            if (__shfl_sync(0xffffffffu, *sErr, 0) == 0)
-                ok = tcc_gemm<NB>(P, L, dtile, (const unsigned char *)(Bin + 0), warp, lane);
-            else
-                P.g += (uint32_t)L.nK;
+            if constexpr (DRES) {
+                // no CTA reads its B tile any more (the wait at the stage's end)
+                push_slab<C, NB>((const unsigned char *)slab, r, L.T);
+                tc::fence_proxy_async_cluster();
+                tc::cluster_sync();
+                if (__shfl_sync(0xffffffffu, *sErr, 0) == 0) tcc_gemm_resident<C, NB>(P, L, warp);
+            } else {
+                // every CTA's slab of this stage's B tile is written
+                tc::fence_proxy_async_global();
+                tc::cluster_sync();
+                const __half *Bin = stage == 0 ? B0 : B1;
+                // a CTA whose pipeline broke skips its waits (read once per warp:
+                // the MMA warp's collectives need the whole warp)
+                if (__shfl_sync(0xffffffffu, *sErr, 0) == 0)
+                    ok = tcc_gemm<C, NB>(P, L, dtile, (const unsigned char *)Bin, warp, lane);
+                else
+                    P.g += (uint32_t)L.nK;
+            }
             ok = (*sErr == 0 ? tcc_epilogue<NB>(P, F, warp, lane) : (P.gemms++, true)) && ok;
             if (!ok) atomicOr(sErr, 1);
             __syncthreads();
+            if constexpr (DRES) tc::cluster_arrive();  // this CTA no longer reads its B tile
             __half *Bout = stage == 0 ? B1 : B0;
             const float hz = stage == 0 ? h1 : h2;
             if (integ) {
 #pragma unroll
                 for (int i = 0; i < ITEMS; i++) {
-                    const int pl = p0 + 7 * i;
+                    const int pl = p0 + C::COLS * i;
                     PairNormals wn;
                     if (stage == 0 && !noise && live[i][0])
                         wn = wiener_pair(seed, (uint64_t)step, (uint32_t)(PAIRS * r + pl));
@@ -703,8 +785,15 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
                             m6[3 * k + 2] = xh[i][k][2];
                         }
                     }
-                    put_pair_g<NB>(Bout, r, pl, j, live[i][0], live[i][1], m6);
+                    if constexpr (DRES) put_pair_s<NB>(slab, pl, j, live[i][0], live[i][1], m6);
+                    else put_pair_g<NB>(Bout, r, pl, j, live[i][0], live[i][1], m6);
                 }
+            }
+            if constexpr (DRES) {
+                tc::fence_proxy_async_cluster();
+                __syncwarp();
+                tc::cluster_wait();
+                __syncthreads();
             }
         }
     }
@@ -719,7 +808,7 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
             for (int i = 0; i < ITEMS; i++)
                 for (int k = 0; k < 2; k++)
                     if (live[i][k]) {
-                        const int64_t o = s * P_ + e * n + PPC * r + 2 * (p0 + 7 * i) + k;
+                        const int64_t o = s * P_ + e * n + PPC * r + 2 * (p0 + C::COLS * i) + k;
                         p.mx[o] = NAN; p.my[o] = NAN; p.mz[o] = NAN;
                     }
     bool bad = false;
@@ -730,7 +819,7 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
                 bad |= !(isfinite(xh[i][k][0]) && isfinite(xh[i][k][1]) &&
                          isfinite(xh[i][k][2]));
     if (bad) atomicOr(&sFlag[j], ST_NONFINITE);
-    tcc_drain<NB>(P, warp, lane);
+    tcc_drain<C>(P, warp, lane);
     // member status: the OR over the cluster's CTAs, written by CTA 0
     tc::cluster_sync();
     if (r == 0 && threadIdx.x < NB && tile * NB + threadIdx.x < p.E) {
@@ -775,7 +864,7 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
     }
     tc::fence_proxy_async_global();
     tc::cluster_sync();
-    bool ok = tcc_gemm<NB>(P, L, dtile, (const unsigned char *)Bt, warp, lane);
+    bool ok = tcc_gemm<C, NB>(P, L, dtile, (const unsigned char *)Bt, warp, lane);
     ok = tcc_epilogue<NB>(P, F, warp, lane) && ok;
     if (__syncthreads_or(!ok)) {
         if (threadIdx.x == 0) atomicOr(flag, 1);
@@ -789,7 +878,7 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
                     h[(e * n + q) * 3 + c] = (double)F[(3 * lq + c) * C::FS + j];
         }
     }
-    tcc_drain<NB>(P, warp, lane);
+    tcc_drain<C>(P, warp, lane);
     tc::cluster_sync();
 }
 
@@ -984,7 +1073,7 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
     auto field = [&]() {
         bool ok = true;
         if (__shfl_sync(0xffffffffu, *sErr, 0) == 0)
-            ok = tcc_gemm<NB>(P, L, dtile, (const unsigned char *)Bbuf[wb], warp, lane);
+            ok = tcc_gemm<C, NB>(P, L, dtile, (const unsigned char *)Bbuf[wb], warp, lane);
         else P.g += (uint32_t)L.nK;
         ok = (*sErr == 0 ? tcc_epilogue<NB>(P, F, warp, lane) : (P.gemms++, true)) && ok;
         if (!ok) atomicOr(sErr, 1);
@@ -1192,7 +1281,7 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
                 bad |= !(isfinite(x[i][k][0]) && isfinite(x[i][k][1]) && isfinite(x[i][k][2]));
     if (bad) atomicOr(&sFlag[j], ST_NONFINITE);
     if (integ && valid && status) atomicOr(&sFlag[j], status);
-    tcc_drain<NB>(P, warp, lane);
+    tcc_drain<C>(P, warp, lane);
     tc::cluster_sync();
     if (r == 0 && threadIdx.x < NB && tile * NB + threadIdx.x < p.E) {
         const int64_t em = tile * NB + threadIdx.x;
@@ -1238,6 +1327,20 @@ cudaError_t tcc_launch(Kern kern, const TccLayout &L, size_t smem, int threads, 
     cfg.attrs = attr;
     cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+// Shared memory of the Heun kernel with a resident D (the same for any n).
+template <int NB> size_t heun_smem() { return tcc_layout(2 * PPC, NB, heun_head<NB>()).total; }
+
+template <int NB>
+cudaError_t tcc_launch_heun(const DevPlan &p, const __half *d, __half *b, const TccLayout &L,
+                            bool dres, int64_t tiles, cudaStream_t stream)
+{
+    if (dres)
+        return tcc_launch(sllg_tcc_kernel<NB, true>, L, heun_smem<NB>(),
+                          HeunCfg<NB, true>::THREADS, tiles, stream, p, d, b, tiles);
+    return tcc_launch(sllg_tcc_kernel<NB, false>, L, L.total, HeunCfg<NB, false>::THREADS, tiles,
+                      stream, p, d, b, tiles);
 }
 
 }  // namespace
@@ -1288,7 +1391,7 @@ cudaError_t tcc_init(int n, int nb, int *max_clusters)
     if (!done[dev][w] && nb == 40) {
         err = tcc_prepare(sllg_tcc_implicit_kernel<40>, Lmax, imp);
         if (err == cudaSuccess) err = tcc_prepare(sllg_tcc_kernel<40, false>, Lmax, Lmax.total);
-        if (err == cudaSuccess) err = tcc_prepare(sllg_tcc_kernel<40, true>, Lmax, Lmax.total);
+        if (err == cudaSuccess) err = tcc_prepare(sllg_tcc_kernel<40, true>, Lmax, heun_smem<40>());
         if (err != cudaSuccess) return err;
         done[dev][w] = true;
     }
@@ -1296,12 +1399,12 @@ cudaError_t tcc_init(int n, int nb, int *max_clusters)
         err = nb == 32 ? tcc_prepare(sllg_tcc_kernel<32, false>, Lmax, Lmax.total)
                        : tcc_prepare(sllg_tcc_kernel<64, false>, Lmax, Lmax.total);
         if (err == cudaSuccess)
-            err = nb == 32 ? tcc_prepare(sllg_tcc_kernel<32, true>, Lmax, Lmax.total)
-                           : tcc_prepare(sllg_tcc_kernel<64, true>, Lmax, Lmax.total);
+            err = nb == 32 ? tcc_prepare(sllg_tcc_kernel<32, true>, Lmax, heun_smem<32>())
+                           : tcc_prepare(sllg_tcc_kernel<64, true>, Lmax, heun_smem<64>());
         if (err == cudaSuccess && nb == 64) {  // the 48-member form, prepared alongside
             const TccLayout L48 = tcc_layout(PPC * TCC_MAX_T, 48);
             err = tcc_prepare(sllg_tcc_kernel<48, false>, L48, L48.total);
-            if (err == cudaSuccess) err = tcc_prepare(sllg_tcc_kernel<48, true>, L48, L48.total);
+            if (err == cudaSuccess) err = tcc_prepare(sllg_tcc_kernel<48, true>, L48, heun_smem<48>());
         }
         if (err == cudaSuccess)
             err = nb == 32 ? tcc_prepare(tcc_dipolar_kernel<32>, Lmax, Lmax.total)
@@ -1354,25 +1457,12 @@ cudaError_t launch_tcc(const DevPlan &p, const __half *d, __half *b, int nb, cud
     }
     if (!tcc_supported(p.n)) return cudaErrorNotSupported;
     const bool dres = tcc_acc_cols(nb) + L.K <= 512;
-    if (nb == 40)
-        return dres ? tcc_launch(sllg_tcc_kernel<40, true>, L, L.total, Cfg<40>::THREADS, tiles,
-                                 stream, p, d, b, tiles)
-                    : tcc_launch(sllg_tcc_kernel<40, false>, L, L.total, Cfg<40>::THREADS, tiles,
-                                 stream, p, d, b, tiles);
-    if (nb == 48)
-        return dres ? tcc_launch(sllg_tcc_kernel<48, true>, L, L.total, Cfg<48>::THREADS, tiles,
-                                 stream, p, d, b, tiles)
-                    : tcc_launch(sllg_tcc_kernel<48, false>, L, L.total, Cfg<48>::THREADS, tiles,
-                                 stream, p, d, b, tiles);
-    if (nb == 32)
-        return dres ? tcc_launch(sllg_tcc_kernel<32, true>, L, L.total, Cfg<32>::THREADS, tiles,
-                                 stream, p, d, b, tiles)
-                    : tcc_launch(sllg_tcc_kernel<32, false>, L, L.total, Cfg<32>::THREADS, tiles,
-                                 stream, p, d, b, tiles);
-    return dres ? tcc_launch(sllg_tcc_kernel<64, true>, L, L.total, Cfg<64>::THREADS, tiles,
-                             stream, p, d, b, tiles)
-                : tcc_launch(sllg_tcc_kernel<64, false>, L, L.total, Cfg<64>::THREADS, tiles,
-                             stream, p, d, b, tiles);
+    switch (nb) {
+    case 32: return tcc_launch_heun<32>(p, d, b, L, dres, tiles, stream);
+    case 40: return tcc_launch_heun<40>(p, d, b, L, dres, tiles, stream);
+    case 48: return tcc_launch_heun<48>(p, d, b, L, dres, tiles, stream);
+    default: return tcc_launch_heun<64>(p, d, b, L, dres, tiles, stream);
+    }
 }
 
 cudaError_t launch_tcc_dipolar(const __half *d, __half *b, int n, int64_t E, const double *m,

@@ -47,6 +47,18 @@ __device__ inline void cluster_sync()
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// The two halves of that barrier: a CTA may work between its arrival and its
+// wait.  Arrivals and waits alternate.
+__device__ inline void cluster_arrive()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+
+__device__ inline void cluster_wait()
+{
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // Address of the same shared-memory location in CTA `rank` of the cluster.
 __device__ inline uint32_t mapa(uint32_t saddr, uint32_t rank)
 {
@@ -67,6 +79,21 @@ __device__ inline int32_t ld_cluster_s32(uint32_t caddr)
     int32_t v;
     asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(caddr) : "memory");
     return v;
+}
+
+__device__ inline void st_cluster_v4(uint32_t caddr, uint4 v)
+{
+    asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};"
+                 :
+                 : "r"(caddr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
+                 : "memory");
+}
+
+// Orders this thread's generic-proxy accesses to the cluster's shared memory
+// with async-proxy (MMA operand) accesses, both ways.
+__device__ inline void fence_proxy_async_cluster()
+{
+    asm volatile("fence.proxy.async.shared::cluster;" ::: "memory");
 }
 
 // Orders this thread's generic-proxy global accesses with its async-proxy

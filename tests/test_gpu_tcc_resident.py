@@ -1,0 +1,27 @@
+"""The cluster Heun kernel for 65 to 126 particles (two or three CTAs a cluster,
+the moments of a member tile in every CTA's shared memory)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nb", [32, 40, 48, 64])
+@pytest.mark.parametrize("n,E", [(65, 1), (83, 33), (84, 64), (85, 65), (125, 41), (126, 97)])
+def test_resident_forms_match_fp64(gpu_lib, n, E, nb):
+    """Against the FP64 kernel on the same increments, at the edges of the CTAs'
+    42 particles and of the member tiles.  A step's FP32 rounding is 6e-8 of
+    increments below 0.1 and the field's error 2e-6 of them: 40 steps stay below
+    40 x 0.1 x 2.1e-6 of the unit moment."""
+    from magpy_gb300 import core
+    rng = np.random.default_rng(n + E)
+    axes = rng.normal(size=(n, 3))
+    axes /= np.linalg.norm(axes, axis=1, keepdims=True)
+    loc = np.stack(np.meshgrid(*[np.arange(6)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n] * 2e-8
+    args = (E, np.full(n, 7e-9), np.full(n, 2e4), axes, axes, loc, 4e5, 0.1, 300.0, False, True,
+            False, 5e-14, 5e-14 * 39.5, 3, np.arange(E) + 11, "sine", 1e4, 3e10)
+    a = core.EnsemblePlan(*args, precision="mixed_tc").set_launch(4, nb).run().arrays()
+    b = core.simulate_ensemble(*args, precision="fp64")
+    assert np.all(a.status == 0) and np.array_equal(a.steps, b.steps)
+    for c in ("mx", "my", "mz"):
+        assert np.abs(getattr(a, c) - getattr(b, c)).max() <= 8.4e-6 * 4e5
