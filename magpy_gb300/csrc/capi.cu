@@ -583,8 +583,8 @@ int run_plan(magpy_plan *plan, cudaStream_t st)
         // clusters, then the fewest members (a wave takes time in proportion
         // to its clusters' members: at N = 512 an implicit step takes 0.184 ms
         // a wave with 32, 0.345 with 64; Heun at E = 1638 measured 64 / 48 /
-        // 40 / 32: N = 84 134 / 123 / 98 / 92 ms per 1e4 steps, N = 125 145 /
-        // 134 / 109 / 197 (32: two waves), and at N = 216, E = 1024 212 / 189
+        // 40 / 32: N = 84 79 / 57 / 53 / 46 ms per 1e4 steps, N = 125 84 /
+        // 65 / 63 / 102 (32: two waves), and at N = 216, E = 1024 212 / 189
         // / 323 / 296 (40 and 32: two waves); every cluster form runs one CTA
         // per SM, so the resident count depends on the cluster size alone)
         const int32_t mpw = plan->p.members_per_warp;

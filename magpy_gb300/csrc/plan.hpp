@@ -100,6 +100,11 @@ cudaError_t tcc_build_d(const double *pt, const double *rt, int n, __half *d,
 // that can be resident at once (*max_clusters, may be NULL).
 cudaError_t tcc_init(int n, int nb, int *max_clusters);
 cudaError_t launch_tcc(const DevPlan &p, const __half *d, __half *b, int nb, cudaStream_t stream);
+// The Heun kernel of clusters whose D fits in tensor memory (two or three CTAs
+// a cluster); launch_tcc calls it, the B buffers are not used.
+constexpr int TCR_MAX_N = 126;
+cudaError_t tcr_init();
+cudaError_t launch_tcr(const DevPlan &p, const __half *d, int nb, cudaStream_t stream);
 cudaError_t launch_tcc_dipolar(const __half *d, __half *b, int n, int64_t E, const double *m,
                                double *h, int *flag, cudaStream_t stream);
 // Ensemble statistics (stats.cu).

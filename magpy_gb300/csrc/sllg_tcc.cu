@@ -25,14 +25,8 @@
 //   3. the accumulators, h = acc_main + acc_corr / 2048, go through a shared
 //      field tile to the threads that integrate the CTA's own particles,
 //      which write the next stage's B slab (step 1).
-// Up to three CTAs (65 to 126 particles) the Heun kernel keeps D in tensor
-// memory and has no chunks to stream: B is in every CTA's shared memory, a CTA
-// stores its K slab in its own tile and copies it to its peers' (distributed
-// shared memory), a cluster barrier orders that before the MMAs, and a second
-// one, waited for only after the integration, tells that no tile is read any
-// more.  Streaming B through L2 gave 18 bytes a clock an SM (a 61 KB tile in
-// 3300 clocks of a stage's 9400).  100 particles, 512 members: 10.0 -> 8.8 us a
-// step, 65 particles 9.2 -> 7.6.
+// Up to three CTAs (65 to 126 particles) the Heun integrator is sllg_tcr.cu's,
+// with D resident in tensor memory.
 // Everything else -- anisotropy and Zeeman terms, the LLG map, increments
 // from the in-kernel generator, the compensated state, samples -- is the
 // tensor-core kernel's (sllg_tc.cu) per-particle arithmetic, on the same
@@ -45,38 +39,23 @@
 // its tensor memory.  Cluster barriers are executed by every thread of every
 // CTA the same number of times, whatever happens.
 #include <algorithm>
-#include <cuda_fp16.h>
-#include "common.cuh"
 #include "implicit32.cuh"
 #include "llg32.cuh"
 #include "llg64.cuh"
-#include "plan.hpp"
-#include "tc_cluster.cuh"
-#include "tc_ptx.cuh"
+#include "tcc_common.cuh"
 
 namespace magpy {
 
 namespace {
 
-constexpr int PPC = 42;           // particles per CTA
-constexpr int RT = 128;           // rows of D per CTA (one MMA tile)
-constexpr int KC = 64;            // K elements per streamed chunk
 constexpr int NS = 3;             // ring stages (D and B chunks)
-constexpr int PAIRS = PPC / 2;    // particle pairs per CTA
 constexpr int ITEMS = 3;          // pair items per integrating thread (implicit, dipolar field)
 constexpr int TCC_MAX_T = 16;     // CTAs per cluster (non-portable above 8)
 constexpr int FIELD_BLOCK = 32;   // steps of applied field computed at a time (one per lane)
-constexpr uint32_t DRAIN_LIMIT = 1u << 24;
-constexpr int32_t ST_WATCHDOG = 16;
 
 // NB members per cluster: 32, 40, 48 or 64 (Heun), 32, 40 or 64 (implicit);
 // a multiple of 8, so that the main MMA's N = 2 NB is a multiple of 16.
-// Accumulator columns the MMAs write: [main NB | corr NB] from the main MMA,
-// and the correction MMA's N = NB rounded up to a multiple of 16 from column
-// NB (for NB = 40, eight columns past 2 NB).
-__host__ __device__ constexpr int tcc_acc_cols(int nb) { return nb + (nb + 15) / 16 * 16; }
 // NI pair items per integrating thread.
-constexpr int EPI_WARPS = 8;  // epilogue warps (0..7)
 template <int NB, int NI = ITEMS> struct Cfg {
     static constexpr int COLS = (PAIRS + NI - 1) / NI;        // threads per member
     static constexpr int IT = COLS * NB;                      // integrating threads
@@ -95,17 +74,11 @@ struct TccLayout {
     int n, T, K, nK, nb;
     size_t a_chunk, b_chunk, stage;  // bytes: D chunk (hi + lo), B chunk, one ring stage
     size_t f_off, par_off, sr_off, flag_off, bar_off, fld_off, total;
-    bool dres;  // D resident in tensor memory: a B tile in place of the ring
 };
 
-__host__ __device__ inline size_t tcc_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
-
-// head: bytes before the field tile, 0 for the ring of D and B chunks (with a
-// resident D, a B tile, the stage hand-off and low words).
-__host__ __device__ inline TccLayout tcc_layout(int n, int nb, size_t head = 0)
+__host__ __device__ inline TccLayout tcc_layout(int n, int nb)
 {
     TccLayout L;
-    L.dres = head != 0;
     L.n = n;
     L.nb = nb;
     L.T = (n + PPC - 1) / PPC;
@@ -114,7 +87,7 @@ __host__ __device__ inline TccLayout tcc_layout(int n, int nb, size_t head = 0)
     L.a_chunk = (size_t)2 * RT * KC * 2;
     L.b_chunk = (size_t)2 * nb * KC * 2;
     L.stage = L.a_chunk + L.b_chunk;
-    L.f_off = head ? tcc_up(head, 16) : NS * L.stage;
+    L.f_off = NS * L.stage;
     L.par_off = tcc_up(L.f_off + (size_t)RT * (nb + 4) * 4, 16);
     L.sr_off = L.par_off + (size_t)16 * PPC;
     L.flag_off = tcc_up(L.sr_off + (size_t)4 * PPC, 16);
@@ -170,24 +143,6 @@ struct Pipe {
     uint32_t commits; // MMA thread: completion commits made on accf
     uint32_t limit;
     uint32_t ncols;   // tensor-memory columns allocated
-};
-
-constexpr int DRES_K = 384;  // largest K of a resident D (3 CTAs a cluster)
-
-// Column of tensor memory from which D is resident (past every accumulator
-// column).
-template <int NB> constexpr uint32_t DCOL = tcc_acc_cols(NB);
-
-
-// The MMAs of one 64-deep K chunk: A main and correction descriptors of
-// k-step s from `a`, B at shared address b0.
-template <int NB> struct Idesc {
-    static constexpr uint32_t MAIN = tc::idesc_f16_f32(RT, 2 * NB);
-    // D_lo B_hi into [NB, NB + NC): N a multiple of 16 (for NB = 40 the
-    // last 8 columns multiply the first B_lo rows into accumulator
-    // columns that nothing reads)
-    static constexpr uint32_t CORR = tc::idesc_f16_f32(RT, tcc_acc_cols(NB) - NB);
-    static constexpr uint32_t B_LBO = (2 * NB / 8) * 128;  // between K-adjacent core matrices of B
 };
 
 // D B for this CTA's 128 rows and the NB members of the cluster: the
@@ -247,28 +202,6 @@ __device__ inline bool tcc_gemm(Pipe &P, const TccLayout &L, const unsigned char
     return ok;
 }
 
-// The same product with D in tensor memory and the whole B tile in shared
-// memory (at the start of the ring): K element k of D's split sp is in column
-// DCOL + sp K/2 + k/2.
-template <class C, int NB>
-__device__ inline void tcc_gemm_resident(Pipe &P, const TccLayout &L, int warp)
-{
-    if (warp != C::MMA) return;
-    tc::fence_proxy_async_cluster();
-    tc::fence_after_sync();
-    constexpr uint32_t b_lbo = Idesc<NB>::B_LBO;
-    const uint32_t b0 = tc::smem_addr(P.ring);
-    const uint32_t ahi = P.tmem + DCOL<NB>, alo = ahi + (uint32_t)(L.K / 2);
-#pragma unroll 2
-    for (int s = 0; s < L.K / 16; s++) {
-        const uint64_t bd = tc::smem_desc(b0 + 2u * b_lbo * s, b_lbo, 128);
-        tc::mma_f16_ta_warp(P.tmem, ahi + 8u * s, bd, Idesc<NB>::MAIN, s > 0 ? 1u : 0u);
-        tc::mma_f16_ta_warp(P.tmem + NB, alo + 8u * s, bd, Idesc<NB>::CORR, 1u);
-    }
-    tc::mma_commit_warp(P.accf);
-    P.commits++;
-}
-
 // Accumulators -> field tile F[row][member] (epilogue warps 0..7: lane quarter
 // warp % 4, member half warp / 4).  Returns false if the completion did not
 // arrive in time.
@@ -280,39 +213,7 @@ __device__ inline bool tcc_epilogue(Pipe &P, float *F, int warp, int lane)
         ok = __all_sync(0xffffffffu, tc::mbar_wait_bounded(P.accf, P.gemms & 1u, P.limit));
         tc::fence_after_sync();
         if (ok) {
-            const int quarter = warp & 3, half = warp >> 2;
-            const uint32_t lanes = (uint32_t)(32 * quarter) << 16;
-            const int row = 32 * quarter + lane;
-            constexpr int HALF = NB / 2;  // member columns per warp (a multiple of 4)
-#pragma unroll
-            for (int cb = 0; cb < HALF / 8; cb++) {
-                const int col = half * HALF + 8 * cb;
-                float vm[8], vc[8];
-                tc::tmem_ld8(P.tmem + lanes + (uint32_t)col, vm);
-                tc::tmem_ld8(P.tmem + lanes + (uint32_t)(NB + col), vc);
-                tc::tmem_ld_wait();
-                float4 *dst = reinterpret_cast<float4 *>(F + row * Cfg<NB>::FS + col);
-                dst[0] = make_float4(fmaf(vc[0], 1.0f / tc::SPLIT_SCALE, vm[0]),
-                                     fmaf(vc[1], 1.0f / tc::SPLIT_SCALE, vm[1]),
-                                     fmaf(vc[2], 1.0f / tc::SPLIT_SCALE, vm[2]),
-                                     fmaf(vc[3], 1.0f / tc::SPLIT_SCALE, vm[3]));
-                dst[1] = make_float4(fmaf(vc[4], 1.0f / tc::SPLIT_SCALE, vm[4]),
-                                     fmaf(vc[5], 1.0f / tc::SPLIT_SCALE, vm[5]),
-                                     fmaf(vc[6], 1.0f / tc::SPLIT_SCALE, vm[6]),
-                                     fmaf(vc[7], 1.0f / tc::SPLIT_SCALE, vm[7]));
-            }
-            if constexpr (HALF % 8 == 4) {  // the last four columns (NB = 40)
-                const int col = half * HALF + HALF - 4;
-                float vm[4], vc[4];
-                tc::tmem_ld4(P.tmem + lanes + (uint32_t)col, vm);
-                tc::tmem_ld4(P.tmem + lanes + (uint32_t)(NB + col), vc);
-                tc::tmem_ld_wait();
-                *reinterpret_cast<float4 *>(F + row * Cfg<NB>::FS + col) =
-                    make_float4(fmaf(vc[0], 1.0f / tc::SPLIT_SCALE, vm[0]),
-                                fmaf(vc[1], 1.0f / tc::SPLIT_SCALE, vm[1]),
-                                fmaf(vc[2], 1.0f / tc::SPLIT_SCALE, vm[2]),
-                                fmaf(vc[3], 1.0f / tc::SPLIT_SCALE, vm[3]));
-            }
+            tcc_field_tile<NB>(P.tmem, F, warp, lane);
         }
     }
     P.gemms++;
@@ -352,47 +253,6 @@ __device__ inline void put_pair_g(__half *btile, int r, int p, int j, bool live0
     }
 }
 
-// The same into the CTA's own slab of a B tile in shared memory.  Eight
-// members by four pairs a warp: 32 different banks.
-template <int NB>
-__device__ inline void put_pair_s(__half *slab, int p, int j, bool live0, bool live1,
-                                  const float m[6])
-{
-    if (!live0) return;
-#pragma unroll
-    for (int w = 0; w < 3; w++) {
-        if (w == 2 && !live1) break;
-        put_word_g<NB>(slab, j, 6 * p + 2 * w, m[2 * w], (w == 1 && !live1) ? 0.f : m[2 * w + 1]);
-    }
-}
-
-// This CTA's slab of the B tile to the same place in the cluster's other CTAs.
-template <class C, int NB>
-__device__ inline void push_slab(const unsigned char *slab, int r, int T)
-{
-    constexpr int V = RT * 2 * NB * 2 / 16;
-    const uint32_t a0 = tc::smem_addr(slab);
-    for (int v = threadIdx.x; v < V; v += C::THREADS) {
-        const uint4 x = reinterpret_cast<const uint4 *>(slab)[v];
-        for (int k = 1; k < T; k++) {
-            const int rr = r + k < T ? r + k : r + k - T;
-            tc::st_cluster_v4(tc::mapa(a0 + 16u * v, (uint32_t)rr), x);
-        }
-    }
-}
-
-// One particle's sample: x = (hi + lo) sc, o its index in a component's
-// [S][P] planes.  Not inlined, as field_block is not: what a step rarely runs
-// is kept out of the step loop's code.
-__device__ __noinline__ void tcc_write_sample(double *mx, double *my, double *mz, int64_t o,
-                                              double sc, float xh, float xl, float yh, float yl,
-                                              float zh, float zl)
-{
-    mx[o] = ((double)xh + (double)xl) * sc;
-    my[o] = ((double)yh + (double)yl) * sc;
-    mz[o] = ((double)zh + (double)zl) * sc;
-}
-
 // The applied field of step FIELD_BLOCK b + 1 + lane, at t or (second) t + dt.
 __device__ __noinline__ void tcc_field_block(float2 *sF2, const MemberDev *md, int64_t b, int64_t K,
                                              int second)
@@ -405,7 +265,7 @@ __device__ __noinline__ void tcc_field_block(float2 *sF2, const MemberDev *md, i
 }
 
 // Common set-up of a CTA: shared-memory carve-up, mbarriers, tensor memory
-// (the accumulators, and D when it is resident: then 512 columns).
+// (the accumulators).
 template <int NB>
 __device__ inline void tcc_setup(Pipe &P, unsigned char *sm, const TccLayout &L, uint32_t limit)
 {
@@ -419,7 +279,7 @@ __device__ inline void tcc_setup(Pipe &P, unsigned char *sm, const TccLayout &L,
     P.issued = 0;
     P.commits = 0;
     P.limit = limit;
-    P.ncols = L.dres ? 512u : Cfg<NB>::TMEM_COLS;
+    P.ncols = Cfg<NB>::TMEM_COLS;
     if (threadIdx.x == 0) {
         for (int i = 0; i < NS; i++) {
             tc::mbar_init(&P.full[i], 1);
@@ -432,34 +292,6 @@ __device__ inline void tcc_setup(Pipe &P, unsigned char *sm, const TccLayout &L,
     __syncthreads();
     tc::fence_after_sync();
     P.tmem = *slot;
-}
-
-// D tile (global, [chunk][split][128 x KC, row groups outermost]) into tensor
-// memory for the MMAs' A operand: row r in lane r, split sp's K element k in
-// column DCOL + sp K/2 + k/2 (two 16-bit elements per column, the even K in
-// the low half).  Warps 0..7: lane quarter warp % 4, split warp / 4.  Ends
-// with the stores complete; a CTA barrier must follow before the first MMA.
-template <int NB>
-__device__ inline void tcc_load_d_tmem(const Pipe &P, const TccLayout &L, const __half *dtile,
-                                       int warp, int lane)
-{
-    if (warp >= 8) return;
-    const int quarter = warp & 3, sp = warp >> 2;
-    const uint32_t row = (uint32_t)(32 * quarter + lane);
-    const uint32_t lanes = (uint32_t)(32 * quarter) << 16;
-    for (int c0 = 0; c0 < L.K / 2; c0 += 8) {
-        uint32_t v[8];
-#pragma unroll
-        for (int c = 0; c < 8; c++) {
-            const int k = 2 * (c0 + c), kc = k / KC, kk = k % KC;
-            const __half *src = dtile + (size_t)(2 * kc + sp) * RT * KC +
-                                tc::cm_offset_rows(row, (uint32_t)kk, KC);
-            v[c] = *reinterpret_cast<const uint32_t *>(src);
-        }
-        tc::tmem_st8(P.tmem + lanes + DCOL<NB> + (uint32_t)(sp * (L.K / 2) + c0), v);
-    }
-    tc::tmem_st_wait();
-    tc::fence_before_sync();
 }
 
 // Before the tensor memory is released: the producer waits (long bound) for
@@ -482,55 +314,27 @@ __device__ inline void tcc_drain(Pipe &P, int warp, int lane)
     }
 }
 
-// The OR over the cluster of each CTA's error word (every thread gets it).
-__device__ inline int cluster_any_error(int *sErr, int T)
-{
-    __shared__ int any;
-    if (threadIdx.x == 0) {
-        int a = 0;
-        const uint32_t base = tc::smem_addr(sErr);
-        for (int r = 0; r < T; r++) a |= tc::ld_cluster_s32(tc::mapa(base, (uint32_t)r));
-        any = a;
-    }
-    __syncthreads();
-    return any;
-}
-
 // ---- the integrator ----
 // Eight consecutive threads serve eight consecutive members j of the
 // cluster's tile, the next eight threads the next pair column p0 of COLS, then
 // the next eight members; a thread integrates the CTA-local particle pairs
 // p = p0 + COLS i.  A warp's reads of the field tile (8 members x 4 pairs, rows
 // 6 (NB + 4) floats apart) then fall into 32 different banks.
-template <int NB, bool DRES> constexpr int HEUN_ITEMS = NB <= 48 ? 2 : 3;
-template <int NB, bool DRES> using HeunCfg = Cfg<NB, HEUN_ITEMS<NB, DRES>>;
-// state low words in shared memory
-template <int NB, bool DRES> constexpr bool HEUN_LO = DRES && NB <= 48;
+template <int NB> constexpr int HEUN_ITEMS = NB <= 48 ? 2 : 3;
+template <int NB> using HeunCfg = Cfg<NB, HEUN_ITEMS<NB>>;
 
-// Bytes before the field tile when D is resident: a whole B tile, the stage
-// hand-off and the states' low words.
-template <int NB> constexpr size_t heun_head()
-{
-    return (size_t)DRES_K * 2 * NB * 2 +
-           (size_t)4 * (HEUN_LO<NB, true> ? 18 : 12) * HEUN_ITEMS<NB, true> * HeunCfg<NB, true>::IT;
-}
-
-template <int NB, bool DRES>
-__global__ void __launch_bounds__(HeunCfg<NB, DRES>::THREADS, 1)
+template <int NB>
+__global__ void __launch_bounds__(HeunCfg<NB>::THREADS, 1)
     sllg_tcc_kernel(DevPlan p, const __half *dglob, __half *bglob, int64_t tiles)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
-    using C = HeunCfg<NB, DRES>;
-    constexpr int ITEMS = HEUN_ITEMS<NB, DRES>;
+    using C = HeunCfg<NB>;
+    constexpr int ITEMS = HEUN_ITEMS<NB>;
     const int n = p.n;
-    const TccLayout L = tcc_layout(n, NB, DRES ? heun_head<NB>() : 0);
+    const TccLayout L = tcc_layout(n, NB);
     const int r = (int)tc::cluster_ctarank();
     const int64_t tile = (int64_t)blockIdx.x / L.T;
     Pipe P;
-    // DRES (up to three CTAs per cluster, n <= 126): the D tile fits in
-    // tensor memory beside the accumulators and is loaded once, the B tile is in
-    // every CTA's shared memory (each CTA stores its slab there and to its
-    // peers), and so is the stage hand-off instead of in registers
     tcc_setup<NB>(P, sm, L, p.wait_limit);
     float *F = (float *)(sm + L.f_off);
     float4 *sPar = (float4 *)(sm + L.par_off);
@@ -558,15 +362,6 @@ __global__ void __launch_bounds__(HeunCfg<NB, DRES>::THREADS, 1)
     __half *B0 = bglob + (size_t)tile * tile_elems;               // states
     __half *B1 = bglob + (size_t)(tiles + tile) * tile_elems;     // predictors
     const unsigned char *dtile = (const unsigned char *)dglob + (size_t)r * L.nK * L.a_chunk;
-    __half *slab = (__half *)sm + (size_t)r * RT * 2 * NB;  // DRES: this CTA's part of B
-    if constexpr (DRES) {
-        // (ordered before the first MMA by the CTA and cluster barriers below)
-        tcc_load_d_tmem<NB>(P, L, (const __half *)dtile, warp, lane);
-        uint4 *bz = (uint4 *)sm;  // padding, absent particles and members stay zero
-        for (int i = threadIdx.x; i < DRES_K * 2 * NB * 2 / 16; i += blockDim.x)
-            bz[i] = make_uint4(0, 0, 0, 0);
-        __syncthreads();
-    }
     const float dt = (float)m0d->dt, sq = (float)m0d->sqrt_dt, alpha = (float)m0d->alpha;
     const bool renorm = m0d->renorm != 0;
     const int64_t S = p.S;
@@ -582,35 +377,18 @@ __global__ void __launch_bounds__(HeunCfg<NB, DRES>::THREADS, 1)
     const uint64_t seed = valid ? p.members[e].seed : 0;
     const double *noise = (p.noise && valid) ? p.noise + p.members[e].noise_off : nullptr;
     bool live[ITEMS][2];
-    // state: float-float per component, the high words in registers; the
-    // low words (read and written once per step) in shared memory when D is
-    // resident and there is room (up to 48 members), else in registers
-    constexpr bool LO_SMEM = HEUN_LO<NB, DRES>;
-    float xh[ITEMS][2][3], xlr[LO_SMEM ? 1 : ITEMS][2][3];
+    // state: float-float per component
+    float xh[ITEMS][2][3], xl[ITEMS][2][3];
     // stage hand-off per pair item: A = F(m, v1)/2 and the increments W
-    float Areg[ITEMS][6], Wreg[ITEMS][6];
-    float *hand = (float *)(sm + DRES_K * 2 * NB * 2);  // DRES: [12 ITEMS][IT]
-    auto HA = [&](int i, int c) -> float & {
-        if constexpr (DRES) return hand[(i * 6 + c) * C::IT + threadIdx.x];
-        else return Areg[i][c];
-    };
-    auto HW = [&](int i, int c) -> float & {
-        if constexpr (DRES) return hand[((ITEMS + i) * 6 + c) * C::IT + threadIdx.x];
-        else return Wreg[i][c];
-    };
-    float *xlo = hand + 2 * ITEMS * 6 * C::IT;  // LO_SMEM: [ITEMS 2 3][IT]
-    auto XL = [&](int i, int k, int c) -> float & {
-        if constexpr (LO_SMEM) return xlo[((i * 2 + k) * 3 + c) * C::IT + threadIdx.x];
-        else return xlr[LO_SMEM ? 0 : i][k][c];
-    };
+    float A[ITEMS][6], W[ITEMS][6];
     auto record = [&](int64_t smp) {
         for (int i = 0; i < ITEMS; i++)
             for (int k = 0; k < 2; k++)
                 if (live[i][k])
                     tcc_write_sample(p.mx, p.my, p.mz,
                                      smp * P_ + e * n + PPC * r + 2 * (p0 + C::COLS * i) + k,
-                                     p.out_scale[e], xh[i][k][0], XL(i, k, 0), xh[i][k][1],
-                                     XL(i, k, 1), xh[i][k][2], XL(i, k, 2));
+                                     p.out_scale[e], xh[i][k][0], xl[i][k][0], xh[i][k][1],
+                                     xl[i][k][1], xh[i][k][2], xl[i][k][2]);
     };
 #pragma unroll
     for (int i = 0; i < ITEMS; i++) {
@@ -628,7 +406,7 @@ __global__ void __launch_bounds__(HeunCfg<NB, DRES>::THREADS, 1)
                     lo = (float)(v - (double)hi);
                 }
                 xh[i][k][c] = hi;
-                if (integ) XL(i, k, c) = lo;
+                xl[i][k][c] = lo;
             }
     }
     // initial state -> B0, sample 0 (lib/simulation.cpp:212-219)
@@ -637,8 +415,7 @@ __global__ void __launch_bounds__(HeunCfg<NB, DRES>::THREADS, 1)
         const int pl = p0 + C::COLS * i;
         const float m6[6] = {xh[i][0][0], xh[i][0][1], xh[i][0][2],
                              xh[i][1][0], xh[i][1][1], xh[i][1][2]};
-        if constexpr (DRES) put_pair_s<NB>(slab, pl, j, live[i][0], live[i][1], m6);
-        else put_pair_g<NB>(B0, r, pl, j, live[i][0], live[i][1], m6);
+        put_pair_g<NB>(B0, r, pl, j, live[i][0], live[i][1], m6);
     }
     if (p.mx) record(0);
     // The producer and MMA warps compute the applied field, FIELD_BLOCK steps
@@ -652,7 +429,6 @@ __global__ void __launch_bounds__(HeunCfg<NB, DRES>::THREADS, 1)
         if (warp == C::PROD || warp == C::MMA) tcc_field_block(sF2, m0d, b, K, warp == C::MMA);
     };
     field_block(0);
-    if constexpr (DRES) tc::cluster_sync();  // every CTA's tile is zeroed
     __syncthreads();
 
     int32_t status = ST_OK;
@@ -684,28 +460,19 @@ __global__ void __launch_bounds__(HeunCfg<NB, DRES>::THREADS, 1)
 #pragma unroll 1
         for (int stage = 0; stage < 2; stage++) {
             bool ok = true;
-            if constexpr (DRES) {
-                // no CTA reads its B tile any more (the wait at the stage's end)
-                push_slab<C, NB>((const unsigned char *)slab, r, L.T);
-                tc::fence_proxy_async_cluster();
-                tc::cluster_sync();
-                if (__shfl_sync(0xffffffffu, *sErr, 0) == 0) tcc_gemm_resident<C, NB>(P, L, warp);
-            } else {
-                // every CTA's slab of this stage's B tile is written
-                tc::fence_proxy_async_global();
-                tc::cluster_sync();
-                const __half *Bin = stage == 0 ? B0 : B1;
-                // a CTA whose pipeline broke skips its waits (read once per warp:
-                // the MMA warp's collectives need the whole warp)
-                if (__shfl_sync(0xffffffffu, *sErr, 0) == 0)
-                    ok = tcc_gemm<C, NB>(P, L, dtile, (const unsigned char *)Bin, warp, lane);
-                else
-                    P.g += (uint32_t)L.nK;
-            }
+            // every CTA's slab of this stage's B tile is written
+            tc::fence_proxy_async_global();
+            tc::cluster_sync();
+            const __half *Bin = stage == 0 ? B0 : B1;
+            // a CTA whose pipeline broke skips its waits (read once per warp:
+            // the MMA warp's collectives need the whole warp)
+            if (__shfl_sync(0xffffffffu, *sErr, 0) == 0)
+                ok = tcc_gemm<C, NB>(P, L, dtile, (const unsigned char *)Bin, warp, lane);
+            else
+                P.g += (uint32_t)L.nK;
             ok = (*sErr == 0 ? tcc_epilogue<NB>(P, F, warp, lane) : (P.gemms++, true)) && ok;
             if (!ok) atomicOr(sErr, 1);
             __syncthreads();
-            if constexpr (DRES) tc::cluster_arrive();  // this CTA no longer reads its B tile
             __half *Bout = stage == 0 ? B1 : B0;
             const float hz = stage == 0 ? h1 : h2;
             if (integ) {
@@ -730,23 +497,23 @@ __global__ void __launch_bounds__(HeunCfg<NB, DRES>::THREADS, 1)
                             if (noise) {
                                 const double *wp = noise + (step - 1) * per_step +
                                                    3 * (PPC * r + 2 * pl + k);
-                                HW(i, 3 * k) = (float)wp[0];
-                                HW(i, 3 * k + 1) = (float)wp[1];
-                                HW(i, 3 * k + 2) = (float)wp[2];
+                                W[i][3 * k] = (float)wp[0];
+                                W[i][3 * k + 1] = (float)wp[1];
+                                W[i][3 * k + 2] = (float)wp[2];
                             } else {
-                                HW(i, 3 * k) = wn.n[3 * k];
-                                HW(i, 3 * k + 1) = wn.n[3 * k + 1];
-                                HW(i, 3 * k + 2) = wn.n[3 * k + 2];
+                                W[i][3 * k] = wn.n[3 * k];
+                                W[i][3 * k + 1] = wn.n[3 * k + 1];
+                                W[i][3 * k + 2] = wn.n[3 * k + 2];
                             }
                         }
-                        const float w[3] = {HW(i, 3 * k), HW(i, 3 * k + 1), HW(i, 3 * k + 2)};
+                        const float w[3] = {W[i][3 * k], W[i][3 * k + 1], W[i][3 * k + 2]};
                         float m[3];
                         if (stage == 0) {
                             m[0] = xh[i][k][0]; m[1] = xh[i][k][1]; m[2] = xh[i][k][2];
                         } else {
-                            m[0] = xh[i][k][0] + 2.f * HA(i, 3 * k);
-                            m[1] = xh[i][k][1] + 2.f * HA(i, 3 * k + 1);
-                            m[2] = xh[i][k][2] + 2.f * HA(i, 3 * k + 2);
+                            m[0] = xh[i][k][0] + 2.f * A[i][3 * k];
+                            m[1] = xh[i][k][1] + 2.f * A[i][3 * k + 1];
+                            m[2] = xh[i][k][2] + 2.f * A[i][3 * k + 2];
                         }
                         const float dot = (m[0] * pa.x + m[1] * pa.y + m[2] * pa.z) * pa.w;
                         const float v[3] = {fmaf(dt, dot * pa.x + hd0, ssr * w[0]),
@@ -758,17 +525,17 @@ __global__ void __launch_bounds__(HeunCfg<NB, DRES>::THREADS, 1)
                             // predictor x~ = x + dt a + sqrt(dt) B w
 #pragma unroll
                             for (int c = 0; c < 3; c++) {
-                                HA(i, 3 * k + c) = 0.5f * inc[c];
+                                A[i][3 * k + c] = 0.5f * inc[c];
                                 m6[3 * k + c] = m[c] + inc[c];
                             }
                         } else {
 #pragma unroll
                             for (int c = 0; c < 3; c++)
                             {
-                                const DDf t = dd_add_ts(DDf{xh[i][k][c], XL(i, k, c)},
-                                                        fmaf(0.5f, inc[c], HA(i, 3 * k + c)));
+                                const DDf t = dd_add_ts(DDf{xh[i][k][c], xl[i][k][c]},
+                                                        fmaf(0.5f, inc[c], A[i][3 * k + c]));
                                 xh[i][k][c] = t.hi;
-                                XL(i, k, c) = t.lo;
+                                xl[i][k][c] = t.lo;
                             }
                             if (renorm) {
                                 const float nrm = sqrtf(xh[i][k][0] * xh[i][k][0] +
@@ -777,7 +544,7 @@ __global__ void __launch_bounds__(HeunCfg<NB, DRES>::THREADS, 1)
                                 const float inv = 1.0f / nrm;
                                 for (int c = 0; c < 3; c++) {
                                     xh[i][k][c] *= inv;
-                                    XL(i, k, c) *= inv;
+                                    xl[i][k][c] *= inv;
                                 }
                             }
                             m6[3 * k] = xh[i][k][0];
@@ -785,15 +552,8 @@ __global__ void __launch_bounds__(HeunCfg<NB, DRES>::THREADS, 1)
                             m6[3 * k + 2] = xh[i][k][2];
                         }
                     }
-                    if constexpr (DRES) put_pair_s<NB>(slab, pl, j, live[i][0], live[i][1], m6);
-                    else put_pair_g<NB>(Bout, r, pl, j, live[i][0], live[i][1], m6);
+                    put_pair_g<NB>(Bout, r, pl, j, live[i][0], live[i][1], m6);
                 }
-            }
-            if constexpr (DRES) {
-                tc::fence_proxy_async_cluster();
-                __syncwarp();
-                tc::cluster_wait();
-                __syncthreads();
             }
         }
     }
@@ -1294,55 +1054,6 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
     tc::cluster_sync();
 }
 
-template <class Kern>
-cudaError_t tcc_prepare(Kern kern, const TccLayout &L, size_t smem)
-{
-    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem);
-    if (err == cudaSuccess && L.T > 8)
-        err = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    return err;
-}
-
-template <class Kern, class... Args>
-cudaError_t tcc_launch(Kern kern, const TccLayout &L, size_t smem, int threads, int64_t tiles,
-                       cudaStream_t stream, Args... args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(tiles * L.T));
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)L.T;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    // the stream's scheduling priority, carried into a captured graph node
-    // (a batch gives its longest group the highest)
-    int prio = 0;
-    if (cudaStreamGetPriority(stream, &prio) != cudaSuccess) prio = 0;
-    attr[1].id = cudaLaunchAttributePriority;
-    attr[1].val.priority = prio;
-    cfg.attrs = attr;
-    cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, kern, args...);
-}
-
-// Shared memory of the Heun kernel with a resident D (the same for any n).
-template <int NB> size_t heun_smem() { return tcc_layout(2 * PPC, NB, heun_head<NB>()).total; }
-
-template <int NB>
-cudaError_t tcc_launch_heun(const DevPlan &p, const __half *d, __half *b, const TccLayout &L,
-                            bool dres, int64_t tiles, cudaStream_t stream)
-{
-    if (dres)
-        return tcc_launch(sllg_tcc_kernel<NB, true>, L, heun_smem<NB>(),
-                          HeunCfg<NB, true>::THREADS, tiles, stream, p, d, b, tiles);
-    return tcc_launch(sllg_tcc_kernel<NB, false>, L, L.total, HeunCfg<NB, false>::THREADS, tiles,
-                      stream, p, d, b, tiles);
-}
-
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -1388,30 +1099,29 @@ cudaError_t tcc_init(int n, int nb, int *max_clusters)
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     const TccLayout Lmax = tcc_layout(PPC * TCC_MAX_T, nb);
     const size_t imp = tcc_imp_smem(Lmax);
+    if (!done[dev][w]) {
+        err = tcr_init();
+        if (err != cudaSuccess) return err;
+    }
     if (!done[dev][w] && nb == 40) {
-        err = tcc_prepare(sllg_tcc_implicit_kernel<40>, Lmax, imp);
-        if (err == cudaSuccess) err = tcc_prepare(sllg_tcc_kernel<40, false>, Lmax, Lmax.total);
-        if (err == cudaSuccess) err = tcc_prepare(sllg_tcc_kernel<40, true>, Lmax, heun_smem<40>());
+        err = tcc_prepare(sllg_tcc_implicit_kernel<40>, Lmax.T, imp);
+        if (err == cudaSuccess) err = tcc_prepare(sllg_tcc_kernel<40>, Lmax.T, Lmax.total);
         if (err != cudaSuccess) return err;
         done[dev][w] = true;
     }
     if (!done[dev][w]) {
-        err = nb == 32 ? tcc_prepare(sllg_tcc_kernel<32, false>, Lmax, Lmax.total)
-                       : tcc_prepare(sllg_tcc_kernel<64, false>, Lmax, Lmax.total);
-        if (err == cudaSuccess)
-            err = nb == 32 ? tcc_prepare(sllg_tcc_kernel<32, true>, Lmax, heun_smem<32>())
-                           : tcc_prepare(sllg_tcc_kernel<64, true>, Lmax, heun_smem<64>());
+        err = nb == 32 ? tcc_prepare(sllg_tcc_kernel<32>, Lmax.T, Lmax.total)
+                       : tcc_prepare(sllg_tcc_kernel<64>, Lmax.T, Lmax.total);
         if (err == cudaSuccess && nb == 64) {  // the 48-member form, prepared alongside
             const TccLayout L48 = tcc_layout(PPC * TCC_MAX_T, 48);
-            err = tcc_prepare(sllg_tcc_kernel<48, false>, L48, L48.total);
-            if (err == cudaSuccess) err = tcc_prepare(sllg_tcc_kernel<48, true>, L48, heun_smem<48>());
+            err = tcc_prepare(sllg_tcc_kernel<48>, L48.T, L48.total);
         }
         if (err == cudaSuccess)
-            err = nb == 32 ? tcc_prepare(tcc_dipolar_kernel<32>, Lmax, Lmax.total)
-                           : tcc_prepare(tcc_dipolar_kernel<64>, Lmax, Lmax.total);
+            err = nb == 32 ? tcc_prepare(tcc_dipolar_kernel<32>, Lmax.T, Lmax.total)
+                           : tcc_prepare(tcc_dipolar_kernel<64>, Lmax.T, Lmax.total);
         if (err == cudaSuccess)
-            err = nb == 32 ? tcc_prepare(sllg_tcc_implicit_kernel<32>, Lmax, imp)
-                           : tcc_prepare(sllg_tcc_implicit_kernel<64>, Lmax, imp);
+            err = nb == 32 ? tcc_prepare(sllg_tcc_implicit_kernel<32>, Lmax.T, imp)
+                           : tcc_prepare(sllg_tcc_implicit_kernel<64>, Lmax.T, imp);
         if (err != cudaSuccess) return err;
         done[dev][w] = true;
     }
@@ -1447,21 +1157,24 @@ cudaError_t launch_tcc(const DevPlan &p, const __half *d, __half *b, int nb, cud
         if (!tcc_implicit_supported(p.n) || !p.hj) return cudaErrorNotSupported;
         const size_t smem = tcc_imp_smem(L);
         if (nb == 32)
-            return tcc_launch(sllg_tcc_implicit_kernel<32>, L, smem, Cfg<32>::THREADS, tiles,
+            return tcc_launch(sllg_tcc_implicit_kernel<32>, L.T, smem, Cfg<32>::THREADS, tiles,
                               stream, p, d, b, tiles);
         if (nb == 40)
-            return tcc_launch(sllg_tcc_implicit_kernel<40>, L, smem, Cfg<40>::THREADS, tiles,
+            return tcc_launch(sllg_tcc_implicit_kernel<40>, L.T, smem, Cfg<40>::THREADS, tiles,
                               stream, p, d, b, tiles);
-        return tcc_launch(sllg_tcc_implicit_kernel<64>, L, smem, Cfg<64>::THREADS, tiles, stream,
+        return tcc_launch(sllg_tcc_implicit_kernel<64>, L.T, smem, Cfg<64>::THREADS, tiles, stream,
                           p, d, b, tiles);
     }
     if (!tcc_supported(p.n)) return cudaErrorNotSupported;
-    const bool dres = tcc_acc_cols(nb) + L.K <= 512;
+    if (p.n <= TCR_MAX_N) return launch_tcr(p, d, nb, stream);
+    const auto heun = [&](auto kern, int threads) {
+        return tcc_launch(kern, L.T, L.total, threads, tiles, stream, p, d, b, tiles);
+    };
     switch (nb) {
-    case 32: return tcc_launch_heun<32>(p, d, b, L, dres, tiles, stream);
-    case 40: return tcc_launch_heun<40>(p, d, b, L, dres, tiles, stream);
-    case 48: return tcc_launch_heun<48>(p, d, b, L, dres, tiles, stream);
-    default: return tcc_launch_heun<64>(p, d, b, L, dres, tiles, stream);
+    case 32: return heun(sllg_tcc_kernel<32>, HeunCfg<32>::THREADS);
+    case 40: return heun(sllg_tcc_kernel<40>, HeunCfg<40>::THREADS);
+    case 48: return heun(sllg_tcc_kernel<48>, HeunCfg<48>::THREADS);
+    default: return heun(sllg_tcc_kernel<64>, HeunCfg<64>::THREADS);
     }
 }
 
@@ -1472,7 +1185,7 @@ cudaError_t launch_tcc_dipolar(const __half *d, __half *b, int n, int64_t E, con
     const int nb = 32;
     const TccLayout L = tcc_layout(n, nb);
     const int64_t tiles = (E + nb - 1) / nb;
-    return tcc_launch(tcc_dipolar_kernel<32>, L, L.total, Cfg<32>::THREADS, tiles, stream, n, E, d,
+    return tcc_launch(tcc_dipolar_kernel<32>, L.T, L.total, Cfg<32>::THREADS, tiles, stream, n, E, d,
                       b, m, h, flag);
 }
 

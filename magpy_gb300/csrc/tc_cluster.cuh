@@ -31,6 +31,19 @@ __device__ inline void bulk_g2s(void *dst_smem, const void *src_gmem, uint32_t b
         : "memory");
 }
 
+// Bulk copy this CTA's shared memory -> a CTA of the cluster's (`dst` and `bar`
+// from mapa, 16-byte aligned, size a multiple of 16), completing `bytes` on that
+// CTA's mbarrier.
+__device__ inline void bulk_s2s(uint32_t dst, const void *src_smem, uint32_t bytes, uint32_t bar)
+{
+    asm volatile(
+        "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes "
+        "[%0], [%1], %2, [%3];"
+        :
+        : "r"(dst), "r"(smem_addr(src_smem)), "r"(bytes), "r"(bar)
+        : "memory");
+}
+
 __device__ inline uint32_t cluster_ctarank()
 {
     uint32_t r;
@@ -47,16 +60,18 @@ __device__ inline void cluster_sync()
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// The two halves of that barrier: a CTA may work between its arrival and its
-// wait.  Arrivals and waits alternate.
-__device__ inline void cluster_arrive()
+// Arrive on an mbarrier of this CTA, after the thread's earlier memory
+// operations, or of a CTA of the cluster (`cbar` from mapa), which orders none.
+__device__ inline void mbar_arrive(void *bar)
 {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar))
+                 : "memory");
 }
 
-__device__ inline void cluster_wait()
+__device__ inline void mbar_arrive_remote_relaxed(uint32_t cbar)
 {
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cbar)
+                 : "memory");
 }
 
 // Address of the same shared-memory location in CTA `rank` of the cluster.
@@ -79,21 +94,6 @@ __device__ inline int32_t ld_cluster_s32(uint32_t caddr)
     int32_t v;
     asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(caddr) : "memory");
     return v;
-}
-
-__device__ inline void st_cluster_v4(uint32_t caddr, uint4 v)
-{
-    asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};"
-                 :
-                 : "r"(caddr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
-                 : "memory");
-}
-
-// Orders this thread's generic-proxy accesses to the cluster's shared memory
-// with async-proxy (MMA operand) accesses, both ways.
-__device__ inline void fence_proxy_async_cluster()
-{
-    asm volatile("fence.proxy.async.shared::cluster;" ::: "memory");
 }
 
 // Orders this thread's generic-proxy global accesses with its async-proxy

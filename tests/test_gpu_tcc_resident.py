@@ -1,4 +1,4 @@
-"""The cluster Heun kernel for 65 to 126 particles (two or three CTAs a cluster,
+"""The cluster Heun kernel for 65 to 126 particles (two or three CTAs a cluster, two member groups,
 the moments of a member tile in every CTA's shared memory)."""
 import numpy as np
 import pytest
