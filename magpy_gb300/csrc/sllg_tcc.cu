@@ -818,6 +818,7 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
     };
     if (threadIdx.x < 2 * NB) pflag[threadIdx.x] = 0;
     write_B(0);
+    tc::fence_proxy_async_global();  // (the first step begins with a cluster barrier)
     if (p.mx)  // sample 0: the initial state (lib/simulation.cpp:212-219)
 #pragma unroll
         for (int i = 0; i < ITEMS; i++)
@@ -1019,6 +1020,9 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
             }
         write_B(wb ^ 1);
         wb ^= 1;
+        // every CTA's slab of the next step's first B tile is written
+        tc::fence_proxy_async_global();
+        tc::cluster_sync();
     }
     step -= 1;
     // a wait that ran out after the last check is reported too
