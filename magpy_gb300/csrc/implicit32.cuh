@@ -3,17 +3,23 @@
 // cores, sllg_tcc.cu on the tensor cores).
 #pragma once
 #include <cstdint>
+#include "mul_int.cuh"
 
 namespace magpy {
 
 // Conversions by integer instructions, the same bits as the hardware's: those
 // run on the FP64 pipe (16 cycles of an SM a warp instruction, as any FP64
 // operation), these take 4-6 cycles of the integer pipes.  Zeros, subnormals,
-// infinities and NaN (and numbers past FP32's range) take the hardware's.
+// infinities and NaN (and numbers past FP32's range) take the hardware's, in a
+// call: as predicated instructions those were issued every time (8 of the 54 FP64
+// instructions of a particle's iteration).
+static __device__ __noinline__ float narrow_any(double x) { return __double2float_rn(x); }
+static __device__ __noinline__ double widen_any(float x) { return (double)x; }
+
 __device__ __forceinline__ float narrow(double x)
 {
     const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
-    if ((hi & 0x7fffffffu) - 0x38100000u >= 0x0fd00000u) return __double2float_rn(x);
+    if ((hi & 0x7fffffffu) - 0x38100000u >= 0x0fd00000u) return narrow_any(x);
     // exponent and 23 mantissa bits; the 29 below round to nearest even
     const uint32_t m = __funnelshift_l(lo, hi, 3) - 0xc0000000u;
     const uint32_t half = (m & 1u) + 0x7fffffffu;
@@ -27,23 +33,66 @@ __device__ __forceinline__ float narrow(double x)
 __device__ __forceinline__ double widen(float x)
 {
     const uint32_t u = __float_as_uint(x);
-    if ((u & 0x7fffffffu) - 0x00800000u >= 0x7f000000u) return (double)x;
+    if ((u & 0x7fffffffu) - 0x00800000u >= 0x7f000000u) return widen_any(x);
     return __hiloint2double((int)((((u & 0x7fffffffu) >> 3) + 0x38000000u) | (u & 0x80000000u)),
                             (int)(u << 29));
 }
 
 // -(m x v) - alpha m x (m x v): drift and diffusion share this map
 // (lib/llg.cpp:14-29, :92-106), linear in v = dt h + sr dwm.
-__device__ inline void stage_map(double o[3], const double m[3], double alpha, const double v[3])
+template <class Mul>
+__device__ __forceinline__ void stage_map_by(double o[3], const double m[3], double alpha,
+                                             const double v[3], Mul mul)
 {
     double u[3], w[3];
-    u[0] = fma(m[1], v[2], -(m[2] * v[1]));
-    u[1] = fma(m[2], v[0], -(m[0] * v[2]));
-    u[2] = fma(m[0], v[1], -(m[1] * v[0]));
-    w[0] = fma(m[1], u[2], -(m[2] * u[1]));
-    w[1] = fma(m[2], u[0], -(m[0] * u[2]));
-    w[2] = fma(m[0], u[1], -(m[1] * u[0]));
+    u[0] = fma(m[1], v[2], -mul(m[2], v[1]));
+    u[1] = fma(m[2], v[0], -mul(m[0], v[2]));
+    u[2] = fma(m[0], v[1], -mul(m[1], v[0]));
+    w[0] = fma(m[1], u[2], -mul(m[2], u[1]));
+    w[1] = fma(m[2], u[0], -mul(m[0], u[2]));
+    w[2] = fma(m[0], u[1], -mul(m[1], u[0]));
     for (int c = 0; c < 3; c++) o[c] = fma(-alpha, w[c], -u[c]);
+}
+
+struct Double3 { double x, y, z; };
+
+// Any operands (not inlined: rarely used).
+static __device__ __noinline__ Double3 stage_map_any(Double3 a, double alpha, Double3 b)
+{
+    const double m[3] = {a.x, a.y, a.z}, v[3] = {b.x, b.y, b.z};
+    double o[3];
+    stage_map_by(o, m, alpha, v, [](double x, double y) { return x * y; });
+    return Double3{o[0], o[1], o[2]};
+}
+
+// Zero or a magnitude in [2^-120, 2^120): mul_int takes every product below (a
+// non-zero u, a multiple of 2^-344, is at least that and below 2^241).
+__device__ __forceinline__ bool map_range(double x)
+{
+    const uint32_t h = __double2hiint(x) & 0x7fffffffu;
+    return h - (903u << 20) < (240u << 20) || (h | (uint32_t)__double2loint(x)) == 0;
+}
+
+// INT: the six plain products on the integer pipes, the same bits.  It pays where
+// the FP64 pipe (19 cycles of an SM an instruction) is the bound: 512 members of
+// 512 particles on the tensor cores 300 -> 284 us a step.  On the CUDA cores the
+// dipolar sum is most of a step and few warps wait for each other: 2.67 -> 2.73 ms
+// for a random ensemble of 13 particles, so those keep the FP64 products.
+template <bool INT>
+__device__ __forceinline__ void stage_map(double o[3], const double m[3], double alpha,
+                                          const double v[3])
+{
+    const auto plain = [](double x, double y) { return x * y; };
+    if constexpr (!INT) {
+        stage_map_by(o, m, alpha, v, plain);
+    } else if (map_range(m[0]) && map_range(m[1]) && map_range(m[2]) && map_range(v[0]) &&
+               map_range(v[1]) && map_range(v[2])) {
+        stage_map_by(o, m, alpha, v, [](double x, double y) { return mul_int(x, y); });
+    } else {
+        const Double3 r =
+            stage_map_any(Double3{m[0], m[1], m[2]}, alpha, Double3{v[0], v[1], v[2]});
+        o[0] = r.x; o[1] = r.y; o[2] = r.z;
+    }
 }
 
 // J = I - 1/2 d(stage_map)/dm in FP32, with v's own dependence on m through

@@ -399,7 +399,7 @@ __device__ inline void stage32(const Member &M, const Particle &pa, const double
     v[0] = fma(dt, fma(dot, pa.ax[0], H[0]), sdw[0]);
     v[1] = fma(dt, fma(dot, pa.ax[1], H[1]), sdw[1]);
     v[2] = fma(dt, fma(dot, pa.ax[2], H[2] + hz), sdw[2]);
-    stage_map(g, s, pa.alpha, v);
+    stage_map<false>(g, s, pa.alpha, v);
 }
 
 __device__ int32_t implicit_step32(const Member &M, const Particle &pa, double x[3],

@@ -669,10 +669,10 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
 // What bounds it: the FP64 pipe (two lanes a clock an SM), on which conversions
 // run too.  A particle's iteration is 35 FP64 instructions (stage increments
 // dt a + B dwm = F(m, dt h + sr dwm), the residual, the update), its
-// conversions are integer (narrow, widen), its share of the stopping norm is
-// summed as float-float (exact squares), and starting from the explicit
-// midpoint saves one iteration of four.  512 members of 512 particles, 40
-// steps: 18.0 -> 12.8 ms.
+// conversions are integer (narrow, widen), as are six of its products (stage_map),
+// its share of the stopping norm is summed as float-float (exact squares), and
+// starting from the explicit midpoint saves one iteration of four.  512 members
+// of 512 particles, 40 steps: 18.0 -> 11.4 ms.
 
 // Per-particle constants of a CTA's 42 particles: FP64 for the residual,
 // FP32 copies for the Jacobian.
@@ -681,24 +681,39 @@ struct ImpPar {
     float axf[PPC][3], dtk[PPC];
 };
 
+// Pair items per thread.  A particle's iteration is a chain of FP64 operations
+// of 64 cycles each, so more warps with fewer items hide more of it, and the
+// items' unrolled code is shorter: two (11 x NB threads) against three took
+// 94 / 120 against 101 / 122 us a step at 32 / 40 members of 64 particles; one
+// (40 members: 64 registers, which spill) 124.  64 members with two would be
+// 704 threads and 80 registers.
+__host__ __device__ constexpr int imp_items(int nb) { return nb == 64 ? 3 : 2; }
+__host__ __device__ constexpr int imp_cols(int nb)
+{
+    return (PAIRS + imp_items(nb) - 1) / imp_items(nb);
+}
+template <int NB> using ImpCfg = Cfg<NB, imp_items(NB)>;
+
 __host__ __device__ inline size_t tcc_imp_smem(const TccLayout &L)
 {
     // after the Heun layout: particle constants, per-(p0, member) partial
     // sums, and the cluster-exchanged partials / flags (double-buffered)
     // ... and, in the 32- and 40-member forms, each particle's step increments
     // sr dwm kept for the Newton iterations
-    const size_t kept =
-        L.nb <= 40 ? (size_t)8 * 3 * 2 * ITEMS * (PAIRS * (size_t)L.nb / ITEMS) : 0;
-    return tcc_up(L.total, 16) + sizeof(ImpPar) + (size_t)8 * 7 * L.nb + (size_t)8 * 2 * L.nb +
-           (size_t)4 * 2 * L.nb + (size_t)8 * L.nb + (size_t)4 * L.nb + 64 + kept;
+    const size_t items = (size_t)imp_items(L.nb) * imp_cols(L.nb) * L.nb;
+    const size_t kept = L.nb <= 40 ? (size_t)8 * 3 * 2 * items : 0;
+    return tcc_up(L.total, 16) + sizeof(ImpPar) + (size_t)8 * imp_cols(L.nb) * L.nb +
+           (size_t)8 * 2 * L.nb + (size_t)4 * 2 * L.nb + (size_t)8 * L.nb + (size_t)4 * L.nb + 64 +
+           kept;
 }
 
 template <int NB>
-__global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
+__global__ void __launch_bounds__(ImpCfg<NB>::THREADS, 1)
     sllg_tcc_implicit_kernel(DevPlan p, const __half *dglob, __half *bglob, int64_t tiles)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
-    using C = Cfg<NB>;
+    using C = ImpCfg<NB>;
+    constexpr int ITEMS = imp_items(NB);
     const int n = p.n;
     const TccLayout L = tcc_layout(n, NB);
     const int r = (int)tc::cluster_ctarank();
@@ -710,8 +725,8 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
     int *sErr = sFlag + NB;
     unsigned char *xs = sm + tcc_up(L.total, 16);
     ImpPar *par = (ImpPar *)xs;
-    double *red = (double *)(xs + sizeof(ImpPar));          // [7][NB]
-    double *part = red + 7 * NB;                              // [2][NB] exchanged
+    double *red = (double *)(xs + sizeof(ImpPar));          // [COLS][NB]
+    double *part = red + C::COLS * NB;                              // [2][NB] exchanged
     int *pflag = (int *)(part + 2 * NB);                      // [2][NB] exchanged
     double *sNorm = (double *)(pflag + 2 * NB);               // [NB] combined norm
     int *sSing = (int *)(sNorm + NB);                         // [NB] combined singular flag
@@ -762,9 +777,9 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
     double x[ITEMS][2][3], px[ITEMS][2][3];
 #pragma unroll
     for (int i = 0; i < ITEMS; i++) {
-        const int q0 = PPC * r + 2 * (p0 + 7 * i);
-        live[i][0] = valid && q0 < n;
-        live[i][1] = valid && q0 + 1 < n;
+        const int q0 = PPC * r + 2 * (p0 + C::COLS * i);
+        live[i][0] = valid && p0 + C::COLS * i < PAIRS && q0 < n;
+        live[i][1] = live[i][0] && q0 + 1 < n;
 #pragma unroll
         for (int k = 0; k < 2; k++)
 #pragma unroll
@@ -780,7 +795,7 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
         for (int i = 0; i < ITEMS; i++) {
             const float m6[6] = {narrow(x[i][0][0]), narrow(x[i][0][1]), narrow(x[i][0][2]),
                                  narrow(x[i][1][0]), narrow(x[i][1][1]), narrow(x[i][1][2])};
-            put_pair_g<NB>(Bbuf[buf], r, p0 + 7 * i, j, live[i][0], live[i][1], m6);
+            put_pair_g<NB>(Bbuf[buf], r, p0 + C::COLS * i, j, live[i][0], live[i][1], m6);
         }
     };
     // Member-wide sum of `v` over the cluster (fixed order); returns it in the
@@ -791,7 +806,7 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
         __syncthreads();
         if (threadIdx.x < NB) {
             double s_ = 0.0;
-            for (int q = 0; q < 7; q++) s_ += red[q * NB + threadIdx.x];
+            for (int q = 0; q < C::COLS; q++) s_ += red[q * NB + threadIdx.x];
             part[pc * NB + threadIdx.x] = s_;
         }
         tc::fence_proxy_async_global();  // this stage's B slab (generic stores) -> bulk reads
@@ -824,7 +839,7 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
         for (int i = 0; i < ITEMS; i++)
             for (int k = 0; k < 2; k++)
                 if (live[i][k]) {
-                    const int64_t o = e * n + PPC * r + 2 * (p0 + 7 * i) + k;
+                    const int64_t o = e * n + PPC * r + 2 * (p0 + C::COLS * i) + k;
                     const double sc = p.out_scale[e];
                     p.mx[o] = x[i][k][0] * sc; p.my[o] = x[i][k][1] * sc; p.mz[o] = x[i][k][2] * sc;
                 }
@@ -860,7 +875,7 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
                 for (int i = 0; i < ITEMS; i++)
                     for (int k = 0; k < 2; k++)
                         if (live[i][k]) {
-                            const int64_t o = s_next * P_ + e * n + PPC * r + 2 * (p0 + 7 * i) + k;
+                            const int64_t o = s_next * P_ + e * n + PPC * r + 2 * (p0 + C::COLS * i) + k;
                             const double sc = p.out_scale[e];
                             p.mx[o] = x[i][k][0] * sc;
                             p.my[o] = x[i][k][1] * sc;
@@ -878,8 +893,8 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
         // The generator's normals never reach the clamp (|w| <= 5.65 < Ah), so
         // only injected increments are clamped.
         auto sdw_of = [&](int i, int k, double out[3]) {
-            const int q = PPC * r + 2 * (p0 + 7 * i) + k;
-            const double sr = par->sr[2 * (p0 + 7 * i) + k];
+            const int q = PPC * r + 2 * (p0 + C::COLS * i) + k;
+            const double sr = par->sr[2 * (p0 + C::COLS * i) + k];
             if (noise) {
                 const double *wp = noise + (step - 1) * per_step + 3 * q;
                 for (int c = 0; c < 3; c++) {
@@ -895,14 +910,14 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
         // stage increment g at m (and its v), hz the applied field
         auto stage = [&](int i, int k, const double m[3], double hz, const double sdw[3],
                          double g[3], double v[3]) {
-            const int lq = 2 * (p0 + 7 * i) + k;
+            const int lq = 2 * (p0 + C::COLS * i) + k;
             const double *ax = par->ax[lq];
             const double dot = par->k[lq] * fma(m[2], ax[2], fma(m[1], ax[1], m[0] * ax[0]));
             const float *f = F + (3 * lq) * C::FS + j;
             v[0] = fma(dt, fma(dot, ax[0], widen(f[0])), sdw[0]);
             v[1] = fma(dt, fma(dot, ax[1], widen(f[C::FS])), sdw[1]);
             v[2] = fma(dt, fma(dot, ax[2], widen(f[2 * C::FS]) + hz), sdw[2]);
-            stage_map(g, m, alpha, v);
+            stage_map<true>(g, m, alpha, v);
         };
         // field at the current state -> the first iterate
         field();
@@ -965,7 +980,7 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
 #pragma unroll
                     for (int k = 0; k < 2; k++) {
                         if (!live[i][k]) continue;
-                        const int lq = 2 * (p0 + 7 * i) + k;
+                        const int lq = 2 * (p0 + C::COLS * i) + k;
                         const double xt[3] = {x[i][k][0], x[i][k][1], x[i][k][2]};
                         double sdw[3], g[3], v[3];
                         if constexpr (KEEP_DW) {
@@ -1034,7 +1049,7 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
             for (int i = 0; i < ITEMS; i++)
                 for (int k = 0; k < 2; k++)
                     if (live[i][k]) {
-                        const int64_t o = s2 * P_ + e * n + PPC * r + 2 * (p0 + 7 * i) + k;
+                        const int64_t o = s2 * P_ + e * n + PPC * r + 2 * (p0 + C::COLS * i) + k;
                         p.mx[o] = NAN; p.my[o] = NAN; p.mz[o] = NAN;
                     }
     bool bad = false;
@@ -1133,8 +1148,8 @@ cudaError_t tcc_init(int n, int nb, int *max_clusters)
     const TccLayout L = tcc_layout(n, nb);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)L.T);
-    cfg.blockDim = dim3((unsigned)(nb == 32 ? Cfg<32>::THREADS
-                                   : nb == 40 ? Cfg<40>::THREADS : Cfg<64>::THREADS));
+    cfg.blockDim = dim3((unsigned)(nb == 32 ? ImpCfg<32>::THREADS
+                                   : nb == 40 ? ImpCfg<40>::THREADS : ImpCfg<64>::THREADS));
     cfg.dynamicSmemBytes = tcc_imp_smem(L);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1161,12 +1176,12 @@ cudaError_t launch_tcc(const DevPlan &p, const __half *d, __half *b, int nb, cud
         if (!tcc_implicit_supported(p.n) || !p.hj) return cudaErrorNotSupported;
         const size_t smem = tcc_imp_smem(L);
         if (nb == 32)
-            return tcc_launch(sllg_tcc_implicit_kernel<32>, L.T, smem, Cfg<32>::THREADS, tiles,
+            return tcc_launch(sllg_tcc_implicit_kernel<32>, L.T, smem, ImpCfg<32>::THREADS, tiles,
                               stream, p, d, b, tiles);
         if (nb == 40)
-            return tcc_launch(sllg_tcc_implicit_kernel<40>, L.T, smem, Cfg<40>::THREADS, tiles,
+            return tcc_launch(sllg_tcc_implicit_kernel<40>, L.T, smem, ImpCfg<40>::THREADS, tiles,
                               stream, p, d, b, tiles);
-        return tcc_launch(sllg_tcc_implicit_kernel<64>, L.T, smem, Cfg<64>::THREADS, tiles, stream,
+        return tcc_launch(sllg_tcc_implicit_kernel<64>, L.T, smem, ImpCfg<64>::THREADS, tiles, stream,
                           p, d, b, tiles);
     }
     if (!tcc_supported(p.n)) return cudaErrorNotSupported;
