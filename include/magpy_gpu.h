@@ -63,11 +63,11 @@ extern "C" {
                                    implicit midpoint: FP64 state, residual and
                                    convergence test; the dipolar pair sum (partial
                                    sums over 32 sources added in FP64), the
-                                   quasi-Jacobian and the 3x3 solve in FP32 */
+                                   Jacobian and the 3x3 solve in FP32 */
 #define MAGPY_PRECISION_MIXED_TC 2 /* as MIXED, with the dipolar field on the tensor cores
                                       (members sharing one geometry, 2 <= n_particles <= 672;
                                       above 64 particles one thread-block cluster of
-                                      ceil(n/42) CTAs per 64 or 32 members) */
+                                      ceil(n/42) CTAs per 32 to 64 members) */
 
 /* Ensemble of clusters (EnsembleModel.simulate, magpy/model.py:159-208).
  * Every member has n_particles particles.  Per-particle inputs are either
@@ -164,7 +164,9 @@ int magpy_plan_shape(const magpy_plan *plan, int64_t *n_members, int64_t *n_part
  * mode), members_per_warp = 32, 40, 48 (Heun only) or 64
  * puts that many members in each thread-block cluster; 0 takes the count
  * with the fewest waves of resident clusters, then the fewest members (a
- * wave's time grows with its clusters' members). */
+ * wave's time grows with its clusters' members).  Up to 64 particles of a Heun
+ * run a CTA takes 8 to 32 members by the ensemble's size, and 32 once a shape
+ * is set.  Results do not depend on the shape. */
 int magpy_plan_set_launch(magpy_plan *plan, int32_t block_warps, int32_t members_per_warp);
 /* No counterpart in the reference.  Bound of the tensor-core kernel's waits
  * for its MMA completions (MAGPY_PRECISION_MIXED_TC), in polls of the

@@ -1745,7 +1745,12 @@ extern "C" int magpy_adjoint_create(const magpy_ensemble_desc *d, int64_t checkp
     // moments' 3) are kept where that takes 4 GiB at most
     const size_t seg = (size_t)std::min(C, std::max<int64_t>(K, 1)) * P2 * sizeof(float);
     A->a.kept = d->interactions && n > 1 && seg <= ((size_t)4 << 30) / 9;
-    CUDA_TRY(pool_alloc(&A->bufs[2], (A->a.kept ? 9 : 3) * seg));
+    if (A->a.kept && pool_alloc(&A->bufs[2], 9 * seg) != cudaSuccess) {
+        (void)cudaGetLastError();  // no room for them: computed again instead
+        A->bufs[2] = nullptr;
+        A->a.kept = false;
+    }
+    if (!A->a.kept) CUDA_TRY(pool_alloc(&A->bufs[2], 3 * seg));
     CUDA_TRY(pool_alloc(&A->bufs[3], std::max<int64_t>(A->S, 1) * sizeof(double)));
     CUDA_TRY(pool_alloc(&A->bufs[4], 5 * sizeof(double)));
     if (R.shape != MAGPY_FIELD_CONSTANT && K > 0) {
