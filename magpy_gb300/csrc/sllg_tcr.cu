@@ -83,6 +83,9 @@ template <int G0, int G1> struct Cfg {
     static constexpr size_t FLAG = BAR + 10 * 8;        // 9 mbarriers, the tensor-memory address
     static constexpr size_t TOTAL = FLAG + (size_t)4 * (NB + 1);
     static_assert(TOTAL <= 232448, "shared memory");
+    // never two on an SM: each takes all of the tensor memory, and clusters that
+    // waited for one another's would not end
+    static_assert(TOTAL > 114 * 1024, "one CTA an SM");
 };
 
 // Named barrier of the integrating warps.

@@ -25,3 +25,31 @@ def test_resident_forms_match_fp64(gpu_lib, n, E, nb):
     assert np.all(a.status == 0) and np.array_equal(a.steps, b.steps)
     for c in ("mx", "my", "mz"):
         assert np.abs(getattr(a, c) - getattr(b, c)).max() <= 8.4e-6 * 4e5
+
+
+@pytest.mark.parametrize("n", [33, 64, 70, 126])
+def test_failed_member_and_single_sample(gpu_lib, n):
+    """A member whose injected increments hold a NaN is reported and leaves the
+    members of its group and of the other one alone; a run of one sample takes no
+    step."""
+    from magpy_gb300 import core
+    E, steps = 21, 70
+    m0 = np.zeros((n, 3))
+    m0[:, 2] = 1.0
+    loc = np.stack(np.meshgrid(*[np.arange(6)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n] * 2e-8
+    noise = np.random.default_rng(n).normal(size=(E, steps * 3 * n))
+    def run(samples, noise):
+        return core.simulate_ensemble(
+            E, np.full(n, 7e-9), np.full(n, 2e4), m0, m0, loc, 4e5, 0.1, 300.0, False, True, False,
+            5e-14, 5e-14 * (steps - 0.5), samples, np.arange(E) + 11, "sine", 1e4, 3e10,
+            precision="mixed_tc", noise=noise)
+    a, one = run(3, noise), run(1, noise)
+    assert np.all(a.status == 0) and np.all(one.status == 0) and np.all(one.steps == 0)
+    np.testing.assert_array_equal(one.mz[0], a.mz[0])
+    bad = noise.copy()
+    bad[5, 3 * n * 2 + 4] = np.nan
+    b = run(3, bad)
+    assert list(np.nonzero(b.status)[0]) == [5] and b.status[5] == 4
+    keep = np.repeat(np.arange(E) != 5, n)
+    for c in ("mx", "my", "mz"):
+        assert np.array_equal(getattr(a, c)[:, keep], getattr(b, c)[:, keep])
