@@ -21,18 +21,19 @@
 // Parameter sensitivities accumulated along the way:
 //     Gh = sum mu.h (d/d dt), Gw = sum mu.(sr w) (d/d sqrt(dt)),
 //     Ga = sum g.dF/dalpha, Ghapp = sum eta_z s, Gc = sum eta.(D x)/c.
-// Checkpoints every C steps keep the float-float state; each segment is
-// recomputed forward (same code, same bits) into a buffer of moments and
-// then swept backward.
+// The forward pass keeps every step's moments and dipolar fields where they fit
+// (4 GiB); otherwise checkpoints every C steps keep the float-float state, and
+// each segment is recomputed forward (same code, same bits) into a buffer of
+// moments (and fields) and then swept backward.
 //
 // What bounds it: the dipolar sums, by their instructions, table reads and
 // chains.  In a large ensemble a thread integrates particle q of two members
 // (they share the cluster), in packed FP32 instructions on (member A, member B)
 // pairs: each table entry read and each instruction of a sum serves both.  The
-// recomputation keeps its dipolar fields beside the moments, so that a backward
-// step forms four sums in all (two forward, two of the adjoint) instead of
-// six.  27 particles, 2048 members, 512 steps with the host's copies: 8.4 ->
-// 5.4 ms.
+// dipolar fields are kept beside the moments, so that a step takes four sums in
+// all (two forward, two of the adjoint), six where a segment is recomputed, eight
+// without kept fields.  27 particles, 2048 members, 512 steps with the host's
+// copies: 8.4 -> 5.4 ms with a segment's fields kept, 4.0 with the run's.
 #include "common.cuh"
 #include "llg32.cuh"
 #include "plan.hpp"
@@ -213,7 +214,10 @@ struct AdjArgs {
     float happ, dt, sq, alpha, c;
     const int64_t *sched;
     float *ck;            // [K/C + 1][6][pairs] V: checkpoints (hi xyz, lo xyz)
-    float *seg;           // [C][3 or 9][pairs] V: moments (and dipolar fields) of the segment being swept
+    // [C][3 or 9][pairs] V: moments (and dipolar fields) of the segment being
+    // swept; `whole`: [K][9][pairs] of the whole run, written by the forward pass
+    float *seg;
+    bool whole;
     const double *out_scale; // [E] Ms
     double *mx, *my, *mz; // samples [S][P]
     const double *wz;     // [S] dJ/d(reduced m_z of any particle at sample s)
@@ -345,7 +349,30 @@ __device__ inline void write_ck(const AdjArgs &A, const AdjMember<V> &M, int64_t
     }
 }
 
-template <class V, int MAXT, bool SPLIT>
+// Moments m of step k (0-based) and, KEPT, the dipolar fields of its two stages
+// into `seg`, the step's planes at `o`.
+template <bool KEPT, class V>
+__device__ inline void keep_fields(const AdjMember<V> &M, V *o, const V d1[3], const V d2[3])
+{
+    if (KEPT && M.writes)
+        for (int i = 0; i < 3; i++) {
+            o[(3 + i) * M.pairs] = d1[i];
+            o[(6 + i) * M.pairs] = d2[i];
+        }
+}
+
+template <class V>
+__device__ inline void keep_moments(const AdjMember<V> &M, V *o, const V m[3])
+{
+    if (M.writes)
+        for (int i = 0; i < 3; i++) o[i * M.pairs] = m[i];
+}
+
+// WHOLE: every step's moments and dipolar fields are kept for the sweep back,
+// which then forms two sums a step, not the forward pass's two again as well (27
+// particles, 2048 members, 512 steps: 5.4 -> 4.0 ms in all; 1000 members, 256
+// steps: 2.30 -> 1.80).
+template <class V, int MAXT, bool SPLIT, bool WHOLE>
 __global__ void __launch_bounds__(MAXT) adj_forward_kernel(AdjArgs A)
 {
     extern __shared__ float4 smem_a[];
@@ -365,8 +392,11 @@ __global__ void __launch_bounds__(MAXT) adj_forward_kernel(AdjArgs A)
     for (int64_t step = 1; step <= A.K; step++) {
         while (s_next < A.S && A.sched[s_next] == step) write_sample_a(A, M, s_next++, hi, lo);
         V d1[3], d2[3];
+        V *o = WHOLE ? (V *)A.seg + (step - 1) * 9 * M.pairs + M.pair : nullptr;
+        if (WHOLE) keep_moments(M, o, hi);
         fstep<SPLIT>(A, M, hi, lo, step, d1, d2);
-        if (step == next_ck) {
+        if (WHOLE) keep_fields<true>(M, o, d1, d2);
+        if (!WHOLE && step == next_ck) {
             write_ck(A, M, ++ck, hi, lo);
             next_ck += A.C;
         }
@@ -463,30 +493,29 @@ __global__ void __launch_bounds__(MAXT, MAXT == 128 ? 3 : 1) adj_backward_kernel
     const int64_t nseg = (A.K + A.C - 1) / A.C;
     for (int64_t c = nseg - 1; c >= 0; c--) {
         const int64_t k0 = c * A.C, k1 = (k0 + A.C < A.K) ? k0 + A.C : A.K;
-        V hi[3], lo[3];
-        const V *ck = (const V *)A.ck + c * 6 * N2 + M.pair;
-        for (int i = 0; i < 3; i++) {
-            hi[i] = ck[i * N2];
-            lo[i] = ck[(3 + i) * N2];
-        }
         // per step the moments and, KEPT, the dipolar fields of its two stages:
         // the sweep back then forms two sums a step instead of four
         constexpr int PLANES = KEPT ? 9 : 3;
         V *sg = (V *)A.seg + M.pair;
-        if (SPLIT) __syncthreads();  // the other warp has read the last segment
-        for (int64_t k = k0; k < k1; k++) {
-            V *o = sg + (k - k0) * PLANES * N2;
-            if (M.writes)
-                for (int i = 0; i < 3; i++) o[i * N2] = hi[i];
-            V d1[3], d2[3];
-            fstep<SPLIT>(A, M, hi, lo, k + 1, d1, d2);
-            if (KEPT && M.writes)
-                for (int i = 0; i < 3; i++) {
-                    o[(3 + i) * N2] = d1[i];
-                    o[(6 + i) * N2] = d2[i];
-                }
+        if (KEPT && A.whole) {
+            sg += k0 * PLANES * N2;
+        } else {
+            V hi[3], lo[3];
+            const V *ck = (const V *)A.ck + c * 6 * N2 + M.pair;
+            for (int i = 0; i < 3; i++) {
+                hi[i] = ck[i * N2];
+                lo[i] = ck[(3 + i) * N2];
+            }
+            if (SPLIT) __syncthreads();  // the other warp has read the last segment
+            for (int64_t k = k0; k < k1; k++) {
+                V *o = sg + (k - k0) * PLANES * N2;
+                keep_moments(M, o, hi);
+                V d1[3], d2[3];
+                fstep<SPLIT>(A, M, hi, lo, k + 1, d1, d2);
+                keep_fields<KEPT>(M, o, d1, d2);
+            }
+            if (SPLIT) __syncthreads();
         }
-        if (SPLIT) __syncthreads();
         V G[5] = {all<V>(0.f), all<V>(0.f), all<V>(0.f), all<V>(0.f), all<V>(0.f)};
         for (int64_t k = k1 - 1; k >= k0; k--) {
             const V *in = sg + (k - k0) * PLANES * N2;
@@ -564,14 +593,18 @@ static void run(const Launch &L, const AdjArgs &A, bool backward, bool kept, cud
     auto go = [&](auto kernel) { kernel<<<L.grid, L.block, L.shmem, stream>>>(A); };
     if constexpr (WIDTH<V> == 1)
         if (L.split) {
-            if (!backward) go(adj_forward_kernel<V, 64, true>);
+            if (!backward && A.whole) go(adj_forward_kernel<V, 64, true, true>);
+            else if (!backward) go(adj_forward_kernel<V, 64, true, false>);
             else if (kept) go(adj_backward_kernel<V, 64, true, true>);
             else go(adj_backward_kernel<V, 64, true, false>);
             return;
         }
-    if (!backward) {
-        if (small) go(adj_forward_kernel<V, 128, false>);
-        else go(adj_forward_kernel<V, 512, false>);
+    if (!backward && A.whole) {
+        if (small) go(adj_forward_kernel<V, 128, false, true>);
+        else go(adj_forward_kernel<V, 512, false, true>);
+    } else if (!backward) {
+        if (small) go(adj_forward_kernel<V, 128, false, false>);
+        else go(adj_forward_kernel<V, 512, false, false>);
     } else if (kept) {
         if (small) go(adj_backward_kernel<V, 128, false, true>);
         else go(adj_backward_kernel<V, 512, false, true>);
@@ -591,7 +624,7 @@ cudaError_t launch_adjoint(const AdjointArgs &a, bool backward, cudaStream_t str
     A.members = a.p.members; A.m0 = a.p.m0; A.axes = a.p.axes; A.k_red = a.p.k_red;
     A.sr = a.p.sr; A.v_red = a.v_red; A.pr = a.p.pr; A.stab = (const float2 *)a.stab;
     A.happ = a.happ; A.dt = a.dt; A.sq = a.sq; A.alpha = a.alpha; A.c = a.c;
-    A.sched = a.p.sched; A.ck = a.ck; A.seg = a.seg; A.out_scale = a.p.out_scale;
+    A.sched = a.p.sched; A.ck = a.ck; A.seg = a.seg; A.whole = a.whole; A.out_scale = a.p.out_scale;
     A.mx = a.p.mx; A.my = a.p.my; A.mz = a.p.mz; A.wz = a.wz; A.grad = a.grad;
     A.status = a.p.status;
     if (A.E == 0) return cudaSuccess;

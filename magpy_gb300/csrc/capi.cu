@@ -1741,14 +1741,21 @@ extern "C" int magpy_adjoint_create(const magpy_ensemble_desc *d, int64_t checkp
     // checkpoints and the segment's moments, two members side by side
     const size_t P2 = (size_t)(E + 1) / 2 * 2 * n;
     CUDA_TRY(pool_alloc(&A->bufs[1], nck * 6 * P2 * sizeof(float)));
-    // the dipolar fields of a segment (6 floats a particle and step beside the
-    // moments' 3) are kept where that takes 4 GiB at most
-    const size_t seg = (size_t)std::min(C, std::max<int64_t>(K, 1)) * P2 * sizeof(float);
-    A->a.kept = d->interactions && n > 1 && seg <= ((size_t)4 << 30) / 9;
-    if (A->a.kept && pool_alloc(&A->bufs[2], 9 * seg) != cudaSuccess) {
-        (void)cudaGetLastError();  // no room for them: computed again instead
+    // the dipolar fields (6 floats a particle and step beside the moments' 3) are
+    // kept where that takes 4 GiB at most: of the whole run, else of a segment;
+    // with no room for them either they are computed again
+    const size_t limit = (size_t)4 << 30, steps = (size_t)std::max<int64_t>(K, 1);
+    const size_t seg = std::min((size_t)C, steps) * P2 * sizeof(float);
+    const auto keep = [&](size_t planes) {
+        if (pool_alloc(&A->bufs[2], planes) == cudaSuccess) return true;
+        (void)cudaGetLastError();
         A->bufs[2] = nullptr;
-        A->a.kept = false;
+        return false;
+    };
+    if (d->interactions && n > 1) {
+        if (P2 > 0 && steps <= limit / (9 * P2 * sizeof(float)))
+            A->a.kept = A->a.whole = keep(9 * steps * P2 * sizeof(float));
+        if (!A->a.kept && seg <= limit / 9) A->a.kept = keep(9 * seg);
     }
     if (!A->a.kept) CUDA_TRY(pool_alloc(&A->bufs[2], 3 * seg));
     CUDA_TRY(pool_alloc(&A->bufs[3], std::max<int64_t>(A->S, 1) * sizeof(double)));

@@ -163,6 +163,7 @@ struct AdjointArgs {
     int C, interactions;
     float *ck, *seg;      // checkpoints, and the moments of the segment being swept
     bool kept = false;    // seg has room for the dipolar fields too
+    bool whole = false;   // ... of every step of the run
     const double *wz;     // [S]
     double *grad;         // [5]
 };

@@ -44,3 +44,15 @@ def test_forms_agree_without_interactions(gpu_lib):
     a, b = _gradient(8, 1, 40, 16, False), _gradient(8, 3001, 40, 16, False)
     for x, y in zip(a[1:], b[1:]):
         np.testing.assert_allclose(x, y, rtol=5e-5)
+
+
+@pytest.mark.parametrize("steps,every", [(1100, 256), (1100, 1000)])
+def test_whole_run_and_segments_agree(gpu_lib, steps, every):
+    """The fields of the whole run kept by the forward pass (2049 members) or of a
+    segment by its recomputation (4098 members, 4.4 GB for the whole run): the same
+    members twice as often, the same bits of each member's sensitivities, their
+    double-precision sums in another order."""
+    a, b = _gradient(27, 683, steps, every), _gradient(27, 1366, steps, every)
+    np.testing.assert_allclose(a[0], b[0], rtol=1e-11)
+    for x, y in zip(a[1:], b[1:]):
+        np.testing.assert_allclose(x, y, rtol=1e-9)
