@@ -231,7 +231,7 @@ finished:
 }
 
 // Two particles per thread: the two of a dimer, or two members of one particle
-// each (SINGLES).
+// each (SINGLES; ONE: one member, the second half unused).
 //
 // What bounds them: instruction issue (531 instructions a particle and step of
 // a dimer with a thread per particle).  The state update and the stage map run
@@ -241,14 +241,14 @@ finished:
 // half: no exchange, no table read.  50000 dimers, 1000 steps: 3.02 -> 0.98 ms.
 // (Two particles per thread with the general pair sum did not pay: 3 particles
 // 1.35 -> 1.07 us a step, but 16 and more slower, 64 14.6 -> 17.4 us.)
-template <bool SINGLES>
+template <bool SINGLES, bool ONE = false>
 __global__ void __launch_bounds__(128)
     sllg_mixed_two_kernel(DevPlan p)
 {
     const int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t e = SINGLES ? 2 * item : item;  // the first member
+    const int64_t e = SINGLES && !ONE ? 2 * item : item;  // the first member
     if (e >= p.E) return;
-    const bool live1 = !SINGLES || e + 1 < p.E;  // a second particle
+    const bool live1 = !SINGLES || (!ONE && e + 1 < p.E);  // a second particle
     const MemberDev *md = p.members + e, *md1 = SINGLES && live1 ? md + 1 : md;
     const float sq = (float)md->sqrt_dt, happ = (float)md->happ;
     const float2 dt2 = f2((float)md->dt);
@@ -331,7 +331,8 @@ __global__ void __launch_bounds__(128)
                 for (int c = 0; c < 3; c++)
                     sw[c] = mul2(ssr, make_float2((float)wp[c], live1 ? (float)wp[noise1 + c] : 0.f));
             } else if (SINGLES) {
-                const Normals4 a = wiener_normals(seed, step, 0), b = wiener_normals(seed1, step, 0);
+                const Normals4 a = wiener_normals(seed, step, 0);
+                const Normals4 b = ONE ? a : wiener_normals(seed1, step, 0);
                 sw[0] = mul2(ssr, make_float2(a.a, b.a));
                 sw[1] = mul2(ssr, make_float2(a.b, b.b));
                 sw[2] = mul2(ssr, make_float2(a.c, b.c));
@@ -690,10 +691,16 @@ cudaError_t launch_mixed(const DevPlan &p, cudaStream_t stream)
     if (n <= 2) {
         // one warp per CTA while that leaves every warp a sub-partition or a
         // few to share one, so that no SM gets a CTA more than another
-        const int64_t items = n == 1 ? (p.E + 1) / 2 : p.E;
+        // single particles: one a thread while every warp has a sub-partition to
+        // itself (a step is then a chain, and two lengthen it: 137 against 177 us
+        // for 400 steps, 170 against 236 with renormalisation, at 19456 members),
+        // two a thread from there (203 against 178, 238 against 235 at 20000)
+        const bool one = n == 1 && p.E <= 32 * 4 * 152;
+        const int64_t items = n == 1 && !one ? (p.E + 1) / 2 : p.E;
         const int threads = items <= 32 * 4 * 4 * 152 ? 32 : 128;
         const unsigned blocks = (unsigned)((items + threads - 1) / threads);
-        if (n == 1) sllg_mixed_two_kernel<true><<<blocks, threads, 0, stream>>>(p);
+        if (one) sllg_mixed_two_kernel<true, true><<<blocks, threads, 0, stream>>>(p);
+        else if (n == 1) sllg_mixed_two_kernel<true><<<blocks, threads, 0, stream>>>(p);
         else sllg_mixed_two_kernel<false><<<blocks, threads, 0, stream>>>(p);
         return cudaGetLastError();
     }

@@ -51,3 +51,20 @@ def test_two_per_thread_status(gpu_lib, n):
     keep = np.repeat(np.arange(E) != 2, n)
     for c in ("mx", "my", "mz"):
         assert np.array_equal(getattr(a, c)[:, keep], getattr(b, c)[:, keep])
+
+
+@pytest.mark.parametrize("renorm", [False, True])
+def test_one_or_two_members_per_thread_agree(gpu_lib, renorm):
+    """Single particles: one member a thread up to 32 x 4 x 152 members, two above;
+    the same bits."""
+    from magpy_gb300 import core
+    one = np.ones(1)
+    def run(E):
+        return core.simulate_ensemble(
+            E, 7e-9 * one, 2e4 * one, np.array([[0, 0.6, 0.8]]), np.array([[1.0, 0, 0]]),
+            np.zeros((1, 3)), 4e5, 0.1, 300.0, renorm, False, False, 1e-13, 1e-13 * 30.5, 3,
+            np.arange(E), "sine", 1e4, 3e10, precision="mixed")
+    a, b = run(32 * 4 * 152), run(32 * 4 * 152 + 1)
+    assert np.all(a.status == 0) and np.all(b.status == 0)
+    for c in ("mx", "my", "mz"):
+        assert np.array_equal(getattr(a, c), getattr(b, c)[:, :-1])
