@@ -442,9 +442,9 @@ __global__ void __launch_bounds__(HeunCfg<NB>::THREADS, 1)
         // CTA (checked every 64 steps, and once after the loop), or injected
         // noise running out
         // (the same for every member of the launch)
-        if ((step & 63) == 1) {
-            tc::cluster_sync();
-            if (cluster_any_error(sErr, L.T)) { status |= ST_WATCHDOG; stop = true; }
+        if ((step - 1) % 64 == 0 && cluster_check(sErr, L.T, (step - 1) / 64)) {
+            status |= ST_WATCHDOG;
+            stop = true;
         }
         if (!stop && step > noise_steps) { status |= ST_NOISE_EXHAUSTED; stop = true; }
         if (stop) break;
@@ -559,9 +559,7 @@ __global__ void __launch_bounds__(HeunCfg<NB>::THREADS, 1)
     }
     // the loop leaves `step` one past the last completed step
     step -= 1;
-    // a wait that ran out after the last check is reported too
-    tc::cluster_sync();
-    if (cluster_any_error(sErr, L.T)) status |= ST_WATCHDOG;
+    if (cluster_last_check(sErr, L.T)) status |= ST_WATCHDOG;
     if (p.mx)  // samples a stopped member never reached
         for (int64_t s = s_next; s < S; s++)
 #pragma unroll
@@ -863,9 +861,9 @@ __global__ void __launch_bounds__(ImpCfg<NB>::THREADS, 1)
     int64_t next_sample = S > 1 ? sched[1] : -1;
     const int64_t noise_steps = p.noise ? m0d->noise_len / per_step : K;
     for (step = 1; step <= K; step++) {
-        if ((step & 63) == 1) {
-            tc::cluster_sync();
-            if (cluster_any_error(sErr, L.T)) { status |= ST_WATCHDOG; stop = true; }
+        if ((step - 1) % 64 == 0 && cluster_check(sErr, L.T, (step - 1) / 64)) {
+            status |= ST_WATCHDOG;
+            stop = true;
         }
         if (!stop && step > noise_steps) { status |= ST_NOISE_EXHAUSTED; stop = true; }
         if (stop) break;
@@ -1040,9 +1038,7 @@ __global__ void __launch_bounds__(ImpCfg<NB>::THREADS, 1)
         tc::cluster_sync();
     }
     step -= 1;
-    // a wait that ran out after the last check is reported too
-    tc::cluster_sync();
-    if (cluster_any_error(sErr, L.T)) status |= ST_WATCHDOG;
+    if (cluster_last_check(sErr, L.T)) status |= ST_WATCHDOG;
     if (p.mx)
         for (int64_t s2 = s_next; s2 < S; s2++)
 #pragma unroll

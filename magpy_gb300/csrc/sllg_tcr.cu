@@ -318,9 +318,9 @@ __global__ void __launch_bounds__(Cfg<G0, G1>::THREADS, 1)
     for (step = 1; step <= K; step++) {
         // every thread of the cluster comes here with the same step: whether to
         // go on is decided together
-        if ((step - 1) % CHECK == 0) {
-            tc::cluster_sync();
-            if (cluster_any_error(sErr, T)) { status |= ST_WATCHDOG; stop = true; }
+        if ((step - 1) % CHECK == 0 && cluster_check(sErr, T, (step - 1) / CHECK)) {
+            status |= ST_WATCHDOG;
+            stop = true;
         }
         if (!stop && step > noise_steps) { status |= ST_NOISE_EXHAUSTED; stop = true; }
         if (stop) break;
@@ -511,9 +511,7 @@ __global__ void __launch_bounds__(Cfg<G0, G1>::THREADS, 1)
         tc::mma_commit_warp(drain_b);
         tc::mbar_wait_bounded(drain_b, 0, DRAIN_LIMIT);
     }
-    // a wait that ran out after the last check is reported too
-    tc::cluster_sync();
-    if (cluster_any_error(sErr, T)) status |= ST_WATCHDOG;
+    if (cluster_last_check(sErr, T)) status |= ST_WATCHDOG;
 #pragma unroll
     for (int g = 0; g < 2; g++)
         if (valid(g)) {

@@ -116,18 +116,43 @@ __device__ inline void tcc_load_d_tmem(uint32_t dcol, int K, const __half *dtile
     tc::fence_before_sync();
 }
 
-// The OR over the cluster of each CTA's error word (every thread gets it).
-__device__ inline int cluster_any_error(int *sErr, int T)
+// The OR over the cluster of a word of each CTA (every thread gets it).  No CTA
+// may write its word before every CTA has read it.
+__device__ inline int cluster_or(const int *word, int T)
 {
     __shared__ int any;
     if (threadIdx.x == 0) {
         int a = 0;
-        const uint32_t base = tc::smem_addr(sErr);
+        const uint32_t base = tc::smem_addr(word);
         for (int r = 0; r < T; r++) a |= tc::ld_cluster_s32(tc::mapa(base, (uint32_t)r));
         any = a;
     }
     __syncthreads();
     return any;
+}
+
+// A check of the step loop: whether any CTA of the cluster was marked before it,
+// the same answer in every CTA.  A CTA that is ahead enters the step, and may mark
+// itself there, while another still reads: so each publishes its error word as it
+// stands before the barrier, in one of two words by the check's number (the word
+// is written again two checks later, past the next check's barrier, at which
+// every CTA arrives after its reads).
+__device__ inline int cluster_check(const int *sErr, int T, int64_t number)
+{
+    __shared__ int marked[2];
+    __syncthreads();  // this CTA's earlier marks
+    int *word = &marked[number & 1];
+    if (threadIdx.x == 0) *word = *(const volatile int *)sErr;
+    tc::cluster_sync();
+    return cluster_or(word, T);
+}
+
+// The check after the last step, past which no CTA marks itself: a wait that ran
+// out after the last check of the loop is reported too.
+__device__ inline int cluster_last_check(const int *sErr, int T)
+{
+    tc::cluster_sync();
+    return cluster_or(sErr, T);
 }
 
 template <class Kern>
