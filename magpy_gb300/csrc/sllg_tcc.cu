@@ -665,11 +665,11 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
 // every CTA takes the same decisions from the same numbers.
 //
 // What bounds it: the FP64 pipe (two lanes a clock an SM), on which conversions
-// run too.  A particle's iteration is 35 FP64 instructions (stage increments
-// dt a + B dwm = F(m, dt h + sr dwm), the residual, the update), its
+// run too.  A particle's iteration is 32 FP64 instructions (stage increments
+// dt a + B dwm = F(m, dt h + sr dwm), the residual, the update and its share of
+// the stopping norm, a sum that squares of any FP32 number do not overflow), its
 // conversions are integer (narrow, widen), as are six of its products (stage_map),
-// its share of the stopping norm is summed as float-float (exact squares), and
-// starting from the explicit midpoint saves one iteration of four.  512 members
+// and starting from the explicit midpoint saves one iteration of four.  512 members
 // of 512 particles, 40 steps: 18.0 -> 11.4 ms.
 
 // Per-particle constants of a CTA's 42 particles: FP64 for the residual,
@@ -970,7 +970,7 @@ __global__ void __launch_bounds__(ImpCfg<NB>::THREADS, 1)
             }
             if (!__syncthreads_or(go)) break;
             field();  // dipolar field at every member's current iterate
-            DDf dsum{0.f, 0.f};
+            double part_d = 0.0;
             int sing = 0;
             if (go) {
 #pragma unroll
@@ -1000,18 +1000,16 @@ __global__ void __launch_bounds__(ImpCfg<NB>::THREADS, 1)
                             continue;  // the member stops with its current iterate
                         }
                         for (int c = 0; c < 3; c++) {
-                            // exact square, added to the float-float sum
-                            const float s2 = sol[c] * sol[c];
-                            dsum.lo += __fmaf_rn(sol[c], sol[c], -s2);
-                            dsum = dd_add_ts(dsum, s2);
-                            x[i][k][c] = xt[c] + widen(sol[c]);
+                            const double d = widen(sol[c]);
+                            part_d = fma(d, d, part_d);
+                            x[i][k][c] = xt[c] + d;
                         }
                     }
             }
             write_B(wb ^ 1);
             wb ^= 1;
             double d2;
-            cluster_sum((double)dsum.hi + (double)dsum.lo, sing, d2, sing_any);
+            cluster_sum(part_d, sing, d2, sing_any);
             err = sqrt(d2);
             if (go && sing_any) { mflag |= ST_SINGULAR; active = false; }
         }
