@@ -34,6 +34,16 @@ __device__ inline DD dd_add(DD a, float d)
     return DD{hi, e - (hi - s)};
 }
 
+// dd_add of two items in packed FP32 instructions.
+__device__ inline void dd_add2(float2 &hi, float2 &lo, float2 d)
+{
+    const float2 s = add2(hi, d);
+    const float2 v = add2(s, neg2(hi));
+    const float2 e = add2(add2(add2(hi, neg2(add2(s, neg2(v)))), add2(d, neg2(v))), lo);
+    hi = add2(s, e);
+    lo = add2(e, neg2(add2(hi, neg2(s))));
+}
+
 struct MemberF {
     float dt, sq, alpha, happ;
     int shape;
@@ -329,7 +339,7 @@ __global__ void __launch_bounds__(128)
             stage(hi, hf.x, sw, a);
             for (int c = 0; c < 3; c++) xt[c] = add2(hi[c], a[c]);
             stage(xt, hf.y, sw, b);
-            for (int c = 0; c < 3; c++) dd_add_ts2(hi[c], lo[c], mul2(f2(0.5f), add2(a[c], b[c])));
+            for (int c = 0; c < 3; c++) dd_add2(hi[c], lo[c], mul2(f2(0.5f), add2(a[c], b[c])));
             if (renorm) {
                 const float2 n2 = fma2(hi[2], hi[2], fma2(hi[1], hi[1], mul2(hi[0], hi[0])));
                 const float2 inv = make_float2(1.0f / sqrtf(n2.x), live1 ? 1.0f / sqrtf(n2.y) : 0.f);
