@@ -9,10 +9,10 @@
 // table computed in FP64 (t = step*dt reaches 1e6 in reduced units, beyond
 // FP32 resolution).
 //
-// Drift and diffusion are the one map F(m, v) they share, of v = dt h + sqrt(dt)
-// sr w (llg32.cuh), evaluated once a stage: with the two apart a step of 11
-// particles took 1.40 us against 1.33 (1000 members), 4.20 against 3.82 (8000),
-// of 27 particles 2.77 against 2.55 and 13.4 against 12.6.
+// Drift and diffusion are the one map F(m, v) they share, of v = h + (sr / sqrt(dt))
+// w, evaluated once a stage and times dt: against the two apart a step of 11
+// particles, 8000 members takes 4.20 us instead of 4.45, of 27 particles 2.83
+// instead of 2.99 (1000 members) and 13.2 instead of 13.7 (8000).
 #include "common.cuh"
 #include <algorithm>
 #include "plan.hpp"
@@ -44,8 +44,35 @@ __device__ inline void dd_add2(float2 &hi, float2 &lo, float2 d)
     lo = add2(e, neg2(add2(hi, neg2(s))));
 }
 
+// F(m, v) = -(m x v) - alpha m x (m x v), written as llg::drift (lib/llg.cpp:14-29):
+// without the products m_i m_i v_i, which cancel in the expanded form (at alpha = 1
+// and T = 0 that form's error is 1.4 to 1.6 times this one's).  With v = h +
+// (sr / sqrt(dt)) w, dt F is the stage's increment dt a + sqrt(dt) B w.
+__device__ inline void llg_map(float o[3], const float m[3], float alpha, const float v[3])
+{
+    const float q0 = m[0] * m[0], q1 = m[1] * m[1], q2 = m[2] * m[2];
+    const float p0 = m[0] * v[0], p1 = m[1] * v[1], p2 = m[2] * v[2];
+    o[0] = fmaf(alpha, v[0] * (q1 + q2) - m[0] * (p1 + p2), m[2] * v[1] - m[1] * v[2]);
+    o[1] = fmaf(alpha, v[1] * (q0 + q2) - m[1] * (p0 + p2), m[0] * v[2] - m[2] * v[0]);
+    o[2] = fmaf(alpha, v[2] * (q0 + q1) - m[2] * (p0 + p1), m[1] * v[0] - m[0] * v[1]);
+}
+
+// ... of two items in packed FP32 instructions.
+__device__ inline void llg_map2(float2 o[3], const float2 m[3], float2 alpha, const float2 v[3])
+{
+    const float2 q0 = mul2(m[0], m[0]), q1 = mul2(m[1], m[1]), q2 = mul2(m[2], m[2]);
+    const float2 p0 = mul2(m[0], v[0]), p1 = mul2(m[1], v[1]), p2 = mul2(m[2], v[2]);
+    const auto row = [&](int c, int i, int j, float2 q, float2 p) {
+        const float2 cross = fma2(m[j], v[i], neg2(mul2(m[i], v[j])));
+        o[c] = fma2(alpha, fma2(v[c], q, neg2(mul2(m[c], p))), cross);
+    };
+    row(0, 1, 2, add2(q1, q2), add2(p1, p2));
+    row(1, 2, 0, add2(q0, q2), add2(p0, p2));
+    row(2, 0, 1, add2(q0, q1), add2(p0, p1));
+}
+
 struct MemberF {
-    float dt, sq, alpha, happ;
+    float dt, alpha, happ;
     int shape;
     const float *ftab;     // [K][2] field at t=step*dt and t+dt, or null (constant)
     const float4 *pr;      // pair table (r0, r1, r2, P), [N][N], index j*n + q
@@ -119,7 +146,6 @@ __global__ void __launch_bounds__(MAXT > 0 ? MAXT : 640)
     M.n = n;
     const MemberDev *md = p.members + e;
     M.dt = (float)md->dt;
-    M.sq = (float)md->sqrt_dt;
     M.alpha = (float)md->alpha;
     M.happ = (float)md->happ;
     M.shape = md->shape;
@@ -138,7 +164,7 @@ __global__ void __launch_bounds__(MAXT > 0 ? MAXT : 640)
         x[c].hi = (float)v;
         x[c].lo = (float)(v - (double)x[c].hi);
     }
-    const float k = (float)p.k_red[g], ssr = M.sq * (float)p.sr[g];
+    const float k = (float)p.k_red[g], sd = (float)(p.sr[g] / md->sqrt_dt);
     const bool renorm = md->renorm != 0;
     const uint64_t seed = md->seed;
     const double scale = p.out_scale[e];
@@ -182,17 +208,15 @@ __global__ void __launch_bounds__(MAXT > 0 ? MAXT : 640)
                 h2 = f.y;
             }
             for (int c = 0; c < 3; c++) px[c] = pxd[c].hi;
-            // drift and diffusion are one map of v = dt h + sqrt(dt) sr w
-            const float sw[3] = {ssr * w[0], ssr * w[1], ssr * w[2]};
-            float h[3], v[3], a[3], b[3], xt[3];
+            float h[3], a[3], b[3], xt[3];
             field32(M, h, px, ax, k, h1);
-            for (int c = 0; c < 3; c++) v[c] = fmaf(M.dt, h[c], sw[c]);
-            llg_F(a, px, M.alpha, v);
-            for (int c = 0; c < 3; c++) xt[c] = px[c] + a[c];
+            for (int c = 0; c < 3; c++) h[c] = fmaf(sd, w[c], h[c]);
+            llg_map(a, px, M.alpha, h);
+            for (int c = 0; c < 3; c++) xt[c] = fmaf(M.dt, a[c], px[c]);
             field32(M, h, xt, ax, k, h2);
-            for (int c = 0; c < 3; c++) v[c] = fmaf(M.dt, h[c], sw[c]);
-            llg_F(b, xt, M.alpha, v);
-            for (int c = 0; c < 3; c++) x[c] = dd_add(pxd[c], 0.5f * (a[c] + b[c]));
+            for (int c = 0; c < 3; c++) h[c] = fmaf(sd, w[c], h[c]);
+            llg_map(b, xt, M.alpha, h);
+            for (int c = 0; c < 3; c++) x[c] = dd_add(pxd[c], 0.5f * M.dt * (a[c] + b[c]));
             if (renorm) {
                 const float nrm = sqrtf(x[0].hi * x[0].hi + x[1].hi * x[1].hi + x[2].hi * x[2].hi);
                 const float inv = 1.0f / nrm;
@@ -231,7 +255,7 @@ finished:
 // on both particles at once in packed FP32 instructions (llg32.cuh), drift and
 // diffusion as the one map they share; the two particles of a dimer share a
 // generator call (six normals), and each one's source is the pair's other
-// half: no exchange, no table read.  50000 dimers, 1000 steps: 3.02 -> 0.98 ms.
+// half: no exchange, no table read.  50000 dimers, 1000 steps: 3.02 -> 1.04 ms.
 // (Two particles per thread with the general pair sum did not pay: 3 particles
 // 1.35 -> 1.07 us a step, but 16 and more slower, 64 14.6 -> 17.4 us.)
 template <bool SINGLES, bool ONE = false>
@@ -243,8 +267,8 @@ __global__ void __launch_bounds__(128)
     if (e >= p.E) return;
     const bool live1 = !SINGLES || (!ONE && e + 1 < p.E);  // a second particle
     const MemberDev *md = p.members + e, *md1 = SINGLES && live1 ? md + 1 : md;
-    const float sq = (float)md->sqrt_dt, happ = (float)md->happ;
-    const float2 dt2 = f2((float)md->dt);
+    const float happ = (float)md->happ;
+    const float2 dt2 = f2((float)md->dt), hdt2 = f2(0.5f * (float)md->dt);
     const float2 al2 = make_float2((float)md->alpha, (float)md1->alpha);
     const float2 *ftab =
         md->shape == FIELD_CONSTANT ? nullptr : reinterpret_cast<const float2 *>(p.ftab);
@@ -268,7 +292,8 @@ __global__ void __launch_bounds__(128)
         plo[c] = lo[c];
     }
     const float2 k = make_float2((float)p.k_red[g], live1 ? (float)p.k_red[g + 1] : 0.f);
-    const float2 ssr = make_float2(sq * (float)p.sr[g], live1 ? sq * (float)p.sr[g + 1] : 0.f);
+    const float2 sd = make_float2((float)(p.sr[g] / md->sqrt_dt),
+                                  live1 ? (float)(p.sr[g + 1] / md->sqrt_dt) : 0.f);
     // dimer: source 1 at particle 0, source 0 at particle 1
     float2 dr[3] = {f2(0.f), f2(0.f), f2(0.f)}, dp = f2(0.f);
     if (!SINGLES && md->interactions) {
@@ -288,20 +313,20 @@ __global__ void __launch_bounds__(128)
             if (live1) out[c][1] = ((double)h[c].y + (double)l[c].y) * scale[1];
         }
     };
-    // v = dt h + sqrt(dt) sr w at the moments m, and the map's increment
-    auto stage = [&](const float2 m[3], float hz, const float2 sw[3], float2 inc[3]) {
+    // the map of h + (sr / sqrt(dt)) w at the moments m
+    auto stage = [&](const float2 m[3], float hz, const float2 w[3], float2 o[3]) {
         float2 hd[3] = {f2(0.f), f2(0.f), f2(hz)};
         if (!SINGLES) {
-            const float2 o[3] = {make_float2(m[0].y, m[0].x), make_float2(m[1].y, m[1].x),
+            const float2 s[3] = {make_float2(m[0].y, m[0].x), make_float2(m[1].y, m[1].x),
                                  make_float2(m[2].y, m[2].x)};
             const float2 d3 =
-                mul2(f2(3.f), fma2(o[2], dr[2], fma2(o[1], dr[1], mul2(o[0], dr[0]))));
-            for (int c = 0; c < 3; c++) hd[c] = fma2(dp, fma2(d3, dr[c], neg2(o[c])), hd[c]);
+                mul2(f2(3.f), fma2(s[2], dr[2], fma2(s[1], dr[1], mul2(s[0], dr[0]))));
+            for (int c = 0; c < 3; c++) hd[c] = fma2(dp, fma2(d3, dr[c], neg2(s[c])), hd[c]);
         }
         const float2 dot = mul2(fma2(m[2], ax[2], fma2(m[1], ax[1], mul2(m[0], ax[0]))), k);
         float2 v[3];
-        for (int c = 0; c < 3; c++) v[c] = fma2(dt2, fma2(dot, ax[c], hd[c]), sw[c]);
-        llg_F2(inc, m, al2, v);
+        for (int c = 0; c < 3; c++) v[c] = fma2(sd, w[c], fma2(dot, ax[c], hd[c]));
+        llg_map2(o, m, al2, v);
     };
 
     sample(0, hi, lo);
@@ -313,7 +338,7 @@ __global__ void __launch_bounds__(128)
         while ((int64_t)step < ks) {
             for (int c = 0; c < 3; c++) { phi[c] = hi[c]; plo[c] = lo[c]; }
             step++;
-            float2 sw[3];
+            float2 w[3];
             if (noise) {
                 if ((int64_t)step * per_step > md->noise_len) {
                     status |= ST_NOISE_EXHAUSTED;
@@ -322,24 +347,24 @@ __global__ void __launch_bounds__(128)
                 }
                 const double *wp = noise + (int64_t)(step - 1) * per_step;
                 for (int c = 0; c < 3; c++)
-                    sw[c] = mul2(ssr, make_float2((float)wp[c], live1 ? (float)wp[noise1 + c] : 0.f));
+                    w[c] = make_float2((float)wp[c], live1 ? (float)wp[noise1 + c] : 0.f);
             } else if (SINGLES) {
                 const Normals4 a = wiener_normals(seed, step, 0);
                 const Normals4 b = ONE ? a : wiener_normals(seed1, step, 0);
-                sw[0] = mul2(ssr, make_float2(a.a, b.a));
-                sw[1] = mul2(ssr, make_float2(a.b, b.b));
-                sw[2] = mul2(ssr, make_float2(a.c, b.c));
+                w[0] = make_float2(a.a, b.a);
+                w[1] = make_float2(a.b, b.b);
+                w[2] = make_float2(a.c, b.c);
             } else {
                 const PairNormals r = wiener_pair(seed, step, 0);
-                for (int c = 0; c < 3; c++) sw[c] = mul2(ssr, make_float2(r.n[c], r.n[3 + c]));
+                for (int c = 0; c < 3; c++) w[c] = make_float2(r.n[c], r.n[3 + c]);
             }
             float2 hf = f2(happ);
             if (ftab) hf = __ldg(ftab + (step - 1));
             float2 a[3], b[3], xt[3];
-            stage(hi, hf.x, sw, a);
-            for (int c = 0; c < 3; c++) xt[c] = add2(hi[c], a[c]);
-            stage(xt, hf.y, sw, b);
-            for (int c = 0; c < 3; c++) dd_add2(hi[c], lo[c], mul2(f2(0.5f), add2(a[c], b[c])));
+            stage(hi, hf.x, w, a);
+            for (int c = 0; c < 3; c++) xt[c] = fma2(dt2, a[c], hi[c]);
+            stage(xt, hf.y, w, b);
+            for (int c = 0; c < 3; c++) dd_add2(hi[c], lo[c], mul2(hdt2, add2(a[c], b[c])));
             if (renorm) {
                 const float2 n2 = fma2(hi[2], hi[2], fma2(hi[1], hi[1], mul2(hi[0], hi[0])));
                 const float2 inv = make_float2(1.0f / sqrtf(n2.x), live1 ? 1.0f / sqrtf(n2.y) : 0.f);
@@ -376,8 +401,7 @@ finished:
 // MPC members (one member per CTA streams the whole n x n table through L1
 // once per field evaluation).  Moments of the CTA's members are exchanged in
 // shared memory, one buffer per Heun stage; between the stages a member
-// keeps its state, its scaled increments sqrt(dt) sr w and s1, the first stage's
-// map.
+// keeps its state, its increments w and s1, the first stage's map.
 template <int MPC, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (MPC == 2 ? 3 : 2) : 1)
     sllg_mixed_multi_kernel(DevPlan p, const float *ftab_all, const float4 *pr_all)
@@ -387,7 +411,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (MPC == 2 ? 3 : 2) : 1)
     const bool active = q < n;
     const int64_t e0 = (int64_t)blockIdx.x * MPC;
     const MemberDev *md0 = p.members + e0;
-    const float dt = (float)md0->dt, sq = (float)md0->sqrt_dt, alpha = (float)md0->alpha;
+    const float dt = (float)md0->dt, alpha = (float)md0->alpha;
     const float happ = (float)md0->happ;
     const float *ftab = (md0->shape == FIELD_CONSTANT) ? nullptr : ftab_all;
     const float4 *pr = pr_all + md0->cluster_off;
@@ -396,7 +420,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (MPC == 2 ? 3 : 2) : 1)
     const int64_t P = p.P;
     const int64_t g0 = md0->pbase + (active ? q : 0);
     const float ax[3] = {(float)p.axes[g0], (float)p.axes[P + g0], (float)p.axes[2 * P + g0]};
-    const float k = (float)p.k_red[g0], ssr = sq * (float)p.sr[g0];
+    const float k = (float)p.k_red[g0], sd = (float)(p.sr[g0] / md0->sqrt_dt);
     const int64_t S = p.S;
     const int64_t *sched = p.sched + md0->sched_off;
     const int64_t per_step = 3 * (int64_t)n;
@@ -483,14 +507,12 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (MPC == 2 ? 3 : 2) : 1)
                 const float h[3] = {dot * ax[0] + hd[m][0], dot * ax[1] + hd[m][1],
                                     dot * ax[2] + h1 + hd[m][2]};
                 float v[3];
-                for (int c = 0; c < 3; c++) {
-                    w[m][c] *= ssr;
-                    v[c] = fmaf(dt, h[c], w[m][c]);
-                }
-                llg_F(s1[m], px, alpha, v);
+                for (int c = 0; c < 3; c++) v[c] = fmaf(sd, w[m][c], h[c]);
+                llg_map(s1[m], px, alpha, v);
                 if (active)
-                    buf1[m * n + q] = make_float4(px[0] + s1[m][0], px[1] + s1[m][1],
-                                                  px[2] + s1[m][2], 0.f);
+                    buf1[m * n + q] = make_float4(fmaf(dt, s1[m][0], px[0]),
+                                                  fmaf(dt, s1[m][1], px[1]),
+                                                  fmaf(dt, s1[m][2], px[2]), 0.f);
             }
             __syncthreads();
             // stage 2: field at the predictor
@@ -510,16 +532,17 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (MPC == 2 ? 3 : 2) : 1)
                 }
 #pragma unroll
             for (int m = 0; m < MPC; m++) {
-                const float xt[3] = {pxd[m][0].hi + s1[m][0], pxd[m][1].hi + s1[m][1],
-                                     pxd[m][2].hi + s1[m][2]};
+                const float xt[3] = {fmaf(dt, s1[m][0], pxd[m][0].hi),
+                                     fmaf(dt, s1[m][1], pxd[m][1].hi),
+                                     fmaf(dt, s1[m][2], pxd[m][2].hi)};
                 const float dot = (xt[0] * ax[0] + xt[1] * ax[1] + xt[2] * ax[2]) * k;
                 const float h[3] = {dot * ax[0] + hd[m][0], dot * ax[1] + hd[m][1],
                                     dot * ax[2] + h2 + hd[m][2]};
                 float v[3], b[3];
-                for (int c = 0; c < 3; c++) v[c] = fmaf(dt, h[c], w[m][c]);
-                llg_F(b, xt, alpha, v);
+                for (int c = 0; c < 3; c++) v[c] = fmaf(sd, w[m][c], h[c]);
+                llg_map(b, xt, alpha, v);
                 for (int c = 0; c < 3; c++)
-                    x[m][c] = dd_add(pxd[m][c], 0.5f * (s1[m][c] + b[c]));
+                    x[m][c] = dd_add(pxd[m][c], 0.5f * dt * (s1[m][c] + b[c]));
                 if (renorm) {
                     const float nrm = sqrtf(x[m][0].hi * x[m][0].hi + x[m][1].hi * x[m][1].hi +
                                             x[m][2].hi * x[m][2].hi);
@@ -688,9 +711,11 @@ cudaError_t launch_mixed(const DevPlan &p, cudaStream_t stream)
         // one warp per CTA while that leaves every warp a sub-partition or a
         // few to share one, so that no SM gets a CTA more than another
         // single particles: one a thread while every warp has a sub-partition to
-        // itself (a step is then a chain, and two lengthen it: 137 against 177 us
-        // for 400 steps, 170 against 236 with renormalisation, at 19456 members),
-        // two a thread from there (203 against 178, 238 against 235 at 20000)
+        // itself (a step is then a chain, and two lengthen it), two a thread from
+        // there.  400 steps, one / two a thread / the general kernel, us: up to
+        // 19456 members 171 / 205 / 218, with renormalisation 205 / 261 / 244; to
+        // twice that 235 / 205 / 278 and 270 / 262 / 306; 50000 members 324 / 290
+        // / 322 and 368 / 347 / 346; 200000 1071 / 767 / 1035 and 1196 / 871 / 1124
         const bool one = n == 1 && p.E <= 32 * 4 * 152;
         const int64_t items = n == 1 && !one ? (p.E + 1) / 2 : p.E;
         const int threads = items <= 32 * 4 * 4 * 152 ? 32 : 128;

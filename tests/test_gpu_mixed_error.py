@@ -97,3 +97,43 @@ def test_increments_are_added_to_the_state_without_error(gpu_lib, n, items):
     exact = _run(m0, ax, sr, al, happ, dt, w, D)
     stated = _rms(_run(m0, ax, sr, al, happ, dt, w, F), exact)
     assert _rms(_gpu(n, ax, m0, sr, alpha, happ, dt, w), exact) <= 1.03 * stated
+
+
+@pytest.mark.parametrize("n", [1, 2, 30, 500, 1000])
+def test_the_stage_map_forms_no_terms_that_cancel(gpu_lib, n):
+    """T = 0 and alpha = 1, where the damping term's rounding is what there is:
+    expanded to v |m|^2 - m (m.v) it has terms that cancel, and the error is 1.4
+    times the statement's."""
+    items, happ, dt, steps = max(1000, n), 0.125, 2.0 ** -10, 300
+    ax, m0, sr, w = _inputs(items // n * n, steps, 0.0, 32)
+    al = np.ones(m0.shape[1])
+    exact = _run(m0, ax, sr, al, happ, dt, w, D)
+    stated = _rms(_run(m0, ax, sr, al, happ, dt, w, F), exact)
+    assert _rms(_gpu(n, ax, m0, sr, 1.0, happ, dt, w), exact) <= 1.1 * stated
+
+
+@pytest.mark.parametrize("n,mpc", [(200, 2), (200, 4), (320, 2), (320, 4)])
+def test_the_map_with_several_members_a_block(gpu_lib, n, mpc):
+    """The same for clusters of more than 32 particles that share their
+    parameters, several members a CTA; the time step and field in SI units are
+    those that reduce to the statement's."""
+    from magpy_gb300 import core
+    E, steps, ms, K, happ, dt = 5, 300, 4e5, 2e4, 0.125, 2.0 ** -10
+    ax, m0, sr, w = _inputs(n, steps, 0.0, 34)
+    exact = _run(m0, ax, sr, np.ones(n), happ, dt, w, D)
+    stated = _rms(_run(m0, ax, sr, np.ones(n), happ, dt, w, F), exact)
+    # lib/simulation.cpp:519-549
+    mu0, gyro = 1.25663706e-6, 1.76086e11
+    hk = 2 * K / mu0 / ms
+    dt_si = dt * 2 / (gyro * mu0 * hk)
+    plan = core.EnsemblePlan(E, np.full(n, 7e-9), np.full(n, K), ax.T, m0.T, np.zeros((n, 3)), ms,
+                             1.0, 0.0, False, False, False, dt_si, (steps + 0.5) * dt_si, 2,
+                             np.arange(E), "constant", happ * hk, precision="mixed")
+    try:
+        a = plan.set_launch(4, mpc).run().arrays()
+    finally:
+        plan.close()
+    assert np.all(a.status == 0) and np.all(a.steps == steps + 1)
+    got = np.stack([a.mx[1], a.my[1], a.mz[1]]).reshape(3, E, n) / ms
+    for e in range(E):
+        assert _rms(got[:, e], exact) <= 1.1 * stated
