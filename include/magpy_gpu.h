@@ -217,17 +217,21 @@ int magpy_batch_destroy(magpy_batch *batch);
  * reference counterpart: the reference computes no gradients).  For an
  * ensemble whose members share one geometry and all parameters (Heun, no
  * renormalisation, in-kernel increments, at most 512 particles per member),
- * magpy_adjoint_forward integrates in
- * mixed precision keeping a float-float checkpoint every checkpoint_every
- * steps, and writes the samples into the plan (magpy_adjoint_plan; its
- * ensemble statistics apply).  For an objective J of the ensemble
- * magnetisation samples M_s = (1/E) sum_e sum_q m_z (A/m), given dJ/dM_s,
- * magpy_adjoint_backward recomputes each segment from its checkpoint and
- * sweeps it backward, returning grad_theta = dJ/d(K, alpha, H0) (J/m^3,
+ * magpy_adjoint_forward integrates in mixed precision and writes the samples
+ * into the plan (magpy_adjoint_plan; its ensemble statistics apply).  For an
+ * objective J of the ensemble magnetisation samples
+ * M_s = (1/E) sum_e sum_q m_z (A/m), given dJ/dM_s, magpy_adjoint_backward
+ * sweeps the run backward and returns grad_theta = dJ/d(K, alpha, H0) (J/m^3,
  * damping, A/m; K is the mean anisotropy with all K_i scaled together) and
  * the sensitivities to the reduced quantities (dt, sqrt(dt), alpha, happ,
  * dipolar prefactor).  Any direct dependence of J on the field (as in the
- * energy dissipated) is the caller's to add. */
+ * energy dissipated) is the caller's to add.
+ * Device memory: with interactions, forward keeps the moments and dipolar fields
+ * of every step (36 bytes a particle and step) where these take at most 4 GiB and
+ * at most a sixteenth of the device's free memory when the object is created.
+ * Otherwise it keeps a float-float checkpoint every checkpoint_every steps (24
+ * bytes a particle), and backward recomputes one segment of that many steps at a
+ * time (36 bytes a particle and step within the same bounds, else 12). */
 typedef struct magpy_adjoint magpy_adjoint;
 int magpy_adjoint_create(const magpy_ensemble_desc *desc, int64_t checkpoint_every,
                          magpy_adjoint **adjoint, void *stream);

@@ -21,12 +21,17 @@ from .core import MU0, _ensemble_desc, _GroupPlan
 
 
 class EnsembleAdjoint:
-    """Forward run with checkpoints and its adjoint for one parameter set.
+    """Forward run and its adjoint for one parameter set.
 
     Arguments as ``core.simulate_ensemble`` (members share the geometry; no
     renormalisation; Heun; in-kernel increments).  The anisotropy argument is
     the per-particle K; the gradient is with respect to the mean K with all
     particles scaled together.
+
+    With interactions the forward run keeps 36 bytes a particle and step for the
+    sweep back where these take 4 GiB and a sixteenth of the free device memory at
+    most; otherwise checkpoints every ``checkpoint_every`` steps, and the sweep
+    recomputes one segment at a time.
     """
 
     def __init__(self, n_members, radius, anisotropy, anisotropy_axis, magnetisation_direction,

@@ -22,9 +22,9 @@
 //     Gh = sum mu.h (d/d dt), Gw = sum mu.(sr w) (d/d sqrt(dt)),
 //     Ga = sum g.dF/dalpha, Ghapp = sum eta_z s, Gc = sum eta.(D x)/c.
 // The forward pass keeps every step's moments and dipolar fields where they fit
-// (4 GiB); otherwise checkpoints every C steps keep the float-float state, and
-// each segment is recomputed forward (same code, same bits) into a buffer of
-// moments (and fields) and then swept backward.
+// (adjoint_keep in rules.hpp); otherwise checkpoints every C steps keep the
+// float-float state, and each segment is recomputed forward (same code, same bits)
+// into a buffer of moments (and fields) and then swept backward.
 //
 // What bounds it: the dipolar sums, by their instructions, table reads and
 // chains.  In a large ensemble a thread integrates particle q of two members
@@ -213,7 +213,7 @@ struct AdjArgs {
     const float2 *stab;   // sin of the applied waveform at t_k and t_k + dt, per step
     float happ, dt, sq, alpha, c;
     const int64_t *sched;
-    float *ck;            // [K/C + 1][6][pairs] V: checkpoints (hi xyz, lo xyz)
+    float *ck;            // [K/C + 1][6][pairs] V: checkpoints (hi xyz, lo xyz); none if `whole`
     // [C][3 or 9][pairs] V: moments (and dipolar fields) of the segment being
     // swept; `whole`: [K][9][pairs] of the whole run, written by the forward pass
     float *seg;
@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(MAXT) adj_forward_kernel(AdjArgs A)
         hi[c] = both<V>((float)v0, (float)v1);
         lo[c] = both<V>((float)(v0 - (double)first(hi[c])), (float)(v1 - (double)last(hi[c])));
     }
-    write_ck(A, M, 0, hi, lo);
+    if (!WHOLE) write_ck(A, M, 0, hi, lo);
     write_sample_a(A, M, 0, hi, lo);
     int64_t s_next = 1, ck = 0, next_ck = A.C;
     for (int64_t step = 1; step <= A.K; step++) {

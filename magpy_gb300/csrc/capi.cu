@@ -24,6 +24,7 @@
 
 #include "../../include/magpy_gpu.h"
 #include "plan.hpp"
+#include "rules.hpp"
 
 namespace magpy {
 namespace {
@@ -1739,25 +1740,26 @@ extern "C" int magpy_adjoint_create(const magpy_ensemble_desc *d, int64_t checkp
     CUDA_TRY(pool_alloc(&A->bufs[0], P * sizeof(double)));
     CUDA_TRY(cudaMemcpy(A->bufs[0], vred.data(), P * sizeof(double), cudaMemcpyHostToDevice));
     // checkpoints and the segment's moments, two members side by side
-    const size_t P2 = (size_t)(E + 1) / 2 * 2 * n;
-    CUDA_TRY(pool_alloc(&A->bufs[1], nck * 6 * P2 * sizeof(float)));
-    // the dipolar fields (6 floats a particle and step beside the moments' 3) are
-    // kept where that takes 4 GiB at most: of the whole run, else of a segment;
-    // with no room for them either they are computed again
-    const size_t limit = (size_t)4 << 30, steps = (size_t)std::max<int64_t>(K, 1);
-    const size_t seg = std::min((size_t)C, steps) * P2 * sizeof(float);
-    const auto keep = [&](size_t planes) {
-        if (pool_alloc(&A->bufs[2], planes) == cudaSuccess) return true;
+    const size_t P2 = (size_t)(E + 1) / 2 * 2 * n, plane = P2 * sizeof(float);
+    const size_t steps = (size_t)std::max<int64_t>(K, 1), seg = std::min((size_t)C, steps);
+    const auto keep = [&](size_t bytes) {
+        if (pool_alloc(&A->bufs[2], bytes) == cudaSuccess) return true;
         (void)cudaGetLastError();
         A->bufs[2] = nullptr;
         return false;
     };
     if (d->interactions && n > 1) {
-        if (P2 > 0 && steps <= limit / (9 * P2 * sizeof(float)))
-            A->a.kept = A->a.whole = keep(9 * steps * P2 * sizeof(float));
-        if (!A->a.kept && seg <= limit / 9) A->a.kept = keep(9 * seg);
+        size_t free_bytes = 0, total_bytes = 0;
+        CUDA_TRY(cudaMemGetInfo(&free_bytes, &total_bytes));
+        AdjointKeep k = adjoint_keep(steps, (size_t)C, P2, free_bytes);
+        if (k == AdjointKeep::whole) {
+            A->a.kept = A->a.whole = keep(9 * steps * plane);
+            k = AdjointKeep::segment;  // where the pool refuses the larger form
+        }
+        if (!A->a.kept && k == AdjointKeep::segment) A->a.kept = keep(9 * seg * plane);
     }
-    if (!A->a.kept) CUDA_TRY(pool_alloc(&A->bufs[2], 3 * seg));
+    if (!A->a.kept) CUDA_TRY(pool_alloc(&A->bufs[2], 3 * seg * plane));
+    if (!A->a.whole) CUDA_TRY(pool_alloc(&A->bufs[1], nck * 6 * plane));
     CUDA_TRY(pool_alloc(&A->bufs[3], std::max<int64_t>(A->S, 1) * sizeof(double)));
     CUDA_TRY(pool_alloc(&A->bufs[4], 5 * sizeof(double)));
     if (R.shape != MAGPY_FIELD_CONSTANT && K > 0) {
