@@ -222,7 +222,7 @@ struct magpy_plan {
     float *ftab = nullptr;
     float4 *pr = nullptr;
     __half *tc_d = nullptr;     // FP16 hi/lo dipolar matrix (tensor-core mode)
-    __half *tcc_b = nullptr;    // B buffers of the cluster kernel (n > 64)
+    __half *tcc_b = nullptr;    // B buffers of the cluster kernels that stream them
     size_t tcc_b_bytes = 0;
     int32_t tcc_last_nb = 0;    // members per cluster of the last run (0: none yet)
     int tcc_max_clusters[3] = {0, 0, 0};  // resident clusters of 32 / 64 / 40 members
@@ -230,6 +230,9 @@ struct magpy_plan {
     bool on_device = false;     // the caller's buffers are device pointers
     int64_t max_steps = 0;
     std::vector<double> times, fields;  // [E][S] host-side sample times and fields
+    // The kernel of a tensor-core plan for clusters of CTAs exchanges B through
+    // global memory (the Heun form of up to TCR_MAX_N particles does not).
+    bool streams_b() const { return p.use_implicit || p.n > magpy::TCR_MAX_N; }
     ~magpy_plan()
     {
         // a run may still be in flight on any stream: wait once, then hand
@@ -559,12 +562,14 @@ int make_plan(const std::vector<const Reduced *> &members, const std::vector<uin
         cudaError_t err = tcc_build_d(p.pt, p.rt, (int)n, plan->tc_d, st);
         if (err != cudaSuccess)
             return fail(MAGPY_ERR_CUDA, std::string("dipolar matrix: ") + cudaGetErrorString(err));
-        plan->tcc_b_bytes = std::max({tcc_b_elems((int)n, E, 32), tcc_b_elems((int)n, E, 40),
-                                      tcc_b_elems((int)n, E, 48),
-                                      tcc_b_elems((int)n, E, 64)}) *
-                            sizeof(__half);
-        CUDA_TRY(pool_alloc((void **)&plan->tcc_b, plan->tcc_b_bytes));
-        CUDA_TRY(cudaMemsetAsync(plan->tcc_b, 0, plan->tcc_b_bytes, st));
+        if (plan->streams_b()) {
+            plan->tcc_b_bytes = std::max({tcc_b_elems((int)n, E, 32), tcc_b_elems((int)n, E, 40),
+                                          tcc_b_elems((int)n, E, 48),
+                                          tcc_b_elems((int)n, E, 64)}) *
+                                sizeof(__half);
+            CUDA_TRY(pool_alloc((void **)&plan->tcc_b, plan->tcc_b_bytes));
+            CUDA_TRY(cudaMemsetAsync(plan->tcc_b, 0, plan->tcc_b_bytes, st));
+        }
     }
     CUDA_TRY(cudaStreamSynchronize(st));  // host tables are released on return
     *out = plan.release();
@@ -603,15 +608,17 @@ int run_plan(magpy_plan *plan, cudaStream_t st)
                 if (waves <= best) { best = waves; nb = m; }  // equal: fewer members
             }
         }
-        // the B buffers were sized for every member count a launch may take
-        if (tcc_b_elems((int)plan->p.n, plan->p.E, nb) * sizeof(__half) > plan->tcc_b_bytes)
-            return fail(MAGPY_ERR_UNSUPPORTED, "cluster B buffer smaller than the " +
-                                                   std::to_string(nb) + "-member layout");
-        if (plan->tcc_last_nb != 0 && plan->tcc_last_nb != nb)
-            // the other layout's words could land on positions this one
-            // never writes: start from zero again
-            CUDA_TRY(cudaMemsetAsync(plan->tcc_b, 0, plan->tcc_b_bytes, st));
-        plan->tcc_last_nb = nb;
+        if (plan->streams_b()) {
+            // the B buffers were sized for every member count a launch may take
+            if (tcc_b_elems((int)plan->p.n, plan->p.E, nb) * sizeof(__half) > plan->tcc_b_bytes)
+                return fail(MAGPY_ERR_UNSUPPORTED, "cluster B buffer smaller than the " +
+                                                       std::to_string(nb) + "-member layout");
+            if (plan->tcc_last_nb != 0 && plan->tcc_last_nb != nb)
+                // the other layout's words could land on positions this one
+                // never writes: start from zero again
+                CUDA_TRY(cudaMemsetAsync(plan->tcc_b, 0, plan->tcc_b_bytes, st));
+            plan->tcc_last_nb = nb;
+        }
         le = launch_tcc(plan->p, plan->tc_d, plan->tcc_b, nb, st);
     } else if (plan->precision == MAGPY_PRECISION_MIXED && !plan->p.use_implicit) {
         le = launch_mixed(plan->p, st);
@@ -1580,7 +1587,7 @@ extern "C" int magpy_batch_create(const magpy_ensemble_desc *groups, int64_t n_g
             float best_ms = 1e30f;
             for (int32_t nb : {64, 48, 40, 32}) {
                 pl->p.members_per_warp = nb;
-                if (pl->tcc_last_nb != nb) {  // no memset node in the captured graph
+                if (pl->streams_b() && pl->tcc_last_nb != nb) {  // no memset node in the graph
                     CUDA_TRY(cudaMemsetAsync(pl->tcc_b, 0, pl->tcc_b_bytes, st));
                     pl->tcc_last_nb = nb;
                 }
@@ -1591,7 +1598,7 @@ extern "C" int magpy_batch_create(const magpy_ensemble_desc *groups, int64_t n_g
             if (rc) break;
             pl->p.members_per_warp = best_nb;
             B->members_per_warp[g] = best_nb;
-            if (pl->tcc_last_nb != best_nb) {
+            if (pl->streams_b() && pl->tcc_last_nb != best_nb) {
                 CUDA_TRY(cudaMemsetAsync(pl->tcc_b, 0, pl->tcc_b_bytes, st));
                 pl->tcc_last_nb = best_nb;
             }
