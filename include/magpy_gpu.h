@@ -187,9 +187,10 @@ int magpy_plan_destroy(magpy_plan *plan);
  * With autotune = 1 the launch configuration of each group is chosen by
  * timing the candidates on a short window of that group's own ensemble:
  * for MAGPY_PRECISION_MIXED / _MIXED_TC groups the kernel (FP32 CUDA-core or
- * tensor-core dipolar field), and for clusters of <= 32 particles the number
- * of warps per CTA (1, 2, 4 or 8) and of members packed per warp (all that
- * fit, a quarter of that, or one).  Choices are cached per process.  For a
+ * tensor-core dipolar field), and for clusters of <= 32 particles (3 to 32 for a
+ * mixed Heun run) the number of warps per CTA (1, 2, 4 or 8) and of members packed
+ * per warp (all that fit, a quarter of that, or one).  Choices are cached per
+ * process.  For a
  * group on the cluster tensor-core kernel (65 or more particles) the members
  * per thread-block cluster (64, 48 or 32) set how many SMs the group holds
  * beside the others, so that count is chosen by timing the whole graph.

@@ -1453,7 +1453,8 @@ extern "C" int magpy_batch_create(const magpy_ensemble_desc *groups, int64_t n_g
                 // launch shapes of the warp-packed kernels: warps per CTA and
                 // members per warp (full packing, a quarter of it, one)
                 std::vector<std::pair<int32_t, int32_t>> shapes{{4, 0}};
-                if (d.n_particles <= 32) {
+                // (one or two particles in mixed precision: the kernel has none to choose)
+                if (d.n_particles <= 32 && !(mixed && d.n_particles <= 2)) {
                     const int32_t full = (int32_t)(32 / d.n_particles);
                     std::vector<int32_t> mpws{0};
                     if (full >= 4) mpws.push_back(full / 4);
