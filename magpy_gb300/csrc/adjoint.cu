@@ -575,7 +575,7 @@ static Launch shape(int n, int64_t E, bool interactions)
         L.grid = dim3((unsigned)items);
     } else {
         // one warp per CTA while every warp has a sub-partition or a few share one
-        const int warps = (items + mpw - 1) / mpw <= 4 * 4 * 152 ? 1 : 4;
+        const int warps = (items + mpw - 1) / mpw <= 4 * sub_partitions() ? 1 : 4;
         L.block = dim3(L.split ? 64 : 32 * warps);
         const int64_t per_block = (int64_t)(L.split ? 1 : warps) * mpw;
         L.grid = dim3((unsigned)((items + per_block - 1) / per_block));

@@ -1010,7 +1010,7 @@ int magpy_dom_dynamics(const magpy_dom_desc *d, double *mz, double *field, doubl
     a.N = N;
     a.members = (const DomMember *)bm.p;
     a.order = (const int64_t *)bo.p;
-    a.lanes = dom_lanes_rule(expected.data(), E);
+    a.lanes = dom_lanes_rule(expected.data(), E, sm_count());
     a.shape = d->field_shape;
     a.ncomp = d->field_n_components;
     a.time_step = d->time_step;

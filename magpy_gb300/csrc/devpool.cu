@@ -8,6 +8,7 @@
 // been synchronised, plan buffers after the device has been (the plan's
 // destructor does it); any other free synchronises the device first, as
 // cudaFree does.
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <unordered_map>
@@ -122,6 +123,20 @@ void pool_trim(int dev)
     if (cur != dev) cudaSetDevice(dev);
     for (void *p : drop) cudaFree(p);
     if (cur != dev) cudaSetDevice(cur);
+}
+
+int sm_count()
+{
+    static std::atomic<int> counts[64];  // by device; 0: not asked yet
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+    if ((n = counts[dev].load(std::memory_order_relaxed)) > 0) return n;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) {
+        (void)cudaGetLastError();
+        return 152;  // a full GB300; the launch reports what is wrong
+    }
+    counts[dev].store(n, std::memory_order_relaxed);
+    return n;
 }
 
 }  // namespace magpy

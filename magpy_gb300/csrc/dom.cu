@@ -17,10 +17,10 @@
 // The reference's retry loop and sampling loop have no bound; here each step
 // gives up after MAX_ATTEMPTS rejected trials and each particle after
 // max_steps steps, with a status bit, so a NaN never turns into a spin.
-#include <algorithm>
 #include <cmath>
 #include "common.cuh"
 #include "plan.hpp"
+#include "rules.hpp"
 
 namespace magpy {
 
@@ -28,11 +28,9 @@ namespace {
 
 constexpr double KB_D = 1.38064852e-23;  // include/constants.hpp:10-12
 constexpr double GYRO_D = 1.76086e11;
-// One warp per CTA: the step counts of particles differ by orders of
-// magnitude, so the launch (heaviest warps first) leaves the balancing of
+// One warp per CTA (DOM_THREADS, rules.hpp): the step counts of particles differ by
+// orders of magnitude, so the launch (heaviest warps first) leaves the balancing of
 // the SMs' FP64 pipes to the CTA scheduler.
-constexpr int DOM_THREADS = 32;
-constexpr int DOM_GROUPS = 6;  // particles per warp with five lanes each
 
 struct DomParams {
     double hpre;   // (tau_N sqrt(pi)) / sigma^1.5
@@ -343,22 +341,6 @@ __global__ void __launch_bounds__(DOM_THREADS) dom_kernel(DomArgs a)
 }
 
 }  // namespace
-
-int64_t dom_lanes_rule(const double *steps, int64_t E)
-{
-    // Five lanes take a particle through a step in 0.42 of the time and in 2.4
-    // times the FP64 issue of one thread.  The first ones of the order get them
-    // while every warp still has a sub-partition of its own; past that, those
-    // that would need more than half the time of the whole batch by themselves.
-    constexpr int64_t SUBS = 4 * 152;
-    const int64_t fill = (SUBS * DOM_THREADS - E) * DOM_GROUPS / (DOM_THREADS - DOM_GROUPS);
-    int64_t lanes = std::min(E, std::max<int64_t>(0, fill));
-    double sum = 0.0;
-    for (int64_t e = 0; e < E; e++) sum += steps[e];
-    const double alone = std::max(1.3 * sum / (double)E, 0.5 * sum / (double)(SUBS * DOM_THREADS));
-    while (lanes < E && steps[lanes] > alone) lanes++;
-    return lanes;
-}
 
 cudaError_t launch_dom(const DomArgs &a, cudaStream_t stream)
 {

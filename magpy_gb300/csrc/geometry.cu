@@ -227,7 +227,7 @@ cudaError_t launch_geometry(const GeoArgs &a, cudaStream_t stream)
     // One warp per member wastes the fewest candidates (the first valid one
     // ends a batch); with fewer members than sub-partitions the chip has idle
     // ones, and a wider batch shortens the search of each.
-    return a.E >= 4 * 152 ? launch_geometry_t<32>(a, stream) : launch_geometry_t<GEO_WIDE>(a, stream);
+    return a.E >= sub_partitions() ? launch_geometry_t<32>(a, stream) : launch_geometry_t<GEO_WIDE>(a, stream);
 }
 
 }  // namespace magpy

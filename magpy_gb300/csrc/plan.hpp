@@ -50,6 +50,10 @@ cudaError_t pool_alloc(void **ptr, size_t bytes);
 void pool_free(void *ptr, bool device_synced = false);
 void pool_trim(int device);
 
+// SMs of the current device, four sub-partitions each (devpool.cu).
+int sm_count();
+inline int sub_partitions() { return 4 * sm_count(); }
+
 // Launchers (one translation unit each).
 cudaError_t launch_fp64(const DevPlan &p, cudaStream_t stream);
 // FP64-faithful kernel for small ensembles of small clusters: several lanes
@@ -136,9 +140,6 @@ struct DomArgs {
     int64_t *steps = nullptr;
 };
 cudaError_t launch_dom(const DomArgs &a, cudaStream_t stream);
-// How many of E particles, in descending order of their expected relative step
-// counts, get five lanes.
-int64_t dom_lanes_rule(const double *steps, int64_t E);
 // Seeded cluster geometry (geometry.cu): one CTA per member.
 struct GeoArgs {
     int64_t E = 0;

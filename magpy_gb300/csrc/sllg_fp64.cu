@@ -650,7 +650,7 @@ cudaError_t launch_fp64(const DevPlan &p, cudaStream_t stream)
             // 64 SMs idle), members apart where that costs no second warp.
             // 10000 dimers, implicit: 8.7-9.2 ms in CTAs of four warps (five SMs
             // take a second CTA), 6.5 ms in CTAs of one.
-            const int64_t subs = 4 * 152;
+            const int64_t subs = sub_partitions();
             if (p.members_per_warp <= 0)
                 mpw = (int)std::min<int64_t>(32 / n, std::max<int64_t>(1, (p.E + subs - 1) / subs));
             warps = (p.E + mpw - 1) / mpw <= 4 * subs ? 1 : 4;

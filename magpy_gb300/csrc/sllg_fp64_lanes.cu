@@ -29,7 +29,6 @@ namespace magpy {
 namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
-constexpr int SUBS = 4 * 152;  // sub-partitions of the chip
 
 // A lane's place: component c, the next two v = c + 1, w = c + 2 (mod 3), the
 // first lane of its particle's group, and its row-column entry.
@@ -437,9 +436,9 @@ finished:
 static int lanes_cols(const DevPlan &p)
 {
     if (p.block_warps > 0 || p.members_per_warp > 0 || !p.one_schedule || p.n > 8) return 0;
-    const int64_t warps = (p.E + 8 / p.n - 1) / (8 / p.n);
-    if (p.use_implicit && p.n <= 2 && (p.E + 2 / p.n - 1) / (2 / p.n) <= SUBS) return 3;
-    return warps <= (p.use_implicit ? SUBS : 2 * SUBS) ? 1 : 0;
+    const int64_t warps = (p.E + 8 / p.n - 1) / (8 / p.n), subs = sub_partitions();
+    if (p.use_implicit && p.n <= 2 && (p.E + 2 / p.n - 1) / (2 / p.n) <= subs) return 3;
+    return warps <= (p.use_implicit ? subs : 2 * subs) ? 1 : 0;
 }
 
 bool fp64_lanes_fit(const DevPlan &p) { return lanes_cols(p) > 0; }
@@ -449,8 +448,8 @@ cudaError_t launch_fp64_lanes(const DevPlan &p, cudaStream_t stream)
     const int cols = lanes_cols(p);
     DevPlan q = p;
     // members apart where every warp still has a sub-partition
-    const int64_t most = (cols == 1 ? 8 : 2) / p.n;
-    q.members_per_warp = (int)std::min<int64_t>(most, std::max<int64_t>(1, (p.E + SUBS - 1) / SUBS));
+    const int64_t most = (cols == 1 ? 8 : 2) / p.n, subs = sub_partitions();
+    q.members_per_warp = (int)std::min<int64_t>(most, std::max<int64_t>(1, (p.E + subs - 1) / subs));
     const unsigned grid = (unsigned)((p.E + q.members_per_warp - 1) / q.members_per_warp);
     if (!p.use_implicit) sllg_fp64_lanes_kernel<false, 1><<<grid, 32, 0, stream>>>(q);
     else if (cols == 1) sllg_fp64_lanes_kernel<true, 1><<<grid, 32, 0, stream>>>(q);

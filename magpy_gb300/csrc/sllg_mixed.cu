@@ -716,9 +716,10 @@ cudaError_t launch_mixed(const DevPlan &p, cudaStream_t stream)
         // 19456 members 171 / 205 / 218, with renormalisation 205 / 261 / 244; to
         // twice that 235 / 205 / 278 and 270 / 262 / 306; 50000 members 324 / 290
         // / 322 and 368 / 347 / 346; 200000 1071 / 767 / 1035 and 1196 / 871 / 1124
-        const bool one = n == 1 && p.E <= 32 * 4 * 152;
+        const int64_t subs = sub_partitions();
+        const bool one = n == 1 && p.E <= 32 * subs;
         const int64_t items = n == 1 && !one ? (p.E + 1) / 2 : p.E;
-        const int threads = items <= 32 * 4 * 4 * 152 ? 32 : 128;
+        const int threads = items <= 32 * 4 * subs ? 32 : 128;
         const unsigned blocks = (unsigned)((items + threads - 1) / threads);
         if (one) sllg_mixed_two_kernel<true, true><<<blocks, threads, 0, stream>>>(p);
         else if (n == 1) sllg_mixed_two_kernel<true><<<blocks, threads, 0, stream>>>(p);

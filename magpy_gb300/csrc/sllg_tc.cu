@@ -29,6 +29,7 @@
 #include <cuda_fp16.h>
 #include "common.cuh"
 #include "plan.hpp"
+#include "rules.hpp"
 #include "tc_ptx.cuh"
 #include "llg32.cuh"
 #include "llg64.cuh"
@@ -930,16 +931,9 @@ cudaError_t launch_tc(const DevPlan &p, const __half *dhi, const __half *dlo, cu
     if (!tc_supported(p.n)) return cudaErrorNotSupported;
     cudaError_t err = tc_init_attributes();
     if (err != cudaSuccess) return err;
-    // Members per CTA: the fewest that need no more waves of CTAs than 32 (a
-    // CTA's step takes less time with fewer: 3.75, 3.9, 4.2 and 4.9 us with 8,
-    // 16, 20 and 32 members of 64 particles, 2.63 and 2.65 with 8 and 32 of 16),
-    // unless a launch shape is set: the groups of a batch share the SMs, and 32 a
-    // CTA cost the least SM time.
-    int nm = NM;
-    if (p.block_warps <= 0) {
-        const int64_t sms = 152, waves = ((p.E + NM - 1) / NM + sms - 1) / sms;
-        while (nm > 8 && (p.E + nm - 5) / (nm - 4) <= waves * sms) nm -= 4;
-    }
+    // Members per CTA by the ensemble's size, unless a launch shape is set: the
+    // groups of a batch share the SMs, and 32 a CTA cost the least SM time.
+    const int nm = p.block_warps > 0 ? NM : tc_members(p.E, sm_count());
     const int gm0 = (nm / 2 + 3) / 4 * 4, gm1 = nm - gm0;
     const unsigned grid = (unsigned)((p.E + nm - 1) / nm);
     // the plan's default phase-wait bound is the compile-time one
