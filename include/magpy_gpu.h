@@ -229,8 +229,8 @@ int magpy_batch_destroy(magpy_batch *batch);
  * energy dissipated) is the caller's to add.
  * Device memory: with interactions, forward keeps the moments and dipolar fields
  * of every step (36 bytes a particle and step) where these take at most 4 GiB and
- * at most a sixteenth of the device's free memory when the object is created.
- * Otherwise it keeps a float-float checkpoint every checkpoint_every steps (24
+ * at most a sixteenth of the device's free memory when the object is created (or
+ * at most 64 MiB).  Otherwise it keeps a float-float checkpoint every checkpoint_every steps (24
  * bytes a particle), and backward recomputes one segment of that many steps at a
  * time (36 bytes a particle and step within the same bounds, else 12). */
 typedef struct magpy_adjoint magpy_adjoint;

@@ -1758,8 +1758,11 @@ extern "C" int magpy_adjoint_create(const magpy_ensemble_desc *d, int64_t checkp
     };
     if (d->interactions && n > 1) {
         size_t free_bytes = 0, total_bytes = 0;
-        CUDA_TRY(cudaMemGetInfo(&free_bytes, &total_bytes));
-        AdjointKeep k = adjoint_keep(steps, (size_t)C, P2, free_bytes);
+        AdjointKeep k = adjoint_keep(steps, (size_t)C, P2, 0);
+        if (k != AdjointKeep::whole) {
+            CUDA_TRY(cudaMemGetInfo(&free_bytes, &total_bytes));
+            k = adjoint_keep(steps, (size_t)C, P2, free_bytes);
+        }
         if (k == AdjointKeep::whole) {
             A->a.kept = A->a.whole = keep(9 * steps * plane);
             k = AdjointKeep::segment;  // where the pool refuses the larger form

@@ -11,12 +11,15 @@ namespace magpy {
 // planes more, of every step of the run (which then needs no checkpoints), of the
 // segment being swept, or of none.  The kept planes are bounded by 4 GiB, and by
 // a sixteenth of the memory that is free, so that objects made side by side never
-// take most of it from the plans that follow them.
+// take most of it from the plans that follow them.  Up to 64 MiB are kept without
+// asking what is free (the driver takes 60 us to tell, a seventh of a small
+// gradient).
 enum class AdjointKeep { none, segment, whole };
+constexpr size_t ADJOINT_KEEP_UNASKED = (size_t)64 << 20;
 
 inline AdjointKeep adjoint_keep(size_t steps, size_t every, size_t particles, size_t free_bytes)
 {
-    const size_t limit = std::min((size_t)4 << 30, free_bytes / 16);
+    const size_t limit = std::max(ADJOINT_KEEP_UNASKED, std::min((size_t)4 << 30, free_bytes / 16));
     const auto fits = [&](size_t n) {
         return particles == 0 || n <= limit / 9 / sizeof(float) / particles;
     };

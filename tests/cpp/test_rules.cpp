@@ -23,14 +23,17 @@ static void adjoint()
     CHECK(adjoint_keep(K, C, P, 19 * GB) == AdjointKeep::whole);
     CHECK(adjoint_keep(K, C, P, 18 * GB) == AdjointKeep::segment);  // 16 times 1.16 GiB
     CHECK(adjoint_keep(K, C, P, GB / 2) == AdjointKeep::segment);
-    CHECK(adjoint_keep(K, C, P, GB / 8) == AdjointKeep::none);
-    CHECK(adjoint_keep(K, C, P, 0) == AdjointKeep::none);
+    CHECK(adjoint_keep(K, 2 * C, 16 * P, 0) == AdjointKeep::none);
+    // up to 64 MiB without asking
+    CHECK(adjoint_keep(K, C, P, 0) == AdjointKeep::segment);
+    CHECK(adjoint_keep(1078, C, P, 0) == AdjointKeep::whole);
+    CHECK(adjoint_keep(1079, C, P, 0) == AdjointKeep::segment);
     // at most 4 GiB whatever is free, at most a sixteenth of what is free
     for (size_t free_gb : {1, 3, 17, 64, 65, 280})
         for (size_t k = 1; k < 3000000; k = k * 3 / 2 + 1) {
             const size_t bytes = 36 * k * P;
             if (adjoint_keep(k, C, P, free_gb * GB) == AdjointKeep::whole)
-                CHECK(bytes <= 4 * GB && bytes <= free_gb * GB / 16);
+                CHECK(bytes <= 4 * GB && bytes <= std::max(GB / 16, free_gb * GB / 16));
         }
     // no size product wraps
     CHECK(adjoint_keep((size_t)1 << 32, (size_t)1 << 62, (size_t)1 << 40, 280 * GB) ==
