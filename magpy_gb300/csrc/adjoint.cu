@@ -370,10 +370,13 @@ __device__ inline void keep_moments(const AdjMember<V> &M, V *o, const V m[3])
 
 // WHOLE: every step's moments and dipolar fields are kept for the sweep back,
 // which then forms two sums a step, not the forward pass's two again as well (27
-// particles, 2048 members, 512 steps: 5.4 -> 4.0 ms in all; 1000 members, 256
-// steps: 2.30 -> 1.80).
+// particles, 2048 members, 512 steps: 5.4 -> 3.9 ms in all; 1000 members, 256
+// steps: 2.30 -> 1.80).  The launch bounds leave registers for the loads that a
+// sum's unrolled sources need in flight: left to itself the compiler took 64 to 87,
+// and the pass was slower than the one without kept fields (us, 100 members: 60
+// particles 994 -> 760, 128 4556 -> 2081; 27 particles 736 -> 629).
 template <class V, int MAXT, bool SPLIT, bool WHOLE>
-__global__ void __launch_bounds__(MAXT) adj_forward_kernel(AdjArgs A)
+__global__ void __launch_bounds__(MAXT, MAXT == 128 ? 3 : 1) adj_forward_kernel(AdjArgs A)
 {
     extern __shared__ float4 smem_a[];
     AdjMember<V> M;
