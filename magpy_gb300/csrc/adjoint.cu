@@ -33,7 +33,7 @@
 // dipolar fields are kept beside the moments, so that a step takes four sums in
 // all (two forward, two of the adjoint), six where a segment is recomputed, eight
 // without kept fields.  27 particles, 2048 members, 512 steps with the host's
-// copies: 8.4 -> 5.4 ms with a segment's fields kept, 4.0 with the run's.
+// copies: 8.4 -> 5.4 ms with a segment's fields kept, 3.9 with the run's.
 #include "common.cuh"
 #include "llg32.cuh"
 #include "plan.hpp"
@@ -565,9 +565,10 @@ static Launch shape(int n, int64_t E, bool interactions)
     // form) about fill the sub-partitions and the sums are most of the work.
     // With few warps the chain is what counts, and two warps share the sources
     // (the rest of a step both do).  Forward and backward, 256 steps, ms with
-    // one member / two members / two warps: 27 particles, 2048 members 3.63 /
-    // 2.97 / 4.41; 1000 2.41 / 2.36 / 2.53; 100 1.91 / 2.20 / 1.46; 13, 1000
-    // 1.51 / 1.70 / 1.51; 8, 8000 2.13 / 1.94 / 2.97; 8, 1000 1.27 / 1.49 / 1.05.
+    // one member / two members / two warps: 27 particles, 2048 members 3.93 /
+    // 2.23 / 4.56; 1000 1.58 / 1.61 / 2.50; 100 1.11 / 1.41 / 1.05; 13, 2500
+    // 1.63 / 1.68 / 2.83; 13, 1000 1.16 / 1.32 / 1.21; 8, 8000 3.78 / 2.77 / 4.49;
+    // 8, 1000 1.08 / 1.26 / 0.90; 60, 500 2.70 / 2.55; 60, 200 1.96 / 2.39.
     L.two = warps1 >= 1000 && warps1 * n >= 16000;
     L.split = !L.two && n <= 32 && interactions && n >= 5 && warps1 <= 400;
     const int W = L.two ? 2 : 1;

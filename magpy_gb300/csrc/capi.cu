@@ -587,11 +587,11 @@ int run_plan(magpy_plan *plan, cudaStream_t st)
         // members per cluster: as the launch shape asks (32, 40 or 64; 48
         // for Heun); else the count with the fewest waves of resident
         // clusters, then the fewest members (a wave takes time in proportion
-        // to its clusters' members: at N = 512 an implicit step takes 0.184 ms
-        // a wave with 32, 0.345 with 64; Heun at E = 1638 measured 64 / 48 /
-        // 40 / 32: N = 84 79 / 57 / 53 / 46 ms per 1e4 steps, N = 125 84 /
-        // 65 / 63 / 102 (32: two waves), and at N = 216, E = 1024 212 / 189
-        // / 323 / 296 (40 and 32: two waves); every cluster form runs one CTA
+        // to its clusters' members: at N = 512 an implicit step takes 0.120 ms
+        // a wave with 32, 0.140 with 40, 0.208 with 64; Heun at E = 1638 measured
+        // 64 / 48 / 40 / 32: N = 84 75 / 53 / 50 / 43 ms per 1e4 steps, N = 125
+        // 80 / 61 / 61 / 97 (32: two waves), and at N = 216, E = 1024 210 / 180
+        // / 309 / 278 (40 and 32: two waves); every cluster form runs one CTA
         // per SM, so the resident count depends on the cluster size alone)
         const int32_t mpw = plan->p.members_per_warp;
         const bool imp = plan->p.use_implicit;

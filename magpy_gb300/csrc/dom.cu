@@ -1,5 +1,5 @@
 // dom.cu -- two-state master equation ("discrete orientation model") for a
-// batch of independent particles, one thread per particle.
+// batch of independent particles, one thread per particle or five.
 //
 // Path restated: magpy/core.pyx:205-278 simulate_dom ->
 // simulation::dom_ensemble_dynamics (lib/simulation.cpp:659-767) ->

@@ -26,8 +26,9 @@
 // formed in FP32 in units of the sphere's radius, with a bound on their
 // error that decides all but ~1e-5 of the comparisons; the rest, and the
 // location of the candidate that is taken, are FP64, the same bits as with
-// FP64 throughout.  Drawing 1000 clusters of 27 at 20 % and simulating them:
-// 20.0 ms a call with 256 FP64 candidates a batch, 18.1 ms with this search.
+// FP64 throughout.  Drawing 1000 clusters of 27, a call: 2.14 ms with 256 FP64
+// candidates a batch, 0.19 ms with this search, at a packing of 20 %; 67 and 66 ms
+// at 45 %, where a few members need thousands of batches (of 100: 990 and 342 ms).
 #include <cmath>
 #include "common.cuh"
 #include "plan.hpp"

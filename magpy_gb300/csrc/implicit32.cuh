@@ -8,8 +8,8 @@
 namespace magpy {
 
 // Conversions by integer instructions, the same bits as the hardware's: those
-// run on the FP64 pipe (16 cycles of an SM a warp instruction, as any FP64
-// operation), these take 4-6 cycles of the integer pipes.  Zeros, subnormals,
+// run on the FP64 pipe (16 cycles of an SM a warp instruction, as FP64 operations on
+// one register do; on two they take 19), these take 4-6 cycles of the integer pipes.  Zeros, subnormals,
 // infinities and NaN (and numbers past FP32's range) take the hardware's, in a
 // call: as predicated instructions those were issued every time (8 of the 54 FP64
 // instructions of a particle's iteration).

@@ -12,8 +12,7 @@ namespace magpy {
 // segment being swept, or of none.  The kept planes are bounded by 4 GiB, and by
 // a sixteenth of the memory that is free, so that objects made side by side never
 // take most of it from the plans that follow them.  Up to 64 MiB are kept without
-// asking what is free (the driver takes 60 us to tell, a seventh of a small
-// gradient).
+// asking what is free (the answer takes 60 us, a seventh of a small gradient).
 enum class AdjointKeep { none, segment, whole };
 constexpr size_t ADJOINT_KEEP_UNASKED = (size_t)64 << 20;
 

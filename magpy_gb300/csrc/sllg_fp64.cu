@@ -207,8 +207,8 @@ __device__ void heun_step(const Member &M, const Particle &pa, double x[3],
 // 2 x y + z and d - 0.5 j are one fused operation with an exact product.  The
 // applied field is the step's, the root of the norm is avoided (norm_above),
 // comparisons are integer: about 335 FP64 instructions an iteration, 470 with
-// the functions called one by one (250 steps of one particle 86.9 -> 66.9 ms;
-// 10 steps of 10000 dimers 6.5 -> 5.3 ms).
+// the functions called one by one (a step of one particle 348 -> 268 us, of 10000
+// dimers 0.65 -> 0.47 ms).
 __device__ int32_t implicit_step(const Member &M, const Particle &pa, double x[3],
                                  const double px[3], const double w[3], double hz1, double hz2)
 {
@@ -341,9 +341,8 @@ __device__ int32_t implicit_step(const Member &M, const Particle &pa, double x[3
 // about one half per iteration and takes 27-40 of them a step, this one by
 // dt |D| (the dipolar coupling is left out of it) and takes 3.  FP64 costs 64
 // issue cycles a warp instruction here, so the step's length is the count of
-// its FP64 operations: iterations times ~60.  700 members of 13 particles, a
-// cluster each, dt = 2e-13: 100 steps (with the planning of the call) took
-// 35.2 ms with the reference's iteration, 5.8 ms with this one.
+// its FP64 operations: iterations times ~60.  700 members of 13 particles, dt =
+// 2e-13: 20 steps 4.38 ms with the reference's iteration, 0.31 ms with this one.
 
 // Member-wide FP32 sum, the same bits in every thread of the member.
 __device__ inline float member_sum32(const Member &M, float v)
@@ -648,8 +647,8 @@ cudaError_t launch_fp64(const DevPlan &p, cudaStream_t stream)
             // sub-partitions is spread over them one warp each (700 members of
             // 13 particles, implicit: 350 warps in 88 CTAs of four warps keep
             // 64 SMs idle), members apart where that costs no second warp.
-            // 10000 dimers, implicit: 8.7-9.2 ms in CTAs of four warps (five SMs
-            // take a second CTA), 6.5 ms in CTAs of one.
+            // 10000 dimers, 10 implicit steps: 6.5 ms in CTAs of four warps (five
+            // SMs take a second CTA), 4.7 ms in CTAs of one.
             const int64_t subs = sub_partitions();
             if (p.members_per_warp <= 0)
                 mpw = (int)std::min<int64_t>(32 / n, std::max<int64_t>(1, (p.E + subs - 1) / subs));

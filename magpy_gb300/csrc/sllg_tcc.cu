@@ -670,7 +670,7 @@ __global__ void __launch_bounds__(Cfg<NB>::THREADS, 1)
 // the stopping norm, a sum that squares of any FP32 number do not overflow), its
 // conversions are integer (narrow, widen), as are six of its products (stage_map),
 // and starting from the explicit midpoint saves one iteration of four.  512 members
-// of 512 particles, 40 steps: 18.0 -> 11.4 ms.
+// of 512 particles, 40 steps: 18.0 -> 11.6 ms.
 
 // Per-particle constants of a CTA's 42 particles: FP64 for the residual,
 // FP32 copies for the Jacobian.
