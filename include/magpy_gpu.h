@@ -208,7 +208,9 @@ int magpy_batch_run(magpy_batch *batch, void *stream);
 /* The plan of one group (owned by the batch): outputs, statistics. */
 int magpy_batch_group_plan(magpy_batch *batch, int64_t group, magpy_plan **plan);
 /* The configuration chosen for a group and its tuned time per step (ms; 0
- * when not tuned). */
+ * when not tuned).  The shape is one that magpy_plan_set_launch takes: where the
+ * launcher's own choice was faster than every shape (the group runs with it then,
+ * and the time is its), the fastest of those. */
 int magpy_batch_group_choice(const magpy_batch *batch, int64_t group, int32_t *precision,
                              int32_t *block_warps, int32_t *members_per_warp,
                              double *ms_per_step);

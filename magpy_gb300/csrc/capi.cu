@@ -1376,7 +1376,14 @@ struct TuneKey {
     }
 };
 std::mutex g_tune_mu;
-std::map<TuneKey, std::tuple<int32_t, int32_t, int32_t, double>> g_tune_cache;
+// A group's tuned kernel and launch shape; `own`: the launcher's own choice was
+// faster than any shape, and the group runs with it.
+struct TuneChoice {
+    int32_t precision, block_warps = 4, members_per_warp = 0;
+    bool own = false;
+    double ms = 0.0;
+};
+std::map<TuneKey, TuneChoice> g_tune_cache;
 
 // Time one configuration of a group on a short window of its own ensemble.
 int tune_time(const magpy_ensemble_desc &d0, int32_t precision, int32_t bw, int32_t mpw,
@@ -1425,8 +1432,8 @@ extern "C" int magpy_batch_create(const magpy_ensemble_desc *groups, int64_t n_g
     std::unique_ptr<magpy_batch> B(new magpy_batch());
     for (int64_t g = 0; g < n_groups; g++) {
         const magpy_ensemble_desc &d = groups[g];
-        int32_t prec = d.precision, bw = 4, mpw = 0;
-        double ms = 0.0;
+        TuneChoice ch;
+        ch.precision = d.precision;
         // the implicit solve has one kernel per precision: only its launch shape is tuned
         const bool mixed = !d.use_implicit && (d.precision == MAGPY_PRECISION_MIXED ||
                                                d.precision == MAGPY_PRECISION_MIXED_TC);
@@ -1438,7 +1445,7 @@ extern "C" int magpy_batch_create(const magpy_ensemble_desc *groups, int64_t n_g
                 std::lock_guard<std::mutex> lock(g_tune_mu);
                 auto it = g_tune_cache.find(key);
                 if (it != g_tune_cache.end()) {
-                    std::tie(prec, bw, mpw, ms) = it->second;
+                    ch = it->second;
                     cached = true;
                 }
             }
@@ -1460,8 +1467,6 @@ extern "C" int magpy_batch_create(const magpy_ensemble_desc *groups, int64_t n_g
                     if (full >= 4) mpws.push_back(full / 4);
                     if (full > 1) mpws.push_back(1);
                     shapes.clear();
-                    // the launcher's own choice, which may take another kernel
-                    if (!mixed) shapes.push_back({0, 0});
                     for (int32_t w : {1, 2, 4, 8})
                         for (int32_t m : mpws) shapes.push_back({w, m});
                 }
@@ -1484,25 +1489,39 @@ extern "C" int magpy_batch_create(const magpy_ensemble_desc *groups, int64_t n_g
                         int rc = tune_time(d, pc, sh.first, sh.second, st, &t);
                         if (rc == MAGPY_ERR_UNSUPPORTED) continue;  // e.g. parameters differ
                         if (rc) return rc;
-                        if (t < best) { best = t; prec = pc; bw = sh.first; mpw = sh.second; }
+                        if (t < best) {
+                            best = t;
+                            ch.precision = pc;
+                            ch.block_warps = sh.first;
+                            ch.members_per_warp = sh.second;
+                        }
                     }
-                ms = best;
+                if (!mixed && d.n_particles <= 32) {
+                    // the launcher's own choice, which may take another kernel (no
+                    // shape says so: the one reported stays the fastest of those)
+                    double t = 0.0;
+                    const int rc = tune_time(d, d.precision, 0, 0, st, &t);
+                    if (rc && rc != MAGPY_ERR_UNSUPPORTED) return rc;
+                    ch.own = rc == MAGPY_SUCCESS && t < best;
+                    if (ch.own) best = t;
+                }
+                ch.ms = best;
                 std::lock_guard<std::mutex> lock(g_tune_mu);
-                g_tune_cache[key] = std::make_tuple(prec, bw, mpw, ms);
+                g_tune_cache[key] = ch;
             }
         }
         magpy_ensemble_desc dd = d;
-        dd.precision = prec;
+        dd.precision = ch.precision;
         magpy_plan *plan = nullptr;
         int rc = plan_from_desc(&dd, true, st, &plan);
         if (rc) return rc;
-        plan->p.block_warps = bw;
-        plan->p.members_per_warp = mpw;
+        plan->p.block_warps = ch.own ? 0 : ch.block_warps;
+        plan->p.members_per_warp = ch.own ? 0 : ch.members_per_warp;
         B->plans.push_back(plan);
-        B->precision.push_back(prec);
-        B->block_warps.push_back(bw);
-        B->members_per_warp.push_back(mpw);
-        B->tuned_ms.push_back(ms);
+        B->precision.push_back(ch.precision);
+        B->block_warps.push_back(ch.block_warps);
+        B->members_per_warp.push_back(ch.members_per_warp);
+        B->tuned_ms.push_back(ch.ms);
     }
     // one graph: fork from the capture stream into a stream per group, join back.
     // The groups' streams get scheduling priorities by the group's time alone,
