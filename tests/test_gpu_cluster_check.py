@@ -33,3 +33,26 @@ def test_every_member_stops_at_the_same_check(gpu_lib, n, E, nb, implicit):
         assert np.all(b.status == 0) and np.all(b.steps == 100)
     finally:
         plan.close()
+
+
+@pytest.mark.parametrize("limit", [1, 4, 16])
+@pytest.mark.parametrize("n,nb,implicit", [(125, 32, False), (300, 32, False), (125, 40, True)])
+def test_a_cluster_stops_as_one(gpu_lib, n, nb, implicit, limit):
+    """Limits at which some waits run out and some do not: the CTAs of a cluster
+    mark themselves at different steps, and its members stop together at a check,
+    or run to the end."""
+    from magpy_gb300 import _lib, core
+    from test_gpu_tc_cluster import _lattice_ensemble
+    args = list(_lattice_ensemble(np.random.default_rng(19 + n), n, 6 * nb))
+    args[11] = implicit
+    args[13] = args[12] * 199.5  # 200 steps
+    plan = core.EnsemblePlan(*args, precision="mixed_tc")
+    try:
+        a = plan.set_launch(4, nb).set_wait_limit(limit).run().arrays()
+    finally:
+        plan.close()
+    steps = a.steps.reshape(6, nb)
+    marked = (a.status & _lib.STATUS_WATCHDOG).reshape(6, nb)
+    assert np.all(steps == steps[:, :1]) and np.all(marked == marked[:, :1])
+    assert np.all(np.isin(steps, [64, 128, 192, 200]))
+    assert np.all(marked[steps < 200])
